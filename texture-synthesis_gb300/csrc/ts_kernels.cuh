@@ -125,7 +125,7 @@ constexpr int kKnnTabRadius = 36;
 
 struct StageDev {
   uint32_t level;
-  int slow_lut;            // LUT holds a non-finite value: exact sequential argmin
+  int slow_lut;            // LUT holds a non-finite or negative value: exact sequential argmin
   // Every texel the cost loop can compare has alpha 255 and both LUTs hold
   // +-0 at |a - b| = 0: the alpha channel's term adds +-0 to a partial sum,
   // which leaves it unchanged, so the fast cost loops skip it

@@ -1547,17 +1547,21 @@ void run_plan(ts_session *s, RunCtx &c) {
       const float a = p.alpha * (1.0f - ((float)n_res / (float)total));
       adaptive = (a * a) * a;
     }
-    // stage LUTs (ms.rs:853-858): content = (1 - a) * cauchy when guided
+    // stage LUTs (ms.rs:853-858): content = (1 - a) * cauchy when guided.
+    // Early exit and any-order argmin need terms that never lower a partial
+    // sum, so a non-finite or negative entry sends the stage to the exact
+    // sequential form.  Negative ones come from guided inpainting: a is
+    // negative once the locked pixels outnumber the ones to synthesise.
     bool slow = false;
     for (int d = 0; d < 256; ++d) {
       const float cv = s->guided ? (1.0f - adaptive) * cauchy[d] : cauchy[d];
       luts.push_back(cv);
-      slow |= !std::isfinite(cv);
+      slow |= !std::isfinite(cv) || cv < 0.0f;
     }
     for (int d = 0; d < 256; ++d) {
       const float gv = s->guided ? adaptive * l2[d] : 0.0f;
       luts.push_back(gv);
-      slow |= !std::isfinite(gv);
+      slow |= !std::isfinite(gv) || gv < 0.0f;
     }
     sp.slow_lut = slow;
     const size_t P_eff = std::min(P, redo + n_unresolved);
