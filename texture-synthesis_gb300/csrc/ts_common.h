@@ -76,6 +76,17 @@ TS_HD uint32_t clz64(uint64_t v) {
   return (uint32_t)__builtin_clzll(v);
 #endif
 }
+// p / d for every p < 2^28 as (p * mul) >> sh.  With 2^l < d <= 2^(l+1) and
+// mul = floor(2^(32+l) / d) + 1, mul * d exceeds 2^(32+l) by e <= d <= 2^(l+1),
+// so the quotient's error p e / (d 2^(32+l)) is below 1/d while
+// p < 2^31.  (d = 1: l = -1.)
+TS_HD void ts_div_multiplier(uint32_t d, uint32_t &mul, uint32_t &sh) {
+  uint32_t l1 = 0;  // l + 1
+  while ((1ull << l1) < d) ++l1;
+  sh = 31 + l1;
+  mul = (uint32_t)((1ull << sh) / d + 1);
+}
+
 TS_HD uint64_t mulhi64(uint64_t a, uint64_t b) {
 #ifdef __CUDA_ARCH__
   return __umul64hi(a, b);
@@ -414,16 +425,19 @@ TS_HD uint64_t ts_div_int_rn(uint64_t bs, uint32_t n) {
 // common path (GB300's f64 rate is a small fraction of its f32 rate).
 //
 // d and mean are the reference's exact doubles.  They are split into
-// double-f32 pairs (48 significant bits), divided and exponentiated in
-// double-f32 arithmetic (error-free transformations: two-sum, fused
-// two-product), giving z ~ exp(-q) / 2^m within z * (2^-44 + q * 2^-45) of
-// the value the exact f64 path produces.  The f32 result is returned only
-// when z lies farther than err from every f32 rounding boundary; then
-// rounding the exact f64 value gives the same f32.
-// Otherwise (about one weight in 2^14) the caller falls back to the exact f64
-// path (ts_div_markstein + ts_exp64).  The bound err = 2^-40 + q 2^-42 is at
-// least four times the error above.  q > 80, NaN and operands outside the
-// normal f32 exponent range always fall back.
+// double-f32 pairs (48 significant bits, the high part rounded to nearest),
+// divided and exponentiated in double-f32 arithmetic (error-free
+// transformations: two-sum, fused two-product).  The quotient comes from the
+// mean's f32 reciprocal y (one division per item, FfMean): q1 = d_hi y is
+// within 2^-23 of d / mean, its exact remainder r = d - q1 mean (below
+// 2^-22 d) within 2^-45.4 d, and q2 = r y within 2^-44.4 of q, so q is known
+// to 2^-43.8; with the exponential's own error z ~ exp(-q) / 2^m lies within
+// z * (2^-44 + q * 2^-43.8) of the value the exact f64 path produces.  The
+// f32 result is returned only when z lies farther than err = 2^-40 + q 2^-42
+// from every f32 rounding boundary; then rounding the exact f64 value gives
+// the same f32.  Otherwise (about one weight in 2^14) the caller falls back
+// to the exact f64 path (ts_div_markstein + ts_exp64).  q > 80, NaN and
+// operands outside the normal f32 exponent range always fall back.
 // ---------------------------------------------------------------------------
 #define TS_EXP2_FF_TABLE_VALUES \
   0x1.0000000000000p+0f, 0x0.0p+0f, 0x1.02c9a40000000p+0f, -0x1.887fa00000000p-28f, \
@@ -495,22 +509,39 @@ TS_HD bool ff_split(double v, float &hi, float &lo) {
   return true;
 }
 
-TS_HD bool ts_weight_ff(double d, double mean, const float *tab_ff, float &w) {
-  float q_hi, q_lo, a_hi, a_lo;
-  // a zero or tiny mean (all distances 0 gives 0/0 = NaN) takes the exact path
-  if (!ff_split(mean, a_hi, a_lo)) return false;
-  if (dbl_bits(d) == 0) {
-    q_hi = 0.0f;
-    q_lo = 0.0f;
-  } else {
-    float d_hi, d_lo;
-    if (!ff_split(d, d_hi, d_lo)) return false;
-    const float q1 = TS_FDIV(d_hi, a_hi);
-    const float p = TS_FMUL(q1, a_hi);
-    const float pe = TS_FFMA(q1, a_hi, -p);
+// v as a double-f32 pair whose high part is v rounded to f32.
+TS_HD bool ff_split_rn(double v, float &hi, float &lo) {
+  float h, l;
+  if (!ff_split(v, h, l)) return false;
+  ff_fast_two_sum(h, l, hi, lo);
+  return true;
+}
+
+// An item's mean as the weights use it; ok = false (a zero or tiny mean: all
+// distances 0 gives 0/0 = NaN) sends every weight to the exact path.
+struct FfMean {
+  float hi, lo, rcp;
+  bool ok;
+};
+TS_HD FfMean ts_ff_mean(double mean) {
+  FfMean a;
+  a.ok = ff_split_rn(mean, a.hi, a.lo) && a.hi < 0x1p+120f;
+  a.rcp = a.ok ? TS_FDIV(1.0f, a.hi) : 0.0f;
+  return a;
+}
+
+// The weight of distance d_hi + d_lo (the high part rounded to nearest; both
+// 0 for a zero distance); false: undecided.
+TS_HD bool ts_weight_ff_pair(float d_hi, float d_lo, const FfMean &a, const float *tab_ff, float &w) {
+  if (!a.ok) return false;
+  float q_hi, q_lo;
+  {
+    const float q1 = TS_FMUL(d_hi, a.rcp);
+    const float p = TS_FMUL(q1, a.hi);
+    const float pe = TS_FFMA(q1, a.hi, -p);
     float r = TS_FSUB(d_hi, p);
-    r = TS_FSUB(TS_FSUB(TS_FADD(r, d_lo), pe), TS_FMUL(q1, a_lo));
-    const float q2 = TS_FDIV(r, a_hi);
+    r = TS_FSUB(TS_FSUB(TS_FADD(r, d_lo), pe), TS_FMUL(q1, a.lo));
+    const float q2 = TS_FMUL(r, a.rcp);
     ff_fast_two_sum(q1, q2, q_hi, q_lo);
   }
   if (!(q_hi >= 0.0f && q_hi <= 80.0f)) return false;
@@ -558,6 +589,12 @@ TS_HD bool ts_weight_ff(double d, double mean, const float *tab_ff, float &w) {
   const int32_t m = ki >> 6;  // w = f * 2^m, normal for q <= 80
   w = TS_FMUL(f, bits_flt((uint32_t)(m + 127) << 23));
   return true;
+}
+
+TS_HD bool ts_weight_ff(double d, double mean, const float *tab_ff, float &w) {
+  float d_hi = 0.0f, d_lo = 0.0f;
+  if (dbl_bits(d) != 0 && !ff_split_rn(d, d_hi, d_lo)) return false;
+  return ts_weight_ff_pair(d_hi, d_lo, ts_ff_mean(mean), tab_ff, w);
 }
 
 // units * 2^qe as the bits of a double, exactly (units < 2^53, normal

@@ -77,6 +77,18 @@ __device__ __forceinline__ int modi(int a, int b) {
   return r < 0 ? r + b : r;
 }
 
+// a in [-n, 2n) wrapped into [0, n): every tree point and its tiling mirrors
+// lie there (the mirror bands are 5% of a side).
+__device__ __forceinline__ int wrap1(int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); }
+
+// (x, y) of a pixel index below 2^28: y = p / W by the host's multiplier
+// (SessionDev::w_mul, exact), not an integer division.
+__device__ __forceinline__ void pixel_xy(const SessionDev &s, uint32_t p, int &x, int &y) {
+  const uint32_t q = (uint32_t)(((uint64_t)p * s.w_mul) >> s.w_sh);
+  y = (int)q;
+  x = (int)(p - q * s.W);
+}
+
 // Tree membership of an output-plane point, tiling mirrors included
 // (flush_resolved, ms.rs:296-331).
 __device__ __forceinline__ bool occupied(const SessionDev &s, int x, int y) {
@@ -228,6 +240,11 @@ __device__ __forceinline__ double neighbour_dist_near(const SessionDev &s, int p
 __device__ __forceinline__ unsigned long long exact_units(const SessionDev &s, int dx, int dy) {
   return ((unsigned long long)(uint32_t)(dx * dx) << s.exact_sx) + ((unsigned long long)(uint32_t)(dy * dy) << s.exact_sy);
 }
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
 __device__ __forceinline__ unsigned long long warp_sum_units(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -325,7 +342,8 @@ __device__ __forceinline__ void knn_walk_body(const SessionDev &s, const StageDe
   const uint32_t nb = b.i1 - b.i0;
   for (uint32_t local = vb * kWalkWarps + (threadIdx.x >> 5); local < nb; local += vg * kWalkWarps) {
     const uint32_t pixel = st.items[b.i0 + local];
-    const int px = (int)(pixel % s.W), py = (int)(pixel / s.W);
+    int px, py;
+    pixel_xy(s, pixel, px, py);
     int32_t *nbo = b.nbuf + (size_t)local * s.k;
     const uint32_t n_tree = item_nres(b, b.i0 + local);
     uint32_t count = 0;
@@ -654,7 +672,8 @@ __device__ uint32_t knn_exhaustive_item(const SessionDev &s, const StageDev &st,
                                         ExhShared &sh, unsigned long long *all, uint32_t cap, bool with_mean,
                                         bool use_grid, bool mean_here) {
   const uint32_t pixel = st.items[b.i0 + local];
-  const int px = (int)(pixel % s.W), py = (int)(pixel / s.W);
+  int px, py;
+  pixel_xy(s, pixel, px, py);
   const uint32_t k = s.k;
   const uint32_t n_res = item_nres(b, b.i0 + local);
   auto d2of = [&](int x, int y) -> uint32_t {
@@ -960,24 +979,25 @@ __device__ __forceinline__ void mean_body(const SessionDev &s, const BatchDev &b
 // ---------------------------------------------------------------------------
 // resolve: warp per item.
 // ---------------------------------------------------------------------------
-// Per-warp shared memory: one 16-byte record per neighbour
-// {offset, own pattern texel, target-guide texel, weight bits}, then the
-// candidates {x | y<<16} and {map | neg flag | source index << 16}.
+// Per-item shared memory: one 16-byte record per neighbour {its texel offset
+// on the padded planes (dy * ppitch + dx), own pattern texel, target-guide
+// texel, weight bits}, its packed offset, and the candidates {x | y<<16,
+// map | neg flag | source index << 16}.
 struct WarpSmem {
   uint4 *nbr;
-  uint32_t *cxy, *caux;
+  uint2 *cand;
   float *term;   // candidate 0's neighbour terms
-  int32_t *lin;  // neighbour offsets as texel offsets on the padded planes (dy * ppitch + dx)
+  int32_t *off;  // packed neighbour offsets
 };
 
 __device__ __forceinline__ size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 
 __host__ __device__ __forceinline__ size_t warp_smem_bytes(uint32_t k, uint32_t m) {
   const size_t kk = k ? k : 1;
-  size_t b = kk * 16;                            // nbr
-  b += (((kk + m) * 4 + 15) & ~(size_t)15) * 2;  // cxy, caux
-  b += (kk * 4 + 15) & ~(size_t)15;              // term
-  b += (kk * 4 + 15) & ~(size_t)15;              // lin
+  size_t b = kk * 16;                        // nbr
+  b += ((kk + m) * 8 + 15) & ~(size_t)15;    // cand
+  b += (kk * 4 + 15) & ~(size_t)15;          // term
+  b += (kk * 4 + 15) & ~(size_t)15;          // off
   return b;
 }
 
@@ -987,17 +1007,24 @@ __device__ __forceinline__ WarpSmem carve(unsigned char *base, uint32_t k, uint3
   unsigned char *p = base;
   w.nbr = (uint4 *)p;
   p += kk * 16;
-  w.cxy = (uint32_t *)p;
-  p += align16((kk + m) * 4);
-  w.caux = (uint32_t *)p;
-  p += align16((kk + m) * 4);
+  w.cand = (uint2 *)p;
+  p += align16((kk + m) * 8);
   w.term = (float *)p;
   p += align16(kk * 4);
-  w.lin = (int32_t *)p;
+  w.off = (int32_t *)p;
   return w;
 }
 
 constexpr uint32_t kAuxNeg = 0x8000u;  // random candidate: neighbourhood c + (p - n)
+
+// Random candidate t of an item's list as a candidate record.
+__device__ __forceinline__ uint2 random_candidate(const SessionDev &s, uint2 v, uint32_t t) {
+  v = use_rcand(s, v);
+  return make_uint2(v.x, v.y | kAuxNeg | (t << 16));
+}
+__device__ __forceinline__ uint2 random_candidate(const SessionDev &s, const uint2 *rc, uint32_t t) {
+  return random_candidate(s, __ldg(&rc[t]), t);
+}
 
 __device__ __forceinline__ uint32_t texel(const uint32_t *lv, const MapDesc &md, int x, int y) {
   if ((unsigned)x < md.w && (unsigned)y < md.h) return __ldg(&lv[(size_t)y * md.w + x]);
@@ -1060,7 +1087,8 @@ __device__ __forceinline__ bool candidate_cost(const SessionDev &s, const StageD
       gt[u] = kOutside;
       if (j0 + u < nk) {
         nr[u] = w.nbr[j0 + u];
-        const int qx = cx + sg * off_dx((int32_t)nr[u].x), qy = cy + sg * off_dy((int32_t)nr[u].x);
+        const int32_t o = w.off[j0 + u];
+        const int qx = cx + sg * off_dx(o), qy = cy + sg * off_dy(o);
         if ((unsigned)qx < md.w && (unsigned)qy < md.h) t[u] = __ldg(&lv[(size_t)qy * md.w + qx]);
         if (kG && s.guided && (unsigned)qx < gd.w && (unsigned)qy < gd.h) gt[u] = __ldg(&gv[(size_t)qy * gd.w + qx]);
       }
@@ -1080,17 +1108,14 @@ __device__ __forceinline__ bool candidate_cost(const SessionDev &s, const StageD
 
 // The same on the padded images, for items whose neighbour offsets all lie
 // within kPad: no bounds checks, gathers issued four neighbours ahead.
+// centre: texel index of the candidate's centre on the padded planes.
 template <bool kGuided, bool kOpaque>
-__device__ __forceinline__ bool candidate_cost_padded_v(const SessionDev &s, const StageDev &st, const WarpSmem &w,
-                                                      const float *lc, const float *lg, uint32_t nk, uint32_t cxy,
-                                                      uint32_t aux, float bound, float &out) {
-  const uint32_t map = aux & 0x7fffu;
-  const int sg = (aux & kAuxNeg) ? -1 : 1;
-  const MapDesc md = s.maps[map];
-  const int cx = (int)(cxy & 0xffffu), cy = (int)(cxy >> 16);
-  const size_t poff = md.poff + (size_t)st.level * md.pw * md.ph + (size_t)(cy + kPad) * md.pw + (cx + kPad);
-  const uint32_t *base = s.plevels + poff;
-  const uint32_t *gbase = kGuided ? s.pguides + poff : nullptr;
+__device__ __forceinline__ bool candidate_cost_padded_v(const SessionDev &s, const WarpSmem &w, const float *lc,
+                                                      const float *lg, uint32_t nk, uint64_t centre, bool neg,
+                                                      float bound, float &out) {
+  const int sg = neg ? -4 : 4;  // bytes per texel, signed: the gather address is one multiply-add
+  const char *base = (const char *)(s.plevels + centre);
+  const char *gbase = kGuided ? (const char *)(s.pguides + centre) : nullptr;
   float score = 0.0f;
   uint32_t j = 0;
   for (; j + 4 <= nk; j += 4) {
@@ -1099,9 +1124,9 @@ __device__ __forceinline__ bool candidate_cost_padded_v(const SessionDev &s, con
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       nr[u] = w.nbr[j + u];
-      const int lin = sg * w.lin[j + u];
-      t[u] = __ldg(base + lin);
-      if (kGuided) gt[u] = __ldg(gbase + lin);
+      const int64_t at = (int64_t)sg * (int32_t)nr[u].x;
+      t[u] = __ldg((const uint32_t *)(base + at));
+      if (kGuided) gt[u] = __ldg((const uint32_t *)(gbase + at));
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -1113,9 +1138,9 @@ __device__ __forceinline__ bool candidate_cost_padded_v(const SessionDev &s, con
   }
   for (; j < nk; ++j) {
     const uint4 nr = w.nbr[j];
-    const int lin = sg * w.lin[j];
-    float nps = lut4<kOpaque>(lc, __vabsdiffu4(nr.y, __ldg(base + lin)), 0.0f);
-    if (kGuided) nps = lut4<kOpaque>(lg, __vabsdiffu4(nr.z, __ldg(gbase + lin)), nps);
+    const int64_t at = (int64_t)sg * (int32_t)nr.x;
+    float nps = lut4<kOpaque>(lc, __vabsdiffu4(nr.y, __ldg((const uint32_t *)(base + at))), 0.0f);
+    if (kGuided) nps = lut4<kOpaque>(lg, __vabsdiffu4(nr.z, __ldg((const uint32_t *)(gbase + at))), nps);
     score = __fadd_rn(score, __fmul_rn(nps, __uint_as_float(nr.w)));
   }
   if (score >= bound) return false;
@@ -1126,10 +1151,15 @@ __device__ __forceinline__ bool candidate_cost_padded_v(const SessionDev &s, con
 // The loop in two versions, chosen per stage (a uniform branch).
 template <bool kGuided>
 __device__ __forceinline__ bool candidate_cost_padded(const SessionDev &s, const StageDev &st, const WarpSmem &w,
-                                                      const float *lc, const float *lg, uint32_t nk, uint32_t cxy,
-                                                      uint32_t aux, float bound, float &out) {
-  if (st.opaque) return candidate_cost_padded_v<kGuided, true>(s, st, w, lc, lg, nk, cxy, aux, bound, out);
-  return candidate_cost_padded_v<kGuided, false>(s, st, w, lc, lg, nk, cxy, aux, bound, out);
+                                                      const float *lc, const float *lg, uint32_t nk, uint64_t centre,
+                                                      bool neg, float bound, float &out) {
+  if (st.opaque) return candidate_cost_padded_v<kGuided, true>(s, w, lc, lg, nk, centre, neg, bound, out);
+  return candidate_cost_padded_v<kGuided, false>(s, w, lc, lg, nk, centre, neg, bound, out);
+}
+
+// Texel index of (x, y) of a map's level on the padded planes.
+__device__ __forceinline__ uint64_t padded_centre(const MapDesc &md, uint32_t level, uint32_t cxy) {
+  return md.poff + (uint64_t)level * md.pw * md.ph + (uint64_t)((cxy >> 16) + kPad) * md.pw + ((cxy & 0xffffu) + kPad);
 }
 
 // Per-neighbour set-up of an item: weight (find_best_match, ms.rs:1198-1203,
@@ -1139,11 +1169,16 @@ __device__ __forceinline__ bool candidate_cost_padded(const SessionDev &s, const
 // shift to the centre, kept if valid.  Returns true for a valid candidate.
 // The weight alone, w = (f32) exp(-(d / mean)) (find_best_match,
 // ms.rs:1198-1203): the double-f32 path when it decides, else the exact f64
-// one.
-__device__ __forceinline__ float neighbour_weight(double dj, double avg, const double *tab, const float *tab_ff) {
+// one (about one weight in 2^15; the empty asm keeps the reciprocal from
+// being computed ahead for every item, on an FP64 pipe that takes 18 cycles
+// of an SM per instruction).
+__device__ __forceinline__ float weight_exact(double dj, double avg) {
+  asm volatile("" : "+d"(avg));
+  return __double2float_rn(ts_exp64(-1.0 * ts_div_markstein(dj, avg, __drcp_rn(avg)), g_exp2_64));
+}
+__device__ __forceinline__ float neighbour_weight(double dj, double avg, const float *tab_ff) {
   float wv;
-  if (!ts_weight_ff(dj, avg, tab_ff, wv))
-    wv = __double2float_rn(ts_exp64(-1.0 * ts_div_markstein(dj, avg, __drcp_rn(avg)), tab));
+  if (!ts_weight_ff(dj, avg, tab_ff, wv)) wv = weight_exact(dj, avg);
   return wv;
 }
 
@@ -1166,63 +1201,79 @@ __device__ __forceinline__ void start_pixel(const SessionDev &s, const BatchDev 
 }
 
 // Everything of neighbour_setup but the weight, which the record gets as wv.
+// A neighbour is a tree point, so it or the pixel it mirrors lies in the
+// image (wrap1).
 template <bool kG = true>
 __device__ __forceinline__ bool neighbour_records(const SessionDev &s, const StageDev &st, const BatchDev &b, int px,
                                                   int py, uint32_t j, int32_t off, float wv, const WarpSmem &w,
                                                   uint32_t &cxy, uint32_t &aux, int &maxoff, bool &bad_map) {
-  const int W = (int)s.W, H = (int)s.H;
-  maxoff = max(maxoff, max(abs(off_dx(off)), abs(off_dy(off))));
-  const int nx = px + off_dx(off), ny = py + off_dy(off);
-  int qx = nx, qy = ny;
-  if (s.tiling) {
-    qx = modi(nx, W);
-    qy = modi(ny, H);
-  }
-  const bool inb = (unsigned)qx < s.W && (unsigned)qy < s.H;
-  // colour and state of the neighbour (inb: (qx, qy) is its wrapped point)
-  const int wx = modi(nx, W), wy = modi(ny, H);
+  const int dx = off_dx(off), dy = off_dy(off);
+  maxoff = max(maxoff, max(abs(dx), abs(dy)));
+  const uint32_t p = (uint32_t)wrap1(py + dy, (int)s.H) * s.W + (uint32_t)wrap1(px + dx, (int)s.W);
   uint32_t pat;
   uint4 sv;
-  start_pixel(s, b, (uint32_t)wy * s.W + (uint32_t)wx, inb, pat, sv);
-  if (!inb) pat = kOutside;
+  start_pixel(s, b, p, true, pat, sv);
   uint32_t gpat = 0;
-  if (kG && s.guided) gpat = inb ? __ldg(&s.tguide[(size_t)st.level * s.W * s.H + (size_t)qy * s.W + qx]) : kOutside;
-  w.nbr[j] = make_uint4((uint32_t)off, pat, gpat, __float_as_uint(wv));
-  w.lin[j] = off_dy(off) * (int)s.ppitch + off_dx(off);
+  if (kG && s.guided) gpat = __ldg(&s.tguide[(size_t)st.level * s.W * s.H + p]);
+  w.nbr[j] = make_uint4((uint32_t)(dy * (int)s.ppitch + dx), pat, gpat, __float_as_uint(wv));
+  w.off[j] = off;
   const uint32_t map = sv.z;
   if (map >= s.n_maps) {
     bad_map = true;
     return false;
   }
-  const int ccx = (int)(sv.x & 0xffffu) + (px - nx);
-  const int ccy = (int)(sv.x >> 16) + (py - ny);
+  const int ccx = (int)(sv.x & 0xffffu) - dx;
+  const int ccy = (int)(sv.x >> 16) - dy;
   if (!coord_valid(s, s.maps[map], ccx, ccy)) return false;
   cxy = (uint32_t)ccx | ((uint32_t)ccy << 16);
   aux = map | (j << 16);
   return true;
 }
 
+// The weight of an item's neighbour j at offset off (fm = ts_ff_mean(avg)).
+// Sessions with exact sums and equal sides: the distance is dx^2 + dy^2 units,
+// an f32 pair (below 2^24 units a single f32).
+__device__ __forceinline__ float item_weight(const SessionDev &s, const BatchDev &b, uint32_t local, uint32_t nb,
+                                             uint32_t j, int32_t off, double avg, const FfMean &fm,
+                                             const float *tab_ff) {
+  float d_hi = 0.0f, d_lo = 0.0f, wv;
+  bool split = true;
+  if (s.exact_sum && (s.exact_sx | s.exact_sy) == 0u) {
+    const int dx = off_dx(off), dy = off_dy(off);
+    const uint32_t u = (uint32_t)(dx * dx + dy * dy);
+    const float hi = (float)u;
+    d_hi = __fmul_rn(hi, s.exact_qf);
+    d_lo = __fmul_rn((float)(int32_t)(u - (uint32_t)hi), s.exact_qf);
+  } else {
+    const double d = s.exact_sum ? bits_dbl(ts_units_bits(exact_units(s, off_dx(off), off_dy(off)), s.exact_qe))
+                                 : b.dist[(size_t)j * nb + local];
+    split = dbl_bits(d) == 0 || ff_split_rn(d, d_hi, d_lo);
+  }
+  if (!(split && ts_weight_ff_pair(d_hi, d_lo, fm, tab_ff, wv)))
+    wv = weight_exact(s.exact_sum ? exact_dist(s, off) : b.dist[(size_t)j * nb + local], avg);
+  return wv;
+}
+
 template <bool kG = true>
 __device__ __forceinline__ bool neighbour_setup(const SessionDev &s, const StageDev &st, const BatchDev &b,
                                                 uint32_t local, uint32_t nb, int px, int py, uint32_t j, int32_t off,
-                                                double avg, const double *tab, const float *tab_ff,
+                                                double avg, const FfMean &fm, const float *tab_ff,
                                                 const WarpSmem &w, uint32_t &cxy, uint32_t &aux, bool &nan_w,
                                                 int &maxoff, bool &bad_map) {
-  const double d = s.exact_sum ? exact_dist(s, off) : b.dist[(size_t)j * nb + local];
-  const float wv = neighbour_weight(d, avg, tab, tab_ff);
+  const float wv = item_weight(s, b, local, nb, j, off, avg, fm, tab_ff);
   nan_w |= (wv != wv);
   return neighbour_records<kG>(s, st, b, px, py, j, off, wv, w, cxy, aux, maxoff, bad_map);
 }
 
 // Candidate 0's exact score (better_match, ms.rs:1225-1288, with no bound):
 // lane j of a group of G lanes (a warp, or a CTA's warp) computes the terms
-// nps_j * w_j of neighbours j, j + G, ..., lane 0 sums them in order; every
-// lane returns the sum.
+// nps_j * w_j of neighbours j, j + G, ..., then every lane sums them in
+// order.
 template <int G, bool kG = true>
 __device__ __forceinline__ float candidate0_score(const SessionDev &s, const StageDev &st, const WarpSmem &w,
                                                   const float *lc, const float *lg, uint32_t nk, int gl,
                                                   uint32_t gmask) {
-  const uint32_t cxy0 = w.cxy[0], aux0 = w.caux[0];
+  const uint32_t cxy0 = w.cand[0].x, aux0 = w.cand[0].y;
   const uint32_t map = aux0 & 0x7fffu;
   const bool neg = (aux0 & kAuxNeg) != 0;
   const MapDesc md = s.maps[map];
@@ -1230,7 +1281,7 @@ __device__ __forceinline__ float candidate0_score(const SessionDev &s, const Sta
   const int cx = (int)(cxy0 & 0xffffu), cy = (int)(cxy0 >> 16);
   for (uint32_t j = gl; j < nk; j += G) {
     const uint4 nr = w.nbr[j];
-    int dx = off_dx((int32_t)nr.x), dy = off_dy((int32_t)nr.x);
+    int dx = off_dx(w.off[j]), dy = off_dy(w.off[j]);
     if (neg) {
       dx = -dx;
       dy = -dy;
@@ -1248,31 +1299,36 @@ __device__ __forceinline__ float candidate0_score(const SessionDev &s, const Sta
   }
   __syncwarp(gmask);
   float sc = 0.0f;
-  if (gl == 0)
-    for (uint32_t j = 0; j < nk; ++j) sc = __fadd_rn(sc, w.term[j]);
-  return __shfl_sync(gmask, sc, 0, G);
+  uint32_t j = 0;
+  for (; j + 4 <= nk; j += 4) {
+    const float4 t4 = *(const float4 *)(w.term + j);
+    sc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sc, t4.x), t4.y), t4.z), t4.w);
+  }
+  for (; j < nk; ++j) sc = __fadd_rn(sc, w.term[j]);
+  return sc;
 }
 
 // The reference's sequential find_best_match (ms.rs:1184-1221), for stages or
-// items with non-finite costs, where early exit and argmin need its exact
-// comparison sequence.  One thread.
+// items with non-finite or negative costs, where early exit and argmin need
+// its exact comparison sequence.  One thread.
 template <bool kG = true>
 __device__ void sequential_best(const SessionDev &s, const StageDev &st, const WarpSmem &w, const float *lc,
                                 const float *lg, uint32_t nk, uint32_t nc, float &best_s, uint32_t &best_i) {
   best_s = FLT_MAX;
   best_i = 0;
   for (uint32_t c = 0; c < nc; ++c) {
-    const uint32_t aux = w.caux[c];
+    const uint2 cd = w.cand[c];
+    const uint32_t aux = cd.y;
     const uint32_t map = aux & 0x7fffu;
     const bool neg = (aux & kAuxNeg) != 0;
     const MapDesc md = s.maps[map];
     const uint32_t *lv = s.levels + md.off + (size_t)st.level * md.w * md.h;
-    const int cx = (int)(w.cxy[c] & 0xffffu), cy = (int)(w.cxy[c] >> 16);
+    const int cx = (int)(cd.x & 0xffffu), cy = (int)(cd.x >> 16);
     float score = 0.0f;
     bool better = true;
     for (uint32_t j = 0; j < nk; ++j) {
       const uint4 nr = w.nbr[j];
-      int dx = off_dx((int32_t)nr.x), dy = off_dy((int32_t)nr.x);
+      int dx = off_dx(w.off[j]), dy = off_dy(w.off[j]);
       if (neg) {
         dx = -dx;
         dy = -dy;
@@ -1327,9 +1383,10 @@ __device__ __forceinline__ void commit_item(const SessionDev &s, const StageDev 
     s.rscore[pos] = r.score;
     if (s.rank) return;  // k-NN made ahead: k_tree_append entered the point already
     s.resolved[pos] = p;
-    const uint32_t x = p % s.W, y = p / s.W;
+    int x, y;
+    pixel_xy(s, p, x, y);
     atomicOr(&s.occ[(size_t)y * s.wpr + (x >> 5)], 1u << (x & 31));
-    add_cell_point(s, (int)x, (int)y);
+    add_cell_point(s, x, y);
     if (s.tiling && (r.flags & kResMirrors)) {
       atomicOr(&s.mir[(size_t)y * s.wpr + (x >> 5)], 1u << (x & 31));
       // the tree's mirror copies (flush_resolved, ms.rs:306-328)
@@ -1349,9 +1406,9 @@ __device__ __forceinline__ void commit_item(const SessionDev &s, const StageDev 
 // (b.fused_commit: no item of the batch is in the tree, so no other item
 // reads its pixel, state or bit during the batch), else kept for k_commit.
 __device__ __forceinline__ void emit_result(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t local,
-                                            const Result &r) {
+                                            const Result &r, bool count_evals = true) {
   if (b.fused_commit) {
-    commit_item(s, st, b, local, r);
+    commit_item(s, st, b, local, r, count_evals);
   } else {
     b.res[local] = r;
     if (b.defer_tag && r.cmap < s.n_maps && r.pixel < s.W * s.H) {
@@ -1372,17 +1429,17 @@ __device__ __forceinline__ void emit_result(const SessionDev &s, const StageDev 
 // index for random ones), score.
 __device__ void write_result(const SessionDev &s, const StageDev &st, const WarpSmem &w, const BatchDev &b,
                              uint32_t local, uint32_t pixel, int px, int py, bool is_new, uint32_t nc, float best_s,
-                             uint32_t best_i) {
-  const uint32_t aux = w.caux[best_i];
+                             uint32_t best_i, bool count_evals = true) {
+  const uint32_t aux = w.cand[best_i].y;
   const uint32_t map = aux & 0x7fffu;
-  const uint32_t cxy = w.cxy[best_i];
+  const uint32_t cxy = w.cand[best_i].x;
   uint32_t idp;
   if (aux & kAuxNeg) {
     idp = (cxy >> 16) * s.maps[map].w + (cxy & 0xffffu);
   } else {
     const uint32_t j = aux >> 16;
-    const int32_t off = (int32_t)w.nbr[j].x;
-    const int wx = modi(px + off_dx(off), (int)s.W), wy = modi(py + off_dy(off), (int)s.H);
+    const int32_t off = w.off[j];
+    const int wx = wrap1(px + off_dx(off), (int)s.W), wy = wrap1(py + off_dy(off), (int)s.H);
     uint32_t unused;
     uint4 sv;
     start_pixel(s, b, (uint32_t)wy * s.W + (uint32_t)wx, false, unused, sv);
@@ -1397,7 +1454,7 @@ __device__ void write_result(const SessionDev &s, const StageDev &st, const Warp
   r.flags = (is_new ? kResAppend : 0u) | kResMirrors;
   r.score = best_s;
   r.ncand = nc;
-  emit_result(s, st, b, local, r);
+  emit_result(s, st, b, local, r, count_evals);
 }
 
 // Result for an item with no resolved neighbour: resolve_at_random with the
@@ -1444,18 +1501,28 @@ __device__ void write_bad_result(const SessionDev &s, const StageDev &st, const 
   emit_result(s, st, b, local, r);
 }
 
-// kLean: sessions without guides only (the guide terms compiled out, which
-// lets the multi-session kernel run more blocks per SM).
+// kLean: sessions without guides only (the guide terms compiled out).  Eight
+// blocks of four warps per SM at 64 registers: nine at 56 ran the last stage
+// of the remix in 0.95 against 0.82 ms (more items wait behind a launch's
+// slowest ones).
+//
+// What bounds it: a step's warps take 3 to 8 items each, one after another,
+// so the latency of an item (dependent gathers, then the issue slots its
+// warps share) and the launch's tail; DRAM carries a few percent.  50 neighbours propose 3 to 8 different coherence candidates
+// on the benchmark workloads, and the first of them costs exactly 0 for 12 to
+// 49% of the items, which ends the item.  Distances stay in integers and f32
+// pairs: an f64 instruction takes 18 cycles of an SM.  Repeats are found with
+// a 32-bit __match_any_sync: 2 cycles of the SM per distinct value, 4 with 64
+// bits (an atomicMin per lane into a shared hash table: 1 per lane of a slot,
+// and most lanes share one).  Resolves of 2048^2 tiling: 25.8 -> 21.5 ms.
 template <bool kLean>
 __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t vb,
                                              uint32_t vg) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double tab[64];
   __shared__ float tab_ff[128];
   float *lc = (float *)smem;
   float *lg = lc + 256;
   for (int i = threadIdx.x; i < 512; i += blockDim.x) lc[i] = st.lut[i];
-  if (threadIdx.x < 64) tab[threadIdx.x] = g_exp2_64[threadIdx.x];
   tab_ff[threadIdx.x] = g_exp2_ff[threadIdx.x];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
@@ -1463,31 +1530,38 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
   __syncthreads();
   const uint32_t nb = b.i1 - b.i0;
   const uint32_t grid_warps = vg * kResolveWarps;
-  // the next item of this warp: the grid stride, or (BatchDev::work_ctr)
-  // the next one nobody has taken once every warp has had its first
-  auto next_item = [&](uint32_t cur) -> uint32_t {
+  uint32_t evals = 0;  // candidates of the items committed here, added once at the end
+  // The next item of this warp: the grid stride, or (BatchDev::work_ctr) the
+  // next one nobody has taken once every warp has had its first (asked for
+  // at an item's end: asked for at its start, the item waits behind a slow
+  // one; remix 0.95 against 0.87 ms in the last stage).  One counter serves
+  // an item per 0.95 ns at best, so there are kWorkCtrs of them (no more than
+  // blocks), each for the items of one residue; a block uses its own.
+  const uint32_t ctrs = min(kWorkCtrs, vg), res = vb % ctrs;
+  const uint32_t res_warps = ((vg - res + ctrs - 1) / ctrs) * kResolveWarps;
+  uint32_t local = vb * kResolveWarps + warp;
+  if (b.work_ctr) local = (vb / ctrs * kResolveWarps + warp) * ctrs + res;
+  auto take = [&](uint32_t cur) -> uint32_t {
     if (!b.work_ctr) return cur + grid_warps;
     uint32_t v = 0;
-    if (lane == 0) v = atomicAdd(b.work_ctr, 1u) + grid_warps;
+    if (lane == 0) v = (atomicAdd(b.work_ctr + res * kWorkCtrStride, 1u) + res_warps) * ctrs + res;
     return __shfl_sync(0xffffffffu, v, 0);
   };
-  for (uint32_t local = vb * kResolveWarps + warp; local < nb; local = next_item(local)) {
+  for (; local < nb; local = take(local)) {
     const uint32_t item = b.i0 + local;
     const uint32_t pixel = st.items[item];
-    const int px = (int)(pixel % s.W), py = (int)(pixel / s.W);
-    const bool is_new = item >= st.redo;
     const uint32_t nk = s.k ? b.ncnt[local] : 0u;
-    Result r;
-    r.pixel = pixel;
-    r.ncand = 0;
     if (nk == 0) {
       // no resolved neighbours: resolve_at_random with the stage seed, kept
       // in the resolved list without tiling mirrors (ms.rs:1002-1010, 473)
       if (lane == 0) write_random_result(s, st, b, local, pixel);
       continue;
     }
+    int px, py;
+    pixel_xy(s, pixel, px, py);
     const int32_t *nbo = b.nbuf + (size_t)local * s.k;
     const double avg = b.mean[local];
+    const FfMean fm = ts_ff_mean(avg);
     // neighbours: offsets, weights, own pattern, coherence candidates.
     // With `dedupe`, a coherence candidate equal to an earlier one (same
     // source and map) is left out: its cost equals the earlier one's, so it
@@ -1504,30 +1578,36 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
         const uint32_t j = j0 + lane;
         bool valid = false;
         uint32_t cxy = 0, aux = 0;
-        if (j < nk)
-          valid = neighbour_setup<!kLean>(s, st, b, local, nb, px, py, j, nbo[j], avg, tab, tab_ff, w, cxy, aux, nan_w,
-                                  maxoff, bad_map);
+        if (j < nk) {
+          const int32_t off = nbo[j];
+          const float wv = item_weight(s, b, local, nb, j, off, avg, fm, tab_ff);
+          nan_w |= (wv != wv);
+          valid = neighbour_records<!kLean>(s, st, b, px, py, j, off, wv, w, cxy, aux, maxoff, bad_map);
+        }
         bool keep = valid;
         if (dedupe) {
-          const unsigned long long key =
-              valid ? (((unsigned long long)(aux & 0x7fffu) << 32) | cxy) : ((1ull << 63) | (unsigned long long)lane);
-          if (__match_any_sync(0xffffffffu, key) & lt) keep = false;  // a lower lane holds it
-          for (uint32_t i = 0; keep && i < ncoh; ++i)
-            if (w.cxy[i] == cxy && (w.caux[i] & 0x7fffu) == (aux & 0x7fffu)) keep = false;
+          const uint32_t map = aux & 0x7fffu, vm = __ballot_sync(0xffffffffu, valid);
+          uint32_t same;  // lanes with the same source and map
+          if (s.n_maps <= 16)
+            same = __match_any_sync(0xffffffffu, (cxy & 0x3fffu) | ((cxy >> 16) << 14) | (map << 28));
+          else
+            same = __match_any_sync(0xffffffffu, ((unsigned long long)map << 32) | cxy);
+          if (same & vm & lt) keep = false;  // a lower lane holds it
+          for (uint32_t i = 0; i < ncoh; ++i) {
+            const uint2 c1 = w.cand[i];
+            if (c1.x == cxy && ((c1.y ^ aux) & 0x7fffu) == 0u) keep = false;
+          }
         }
         ncoh_all += __popc(__ballot_sync(0xffffffffu, valid));
         const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-        if (keep) {
-          const uint32_t slot = ncoh + __popc(bal & lt);
-          w.cxy[slot] = cxy;
-          w.caux[slot] = aux;
-        }
+        if (keep) w.cand[ncoh + __popc(bal & lt)] = make_uint2(cxy, aux);
         ncoh += __popc(bal);
         __syncwarp();
       }
     };
     coherence(!st.slow_lut);
-    if (!st.slow_lut && __any_sync(0xffffffffu, nan_w)) coherence(false);
+    const bool nan_any = __any_sync(0xffffffffu, nan_w);
+    if (!st.slow_lut && nan_any) coherence(false);
     if (__any_sync(0xffffffffu, bad_map)) {
       // the reference panics on this index; record the error and leave the
       // pixel untouched (commit skips results with an invalid map)
@@ -1536,14 +1616,9 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
     }
     // random candidates after the coherence ones
     const uint2 *rc = st.rcand + (size_t)item * s.m;
-    for (uint32_t t = lane; t < s.m; t += kWarp) {
-      const uint2 v = use_rcand(s, rc[t]);
-      w.cxy[ncoh + t] = v.x;
-      w.caux[ncoh + t] = v.y | kAuxNeg | (t << 16);
-    }
-    const bool slow = st.slow_lut || __any_sync(0xffffffffu, nan_w);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) maxoff = max(maxoff, __shfl_xor_sync(0xffffffffu, maxoff, o));
+    for (uint32_t t = lane; t < s.m; t += kWarp) w.cand[ncoh + t] = random_candidate(s, rc, t);
+    const bool slow = st.slow_lut || nan_any;
+    maxoff = __reduce_max_sync(0xffffffffu, maxoff);
     const bool padded = maxoff <= kPad && !s.guide_dims_differ;
     __syncwarp();
     const uint32_t nc = ncoh + s.m;
@@ -1551,45 +1626,46 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
     uint32_t best_i = 0;
     if (!slow) {
       // candidate 0 first: its terms on all lanes, their in-order sum on
-      // lane 0; it wins ties with every later candidate, so the rest run
-      // against min(S_0, f32::MAX) from the start
-      {
-        const float s0 = candidate0_score<kWarp, !kLean>(s, st, w, lc, lg, nk, lane, 0xffffffffu);
-        if (s0 < best_s) best_s = s0;
-      }
-      for (uint32_t base = 1; base < nc; base += kWarp) {
+      // every lane; it wins ties with every later candidate, so the rest run
+      // against min(S_0, f32::MAX) from the start, and a cost of 0 ends the
+      // item (no term is negative)
+      const float s0 = candidate0_score<kWarp, !kLean>(s, st, w, lc, lg, nk, lane, 0xffffffffu);
+      if (s0 < best_s) best_s = s0;
+      for (uint32_t base = 1; base < nc && best_s > 0.0f; base += kWarp) {
         const uint32_t c = base + lane;
-        float sc = 0.0f;
-        bool alive = false;
+        float sc = __builtin_huge_valf(), v = 0.0f;
         if (c < nc) {
-          if (!padded)
-            alive = candidate_cost<!kLean>(s, st, w, lc, lg, nk, w.cxy[c], w.caux[c], best_s, sc);
-          else if (!kLean && s.guided)
-            alive = candidate_cost_padded<true>(s, st, w, lc, lg, nk, w.cxy[c], w.caux[c], best_s, sc);
-          else
-            alive = candidate_cost_padded<false>(s, st, w, lc, lg, nk, w.cxy[c], w.caux[c], best_s, sc);
-        }
-        float v = alive ? sc : __int_as_float(0x7f800000);
-        uint32_t idx = alive ? c : 0xffffffffu;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-          const uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
-          if (ov < v || (ov == v && oi < idx)) {
-            v = ov;
-            idx = oi;
+          const uint2 cd = w.cand[c];
+          bool alive;
+          if (!padded) {
+            alive = candidate_cost<!kLean>(s, st, w, lc, lg, nk, cd.x, cd.y, best_s, v);
+          } else {
+            const uint64_t centre = padded_centre(s.maps[cd.y & 0x7fffu], st.level, cd.x);
+            const bool neg = (cd.y & kAuxNeg) != 0;
+            if (!kLean && s.guided)
+              alive = candidate_cost_padded<true>(s, st, w, lc, lg, nk, centre, neg, best_s, v);
+            else
+              alive = candidate_cost_padded<false>(s, st, w, lc, lg, nk, centre, neg, best_s, v);
           }
+          if (alive) sc = v;
         }
-        if (idx != 0xffffffffu && v < best_s) {
-          best_s = v;
-          best_i = idx;
+        // the round's lowest cost, its first lane
+        const float lo = warp_min(sc);
+        if (lo < best_s) {
+          best_s = lo;
+          best_i = base + __ffs(__ballot_sync(0xffffffffu, sc == lo)) - 1;
         }
       }
     } else if (lane == 0) {
       sequential_best<!kLean>(s, st, w, lc, lg, nk, nc, best_s, best_i);
     }
-    if (lane == 0) write_result(s, st, w, b, local, pixel, px, py, is_new, ncoh_all + s.m, best_s, best_i);
+    if (lane == 0)
+      write_result(s, st, w, b, local, pixel, px, py, item >= st.redo, ncoh_all + s.m, best_s, best_i, false);
+    evals += ncoh_all + s.m;
+    __syncwarp();  // the records and candidates are rebuilt for the next item
   }
+  // (a batch left to a later commit is counted there)
+  if (b.fused_commit && lane == 0 && evals) atomicAdd(s.evals, (unsigned long long)evals);
 }
 
 
@@ -1609,7 +1685,6 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
                                                   uint32_t vb, uint32_t vg) {
   constexpr int NW = T / 32;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double tab[64];
   __shared__ float tab_ff[128];
   __shared__ uint32_t wcnt[NW];
   __shared__ float red_s[NW];
@@ -1619,7 +1694,6 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
   float *lc = (float *)smem;
   float *lg = lc + 256;
   for (int i = threadIdx.x; i < 512; i += T) lc[i] = st.lut[i];
-  for (int i = threadIdx.x; i < 64; i += T) tab[i] = g_exp2_64[i];
   for (int i = threadIdx.x; i < 128; i += T) tab_ff[i] = g_exp2_ff[i];
   const WarpSmem w = carve(smem + 2048, s.k, s.m);
   float *term = (float *)(smem + 2048 + warp_smem_bytes(s.k, s.m));
@@ -1630,7 +1704,8 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
   for (uint32_t local = vb; local < nb; local += vg) {
     const uint32_t item = b.i0 + local;
     const uint32_t pixel = st.items[item];
-    const int px = (int)(pixel % s.W), py = (int)(pixel / s.W);
+    int px, py;
+    pixel_xy(s, pixel, px, py);
     const bool is_new = item >= st.redo;
     const uint32_t nk = s.k ? b.ncnt[local] : 0u;
     if (nk == 0) {
@@ -1644,6 +1719,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
     __syncthreads();
     const int32_t *nbo = b.nbuf + (size_t)local * s.k;
     const double avg = b.mean[local];
+    const FfMean fm = ts_ff_mean(avg);
     bool nan_w = false, bad_map = false;
     int maxoff = 0;
     uint32_t ncoh = 0;
@@ -1652,7 +1728,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
       bool valid = false;
       uint32_t cxy = 0, aux = 0;
       if (j < nk)
-        valid = neighbour_setup(s, st, b, local, nb, px, py, j, nbo[j], avg, tab, tab_ff, w, cxy, aux, nan_w,
+        valid = neighbour_setup(s, st, b, local, nb, px, py, j, nbo[j], avg, fm, tab_ff, w, cxy, aux, nan_w,
                                 maxoff, bad_map);
       // order-preserving compaction of the valid coherence candidates
       const uint32_t bal = __ballot_sync(0xffffffffu, valid);
@@ -1666,8 +1742,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
       }
       if (valid) {
         const uint32_t slot = base + __popc(bal & lt);
-        w.cxy[slot] = cxy;
-        w.caux[slot] = aux;
+        w.cand[slot] = make_uint2(cxy, aux);
       }
       ncoh += total;
       __syncthreads();
@@ -1678,8 +1753,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
     const uint2 *rc = st.rcand + (size_t)item * s.m;
     for (uint32_t t = tid; t < s.m; t += T) {
       const uint2 v = use_rcand(s, rc[t]);
-      w.cxy[ncoh + t] = v.x;
-      w.caux[ncoh + t] = v.y | kAuxNeg | (t << 16);
+      w.cand[ncoh + t] = make_uint2(v.x, v.y | kAuxNeg | (t << 16));
     }
     __syncthreads();
     if (sh_flags & 2) {
@@ -1699,11 +1773,8 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
       // loads in flight per thread before their terms are formed.
       unsigned long long *cb = (unsigned long long *)(term + (((size_t)nk * nc + 1) & ~(size_t)1));
       for (uint32_t c = tid; c < nc; c += T) {
-        const uint32_t cxy = w.cxy[c], aux = w.caux[c];
-        const MapDesc md = s.maps[aux & 0x7fffu];
-        const unsigned long long off = md.poff + (unsigned long long)st.level * md.pw * md.ph +
-                                       (unsigned long long)((cxy >> 16) + kPad) * md.pw + ((cxy & 0xffffu) + kPad);
-        cb[c] = off | ((aux & kAuxNeg) ? (1ull << 63) : 0ull);
+        const uint32_t cxy = w.cand[c].x, aux = w.cand[c].y;
+        cb[c] = padded_centre(s.maps[aux & 0x7fffu], st.level, cxy) | ((aux & kAuxNeg) ? (1ull << 63) : 0ull);
       }
       __syncthreads();
       const uint32_t total = nc * nk;
@@ -1717,7 +1788,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
             const uint32_t c = i / nk;
             jj[u] = i - c * nk;
             const unsigned long long v = cb[c];
-            const int lin = (v >> 63) ? -w.lin[jj[u]] : w.lin[jj[u]];
+            const int lj = (int32_t)w.nbr[jj[u]].x, lin = (v >> 63) ? -lj : lj;
             const size_t off = (size_t)(v & 0x7fffffffffffffffull) + lin;
             tx[u] = __ldg(s.plevels + off);
             if (s.guided) gx[u] = __ldg(s.pguides + off);
@@ -1741,13 +1812,13 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
       uint32_t c = tid / nk, j = tid - c * nk;
       const uint32_t dc = T / nk, dj = T - dc * nk;
       for (uint32_t i = tid; i < nc * nk; i += T) {
-        const uint32_t cxy = w.cxy[c], aux = w.caux[c];
+        const uint32_t cxy = w.cand[c].x, aux = w.cand[c].y;
         const uint32_t map = aux & 0x7fffu;
         const int sg = (aux & kAuxNeg) ? -1 : 1;
         const MapDesc md = s.maps[map];
         const uint4 nr = w.nbr[j];
-        const int qx = (int)(cxy & 0xffffu) + sg * off_dx((int32_t)nr.x);
-        const int qy = (int)(cxy >> 16) + sg * off_dy((int32_t)nr.x);
+        const int qx = (int)(cxy & 0xffffu) + sg * off_dx(w.off[j]);
+        const int qy = (int)(cxy >> 16) + sg * off_dy(w.off[j]);
         uint32_t t = kOutside;
         if ((unsigned)qx < md.w && (unsigned)qy < md.h)
           t = __ldg(&s.levels[md.off + (size_t)st.level * md.w * md.h + (size_t)qy * md.w + qx]);
@@ -1810,7 +1881,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
     } else if (!slow) {
       // S_0: candidate 0's terms nps_j * w_j in parallel, summed in order
       {
-        const uint32_t cxy0 = w.cxy[0], aux0 = w.caux[0];
+        const uint32_t cxy0 = w.cand[0].x, aux0 = w.cand[0].y;
         const uint32_t map = aux0 & 0x7fffu;
         const bool neg = (aux0 & kAuxNeg) != 0;
         const MapDesc md = s.maps[map];
@@ -1818,7 +1889,7 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
         const int cx = (int)(cxy0 & 0xffffu), cy = (int)(cxy0 >> 16);
         for (uint32_t j = tid; j < nk; j += T) {
           const uint4 nr = w.nbr[j];
-          int dx = off_dx((int32_t)nr.x), dy = off_dy((int32_t)nr.x);
+          int dx = off_dx(w.off[j]), dy = off_dy(w.off[j]);
           if (neg) {
             dx = -dx;
             dy = -dy;
@@ -1847,12 +1918,16 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
       for (uint32_t c = 1 + tid; c < nc; c += T) {
         float sc;
         bool alive;
+        const uint2 cd = w.cand[c];
+        const bool neg = (cd.y & kAuxNeg) != 0;
         if (!padded)
-          alive = candidate_cost(s, st, w, lc, lg, nk, w.cxy[c], w.caux[c], my_s, sc);
+          alive = candidate_cost(s, st, w, lc, lg, nk, cd.x, cd.y, my_s, sc);
         else if (s.guided)
-          alive = candidate_cost_padded<true>(s, st, w, lc, lg, nk, w.cxy[c], w.caux[c], my_s, sc);
+          alive = candidate_cost_padded<true>(s, st, w, lc, lg, nk, padded_centre(s.maps[cd.y & 0x7fffu], st.level, cd.x),
+                                              neg, my_s, sc);
         else
-          alive = candidate_cost_padded<false>(s, st, w, lc, lg, nk, w.cxy[c], w.caux[c], my_s, sc);
+          alive = candidate_cost_padded<false>(s, st, w, lc, lg, nk, padded_centre(s.maps[cd.y & 0x7fffu], st.level, cd.x),
+                                               neg, my_s, sc);
         if (alive) {
           my_s = sc;
           my_i = c;
@@ -2350,14 +2425,16 @@ __global__ void __launch_bounds__(128) k_mean_multi(MultiLaunch ml) {
 // here by every thread of the grid before its own item; this launch's
 // readers of those pixels take their values from pc.b.res instead.
 __global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
-    k_resolve(SessionDev s, StageDev st, BatchDev b, const __grid_constant__ PendingCommit pc) {
+    k_resolve(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+              const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
   pdl_enter();
   if (pc.n) pending_commit(s, pc);
   resolve_body<false>(s, st, b, blockIdx.x, gridDim.x);
 }
 // Sessions without guides (the guide terms compiled out).
-__global__ void __launch_bounds__(kResolveWarps *kWarp, 9)
-    k_resolve_lean(SessionDev s, StageDev st, BatchDev b, const __grid_constant__ PendingCommit pc) {
+__global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
+    k_resolve_lean(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+                   const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
   pdl_enter();
   if (pc.n) pending_commit(s, pc);
   resolve_body<true>(s, st, b, blockIdx.x, gridDim.x);
@@ -2367,8 +2444,8 @@ __global__ void __launch_bounds__(kResolveWarps *kWarp, 8) k_resolve_multi(Multi
   const SegView v = find_segment(ml);
   resolve_body<false>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
 }
-// Segments of sessions without guides: 56 registers, nine blocks per SM.
-__global__ void __launch_bounds__(kResolveWarps *kWarp, 9) k_resolve_multi_lean(MultiLaunch ml) {
+// Segments of sessions without guides.
+__global__ void __launch_bounds__(kResolveWarps *kWarp, 8) k_resolve_multi_lean(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
   resolve_body<true>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
@@ -2376,7 +2453,8 @@ __global__ void __launch_bounds__(kResolveWarps *kWarp, 9) k_resolve_multi_lean(
 
 template <int T, bool kFull>
 __global__ void __launch_bounds__(T)
-    k_resolve_team(SessionDev s, StageDev st, BatchDev b, const __grid_constant__ PendingCommit pc) {
+    k_resolve_team(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+                   const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
   pdl_enter();
   if (pc.n) pending_commit(s, pc);
   resolve_team_body<T, kFull>(s, st, b, blockIdx.x, gridDim.x);
@@ -2409,10 +2487,10 @@ __device__ __forceinline__ void setup_bar() {
 // T = 256, or 512 for steps of at most one item per SM, where the extra
 // warps shorten each item's latency-bound k-NN and gathers.
 template <int T>
-__global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st, BatchDev b, uint32_t cap) {
+__global__ void __launch_bounds__(T) k_step_team_full(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+                     const __grid_constant__ BatchDev b, uint32_t cap) {
   constexpr int NW = T / kWarp, TS = T - kWarp;
   __shared__ ExhShared sh;
-  __shared__ double tab[64];
   __shared__ float tab_ff[128];
   __shared__ uint32_t wcnt[NW];
   __shared__ float red_s[NW];
@@ -2434,7 +2512,8 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
     __syncthreads();  // sh.dist, sh.nbo; the key buffer is free again
     const uint32_t item = b.i0 + local;
     const uint32_t pixel = st.items[item];
-    const int px = (int)(pixel % s.W), py = (int)(pixel / s.W);
+    int px, py;
+    pixel_xy(s, pixel, px, py);
     const bool is_new = item >= st.redo;
     if (nk == 0) {
       if (tid == 0) write_random_result(s, st, b, local, pixel);
@@ -2470,7 +2549,6 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
         const int i = t + u * TS;
         lreg[u] = i < 512 ? st.lut[i] : 0.0f;
       }
-      const double treg = t < 64 ? g_exp2_64[t] : 0.0;
       const float freg = t < 128 ? g_exp2_ff[t] : 0.0f;
       const uint2 *rc = st.rcand + (size_t)item * s.m;
       const uint2 rv0 = (uint32_t)t < s.m ? rc[t] : make_uint2(0u, 0u);
@@ -2498,8 +2576,7 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
         }
         if (valid) {
           const uint32_t slot = base + __popc(bal & lt);
-          w.cxy[slot] = cxy;
-          w.caux[slot] = aux;
+          w.cand[slot] = make_uint2(cxy, aux);
         }
         ncoh += total;
         setup_bar<TS>();
@@ -2509,14 +2586,12 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
         const int i = t + u * TS;
         if (i < 512) lc[i] = lreg[u];
       }
-      if (t < 64) tab[t] = treg;
       if (t < 128) tab_ff[t] = freg;
       if (bad_map) atomicOr(&sh_flags, 2);
       if (maxoff) atomicMax(&sh_maxoff, maxoff);
       for (uint32_t q = t; q < s.m; q += TS) {
         const uint2 v = use_rcand(s, q == (uint32_t)t ? rv0 : rc[q]);
-        w.cxy[ncoh + q] = v.x;
-        w.caux[ncoh + q] = v.y | kAuxNeg | (q << 16);
+        w.cand[ncoh + q] = make_uint2(v.x, v.y | kAuxNeg | (q << 16));
       }
       if (t == 0) sh_ncoh = ncoh;
       setup_bar<TS>();
@@ -2526,11 +2601,8 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
         if (sh_maxoff <= kPad && !s.guide_dims_differ) {
           unsigned long long *cb = (unsigned long long *)(term + (((size_t)nk * nc + 1) & ~(size_t)1));
           for (uint32_t c = t; c < nc; c += TS) {
-            const uint32_t cxy = w.cxy[c], aux = w.caux[c];
-            const MapDesc md = s.maps[aux & 0x7fffu];
-            const unsigned long long off = md.poff + (unsigned long long)st.level * md.pw * md.ph +
-                                           (unsigned long long)((cxy >> 16) + kPad) * md.pw + ((cxy & 0xffffu) + kPad);
-            cb[c] = off | ((aux & kAuxNeg) ? (1ull << 63) : 0ull);
+            const uint32_t cxy = w.cand[c].x, aux = w.cand[c].y;
+            cb[c] = padded_centre(s.maps[aux & 0x7fffu], st.level, cxy) | ((aux & kAuxNeg) ? (1ull << 63) : 0ull);
           }
           setup_bar<TS>();
           constexpr int kRound = 16;  // gathers in flight per thread
@@ -2544,7 +2616,7 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
                 const uint32_t c = i / nk;
                 jj[u] = i - c * nk;
                 const unsigned long long v = cb[c];
-                const int lin = (v >> 63) ? -w.lin[jj[u]] : w.lin[jj[u]];
+                const int lj = (int32_t)w.nbr[jj[u]].x, lin = (v >> 63) ? -lj : lj;
                 const size_t off = (size_t)(v & 0x7fffffffffffffffull) + lin;
                 tx[u] = __ldg(s.plevels + off);
                 if (s.guided) gx[u] = __ldg(s.pguides + off);
@@ -2565,13 +2637,13 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
           uint32_t c = (uint32_t)t / nk, j = (uint32_t)t - c * nk;
           const uint32_t dc = (uint32_t)TS / nk, dj = (uint32_t)TS - dc * nk;
           for (uint32_t i = t; i < total; i += TS) {
-            const uint32_t cxy = w.cxy[c], aux = w.caux[c];
+            const uint32_t cxy = w.cand[c].x, aux = w.cand[c].y;
             const uint32_t map = aux & 0x7fffu;
             const int sg = (aux & kAuxNeg) ? -1 : 1;
             const MapDesc md = s.maps[map];
             const uint4 nr = w.nbr[j];
-            const int qx = (int)(cxy & 0xffffu) + sg * off_dx((int32_t)nr.x);
-            const int qy = (int)(cxy >> 16) + sg * off_dy((int32_t)nr.x);
+            const int qx = (int)(cxy & 0xffffu) + sg * off_dx(w.off[j]);
+            const int qy = (int)(cxy >> 16) + sg * off_dy(w.off[j]);
             uint32_t tt = kOutside;
             if ((unsigned)qx < md.w && (unsigned)qy < md.h)
               tt = __ldg(&s.levels[md.off + (size_t)st.level * md.w * md.h + (size_t)qy * md.w + qx]);
@@ -2607,7 +2679,7 @@ __global__ void __launch_bounds__(T) k_step_team_full(SessionDev s, StageDev st,
       const double avg = sh_mean;
       bool nan_w = false;
       for (uint32_t j = tid; j < nk; j += T) {
-        const float wv = neighbour_weight(sh.dist[j], avg, tab, tab_ff);
+        const float wv = neighbour_weight(sh.dist[j], avg, tab_ff);
         nan_w |= (wv != wv);
         w.nbr[j].w = __float_as_uint(wv);
         w.term[j] = wv;
@@ -2701,7 +2773,7 @@ void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cu
 
 }  // namespace
 
-size_t resolve_smem_bytes(uint32_t k, uint32_t m, int) { return 2048 + (size_t)kResolveWarps * warp_smem_bytes(k, m); }
+size_t resolve_smem_bytes(uint32_t k, uint32_t m) { return 2048 + (size_t)kResolveWarps * warp_smem_bytes(k, m); }
 static size_t team_smem_bytes(uint32_t k, uint32_t m) { return 2048 + warp_smem_bytes(k, m) + (size_t)(k ? k : 1) * 4; }
 // the full-evaluation team form keeps every (candidate, neighbour) term
 static size_t team_full_smem_bytes(uint32_t k, uint32_t m) {
@@ -2739,9 +2811,9 @@ static cudaError_t raise_smem(K *kernel, size_t bytes) {
 }
 
 cudaError_t configure_kernels(uint32_t k, uint32_t m) {
-  cudaError_t e = raise_smem(k_resolve, resolve_smem_bytes(k, m, 0));
+  cudaError_t e = raise_smem(k_resolve, resolve_smem_bytes(k, m));
   if (e != cudaSuccess) return e;
-  e = raise_smem(k_resolve_lean, resolve_smem_bytes(k, m, 0));
+  e = raise_smem(k_resolve_lean, resolve_smem_bytes(k, m));
   if (e != cudaSuccess) return e;
   e = raise_smem(k_knn_exhaustive, kExhAllKeys * 8);
   if (e != cudaSuccess) return e;
@@ -2816,7 +2888,7 @@ uint32_t multi_blocks(int phase, uint32_t n, uint32_t cap) {
 size_t multi_smem_bytes(int phase, uint32_t k, uint32_t m) {
   switch (phase) {
     case kPhaseExhaustive: return (size_t)kExhAllKeys * 8;
-    case kPhaseResolve: return resolve_smem_bytes(k, m, 0);
+    case kPhaseResolve: return resolve_smem_bytes(k, m);
     case kPhaseTeamPart: return team_smem_bytes(k, m);
     case kPhaseTeamFull: return team_full_smem_bytes(k, m);
     default: return 0;
@@ -2913,7 +2985,7 @@ void launch_resolve(const SessionDev &s, const StageDev &st, const BatchDev &b, 
                     const PendingCommit &pc) {
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 && pc.n == 0) return;
-  const size_t smem = resolve_smem_bytes(s.k, s.m, s.guided);
+  const size_t smem = resolve_smem_bytes(s.k, s.m);
   uint32_t grid = cdiv(n, kResolveWarps);
   if (b.work_ctr) {
     // a resident grid whose warps take further items from the counter

@@ -94,7 +94,10 @@ struct SessionDev {
   uint32_t exact_sx, exact_sy;
   double exact_q;
   int32_t exact_qe;  // exact_q = 2^exact_qe
+  float exact_qf;    // exact_q as f32
   uint32_t W, H, wpr;  // wpr: 32-bit words per bitmap row
+  // p / W == (p * w_mul) >> w_sh for every p < 2^28 (ts_div_multiplier)
+  uint32_t w_mul, w_sh;
   int tiling;
   int32_t x_l, x_r, y_b, y_t;
   uint32_t k, m;
@@ -163,11 +166,14 @@ struct BatchDev {
   // tag) commits them while it runs (PendingCommit) and reads a tagged
   // pixel's batch-start colour and state from the shadow instead of the image
   uint32_t defer_tag, prev_tag;
-  // warp resolve of the plain path: a counter (zeroed) from which the warps
-  // of a resident grid take items after their first, so that no warp waits
-  // for its block's slowest item; null: one item per warp of a full grid
+  // warp resolve of the plain path: kWorkCtrs counters (zeroed), kWorkCtrStride
+  // words apart, from which the warps of a resident grid take items after
+  // their first, so that no warp waits for its block's slowest item; null:
+  // one item per warp of a full grid
   uint32_t *work_ctr;
 };
+
+constexpr uint32_t kWorkCtrs = 16, kWorkCtrStride = 8;
 
 // One batch step of one session as the multi-session kernels read it.
 struct StepDev {
@@ -330,7 +336,7 @@ void launch_pad(const uint32_t *src, uint32_t w, uint32_t h, uint32_t levels, ui
                 cudaStream_t stream);
 
 // Bytes of dynamic shared memory the resolve kernel needs per CTA.
-size_t resolve_smem_bytes(uint32_t k, uint32_t m, int guided);
+size_t resolve_smem_bytes(uint32_t k, uint32_t m);
 // Per-device kernel attributes for a (k, m) session (current device).
 cudaError_t configure_kernels(uint32_t k, uint32_t m);
 
