@@ -163,8 +163,8 @@ typedef struct ts_run_stats {
    * copies, which wait for the device). */
   double host_pick_ms, host_launch_ms;
   /* Chunks of batches whose neighbour lists were made ahead on a side
-   * stream (power-of-two outputs with k > 0); 0 when every batch step made
-   * its own. */
+   * stream (k > 0; power-of-two outputs, others from 2048 pixels on); 0 when
+   * every batch step made its own. */
   uint64_t knn_chunks;
 } ts_run_stats;
 

@@ -208,15 +208,14 @@ __device__ __forceinline__ uint2 use_rcand(const SessionDev &s, uint2 v) {
 }
 
 // Exact squared normalised distance of a neighbour at offset (dx, dy).
-__device__ __forceinline__ double neighbour_dist(const SessionDev &s, int px, int py, int dx, int dy, double x2,
-                                                  double y2) {
+__device__ __forceinline__ double neighbour_dist(const SessionDev &s, int px, int py, int dx, int dy) {
   const int R = s.dtab_r;
   if (dx >= -R && dx <= R && dy >= -R && dy <= R) {
     const double ddx = __ldg(&s.dxt[(size_t)px * (2 * R + 1) + dx + R]);
     return __fma_rn(ddx, ddx, __ldg(&s.dy2t[(size_t)py * (2 * R + 1) + dy + R]));
   }
-  const double ddx = __dsub_rn(s.xdiv[px + dx + s.xdiv_off], x2);
-  const double ddy = __dsub_rn(s.ydiv[py + dy + s.ydiv_off], y2);
+  const double ddx = __dsub_rn(__ldg(&s.xdiv[px + dx + s.xdiv_off]), __ldg(&s.xdiv[px + s.xdiv_off]));
+  const double ddy = __dsub_rn(__ldg(&s.ydiv[py + dy + s.ydiv_off]), __ldg(&s.ydiv[py + s.ydiv_off]));
   return __fma_rn(ddx, ddx, __dmul_rn(ddy, ddy));
 }
 
@@ -400,9 +399,11 @@ __device__ __forceinline__ void knn_walk_body(const SessionDev &s, const StageDe
       // lanes, and GB300's f64 pipe is narrow)
       __syncwarp();
       // (sessions with exact sums store no distances: the resolve derives
-      // each one from its offset, exact_dist)
+      // each one from its offset, exact_dist;
+      // nor do lists made ahead: k_mean_ahead and the resolve derive them
+      // from the coordinate tables)
       unsigned long long part = 0;
-      for (uint32_t j = lane; j < s.k; j += kWarp) {
+      for (uint32_t j = lane; j < (s.exact_sum || b.dist ? s.k : 0u); j += kWarp) {
         const int32_t o = nbo[j];
         if (s.exact_sum)
           part += exact_units(s, off_dx(o), off_dy(o));
@@ -910,24 +911,22 @@ __device__ uint32_t knn_exhaustive_item(const SessionDev &s, const StageDev &st,
   int32_t *nbo = b.nbuf + (size_t)local * k;
   const uint32_t nb = b.i1 - b.i0;
   // the f64 distances from the coordinate tables, where something reads
-  // them: every list of an inexact session, and the caller's weights when the
-  // mean is not made here (exact sums derive the rest from the offsets; runs
-  // with the k-NN made ahead have no coordinate tables)
-  const bool want_d = !s.exact_sum || (with_mean && !mean_here);
-  double x2 = 0.0, y2 = 0.0;
-  if (want_d) {
-    x2 = s.xdiv[px + s.xdiv_off];
-    y2 = s.ydiv[py + s.ydiv_off];
-  }
+  // them: the stored lists of an inexact session, and the caller's weights
+  // when the mean is not made here (exact sums derive the rest from the
+  // offsets, lists made ahead leave theirs to k_mean_ahead)
+  const bool ahead = s.rank != nullptr;
+  const bool want_d = (!s.exact_sum && !ahead) || (with_mean && !mean_here);
   unsigned long long part = 0;
   for (uint32_t i = threadIdx.x; i < nout; i += blockDim.x) {
     const unsigned long long key = sorted[i];
     const int x = (int)(key & 0xffffu) - 32768, y = (int)((key >> 16) & 0xffffu) - 32768;
     nbo[i] = pack_off(x - px, y - py);
-    const double d = want_d ? neighbour_dist(s, px, py, x - px, y - py, x2, y2) : 0.0;
+    const double d = !want_d ? 0.0
+                     : s.exact_sum ? exact_dist(s, pack_off(x - px, y - py))
+                                   : neighbour_dist(s, px, py, x - px, y - py);
     if (s.exact_sum)
       part += exact_units(s, x - px, y - py);
-    else
+    else if (!ahead)
       b.dist[(size_t)i * nb + local] = d;
     if (with_mean) {
       sh.dist[i] = d;
@@ -944,7 +943,7 @@ __device__ uint32_t knn_exhaustive_item(const SessionDev &s, const StageDev &st,
       for (uint32_t w = 0; w < blockDim.x / 32; ++w) sum += sh.wsum[w];
       b.mean[local] = exact_mean(s, sum, nout);
     }
-  } else if (with_mean && mean_here) {
+  } else if (with_mean && mean_here && !ahead) {
     __syncthreads();
     if (threadIdx.x == 0 && nout > 0) b.mean[local] = mean_chain(sh.dist, nout);
   }
@@ -1233,8 +1232,15 @@ __device__ __forceinline__ bool neighbour_records(const SessionDev &s, const Sta
 // The weight of an item's neighbour j at offset off (fm = ts_ff_mean(avg)).
 // Sessions with exact sums and equal sides: the distance is dx^2 + dy^2 units,
 // an f32 pair (below 2^24 units a single f32).
+// Other sessions: the stored list, or (made ahead) the coordinate tables.
+__device__ __forceinline__ double item_dist(const SessionDev &s, const BatchDev &b, uint32_t local, uint32_t nb,
+                                            int px, int py, uint32_t j, int32_t off) {
+  if (s.exact_sum) return exact_dist(s, off);
+  if (!s.rank) return b.dist[(size_t)j * nb + local];
+  return neighbour_dist(s, px, py, off_dx(off), off_dy(off));
+}
 __device__ __forceinline__ float item_weight(const SessionDev &s, const BatchDev &b, uint32_t local, uint32_t nb,
-                                             uint32_t j, int32_t off, double avg, const FfMean &fm,
+                                             int px, int py, uint32_t j, int32_t off, double avg, const FfMean &fm,
                                              const float *tab_ff) {
   float d_hi = 0.0f, d_lo = 0.0f, wv;
   bool split = true;
@@ -1246,11 +1252,11 @@ __device__ __forceinline__ float item_weight(const SessionDev &s, const BatchDev
     d_lo = __fmul_rn((float)(int32_t)(u - (uint32_t)hi), s.exact_qf);
   } else {
     const double d = s.exact_sum ? bits_dbl(ts_units_bits(exact_units(s, off_dx(off), off_dy(off)), s.exact_qe))
-                                 : b.dist[(size_t)j * nb + local];
+                                 : item_dist(s, b, local, nb, px, py, j, off);
     split = dbl_bits(d) == 0 || ff_split_rn(d, d_hi, d_lo);
   }
   if (!(split && ts_weight_ff_pair(d_hi, d_lo, fm, tab_ff, wv)))
-    wv = weight_exact(s.exact_sum ? exact_dist(s, off) : b.dist[(size_t)j * nb + local], avg);
+    wv = weight_exact(item_dist(s, b, local, nb, px, py, j, off), avg);
   return wv;
 }
 
@@ -1260,7 +1266,7 @@ __device__ __forceinline__ bool neighbour_setup(const SessionDev &s, const Stage
                                                 double avg, const FfMean &fm, const float *tab_ff,
                                                 const WarpSmem &w, uint32_t &cxy, uint32_t &aux, bool &nan_w,
                                                 int &maxoff, bool &bad_map) {
-  const float wv = item_weight(s, b, local, nb, j, off, avg, fm, tab_ff);
+  const float wv = item_weight(s, b, local, nb, px, py, j, off, avg, fm, tab_ff);
   nan_w |= (wv != wv);
   return neighbour_records<kG>(s, st, b, px, py, j, off, wv, w, cxy, aux, maxoff, bad_map);
 }
@@ -1580,7 +1586,7 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
         uint32_t cxy = 0, aux = 0;
         if (j < nk) {
           const int32_t off = nbo[j];
-          const float wv = item_weight(s, b, local, nb, j, off, avg, fm, tab_ff);
+          const float wv = item_weight(s, b, local, nb, px, py, j, off, avg, fm, tab_ff);
           nan_w |= (wv != wv);
           valid = neighbour_records<!kLean>(s, st, b, px, py, j, off, wv, w, cxy, aux, maxoff, bad_map);
         }
@@ -2415,6 +2421,88 @@ __global__ void __launch_bounds__(kMeanThreads) k_mean_staged(SessionDev s, Stag
   mean_body_staged(b, blockIdx.x);
 }
 
+// The means of lists made ahead (sessions without exact sums): a block's
+// items' distances from the coordinate tables into shared memory, one column
+// per item (an odd pitch of doubles spreads the columns' writes over the
+// banks), then each item's chain of 4k f64 adds on one lane.  The chain keeps
+// the FP64 pipe busy (an f64 warp instruction takes it 18 cycles whatever its
+// active lanes), so every lane of a warp carries an item; the launches run on
+// the side stream, off the step chain.
+constexpr uint32_t kMeanPitch = kMeanThreads + 1;
+__global__ void __launch_bounds__(kMeanThreads)
+    k_mean_ahead(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+                 const __grid_constant__ BatchDev b) {
+  pdl_enter();
+  extern __shared__ double md[];  // [k][kMeanPitch]
+  __shared__ int xs[kMeanThreads], ys[kMeanThreads];
+  __shared__ uint32_t cnt[kMeanThreads];
+  const uint32_t first = blockIdx.x * kMeanThreads, n = min(kMeanThreads, b.i1 - b.i0 - first);
+  const uint32_t tid = threadIdx.x;
+  cnt[tid] = 0;
+  if (tid < n) {
+    pixel_xy(s, st.items[b.i0 + first + tid], xs[tid], ys[tid]);
+    cnt[tid] = b.ncnt[first + tid];
+  }
+  __syncthreads();
+  const int32_t *nbo = b.nbuf + (size_t)first * s.k;
+  uint32_t i = tid / s.k, j = tid - i * s.k;
+  for (uint32_t e = tid; e < n * s.k; e += kMeanThreads) {
+    if (j < cnt[i]) {
+      const int32_t off = nbo[e];
+      md[j * kMeanPitch + i] = neighbour_dist(s, xs[i], ys[i], off_dx(off), off_dy(off));
+    }
+    j += kMeanThreads;
+    while (j >= s.k) {
+      j -= s.k;
+      ++i;
+    }
+  }
+  __syncthreads();
+  if (tid >= n || cnt[tid] == 0) return;
+  double sum = 0.0;
+#pragma unroll 4
+  for (uint32_t q = 0; q < cnt[tid]; ++q) {
+    const double d = md[q * kMeanPitch + tid];
+    sum = __dadd_rn(sum, d);
+    sum = __dadd_rn(sum, d);
+    sum = __dadd_rn(sum, d);
+    sum = __dadd_rn(sum, d);
+  }
+  b.mean[first + tid] = __ddiv_rn(sum, (double)(cnt[tid] * 4u));
+}
+
+// The coordinate tables of a session without exact sums (SessionDev::xdiv,
+// ydiv, dxt, dy2t), with the IEEE operations of get_distances_to_k_neighs
+// (ms.rs:410-415): n_x, n_y entries of xdiv and ydiv, then 2 R + 1 offsets
+// per column and per row.
+__global__ void k_dist_tables(const __grid_constant__ SessionDev s, double *xdiv, double *ydiv, double *dxt,
+                              double *dy2t, uint32_t n_x, uint32_t n_y) {
+  const uint32_t w = 2u * (uint32_t)s.dtab_r + 1u, n_dx = s.W * w, n_dy = s.H * w;
+  const double dw = (double)s.W, dh = (double)s.H;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_x + n_y + n_dx + n_dy; i += gridDim.x * blockDim.x) {
+    uint32_t e = i;
+    if (e < n_x) {
+      xdiv[e] = __ddiv_rn((double)((int)e - s.xdiv_off), dw);
+      continue;
+    }
+    e -= n_x;
+    if (e < n_y) {
+      ydiv[e] = __ddiv_rn((double)((int)e - s.ydiv_off), dh);
+      continue;
+    }
+    e -= n_y;
+    const bool col = e < n_dx;
+    if (!col) e -= n_dx;
+    const int q = (int)(e / w), o = (int)(e - (uint32_t)q * w) - s.dtab_r;
+    const double side = col ? dw : dh;
+    const double d = __dsub_rn(__ddiv_rn((double)(q + o), side), __ddiv_rn((double)q, side));
+    if (col)
+      dxt[e] = d;
+    else
+      dy2t[e] = __dmul_rn(d, d);
+  }
+}
+
 __global__ void __launch_bounds__(128) k_mean_multi(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
@@ -2819,6 +2907,8 @@ cudaError_t configure_kernels(uint32_t k, uint32_t m) {
   if (e != cudaSuccess) return e;
   e = raise_smem(k_mean_staged, (size_t)k * kMeanThreads * 8);
   if (e != cudaSuccess) return e;
+  e = raise_smem(k_mean_ahead, (size_t)k * kMeanPitch * 8);
+  if (e != cudaSuccess) return e;
   e = raise_smem(k_resolve_team<kTeamThreads, false>, team_smem_bytes(k, m));
   if (e != cudaSuccess) return e;
   const size_t fsm = team_full_smem_bytes(k, m);
@@ -2961,6 +3051,19 @@ void launch_mean(const SessionDev &s, const StageDev &st, const BatchDev &b, cud
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 || s.k == 0) return;
   launch_pdl(k_mean_staged, cdiv(n, kMeanThreads), kMeanThreads, (size_t)s.k * kMeanThreads * 8, stream, s, st, b);
+}
+
+void launch_mean_ahead(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream) {
+  const uint32_t n = b.i1 - b.i0;
+  if (n == 0 || s.k == 0) return;
+  launch_pdl(k_mean_ahead, cdiv(n, kMeanThreads), kMeanThreads, (size_t)s.k * kMeanPitch * 8, stream, s, st, b);
+}
+
+void launch_dist_tables(const SessionDev &s, double *xdiv, double *ydiv, double *dxt, double *dy2t, uint32_t n_x,
+                        uint32_t n_y, cudaStream_t stream) {
+  const uint64_t n = (uint64_t)n_x + n_y + (uint64_t)(s.W + s.H) * (2 * s.dtab_r + 1);
+  k_dist_tables<<<(uint32_t)std::min<uint64_t>((n + 255) / 256, 152 * 8), 256, 0, stream>>>(s, xdiv, ydiv, dxt, dy2t,
+                                                                                             n_x, n_y);
 }
 
 // Resident blocks of a kernel on the current device (cached per kernel and

@@ -263,6 +263,12 @@ void launch_knn_walk(const SessionDev &s, const StageDev &st, const BatchDev &b,
 void launch_knn_exhaustive(const SessionDev &s, const StageDev &st, const BatchDev &b, bool all_items,
                            cudaStream_t stream, const PendingCommit &pc = PendingCommit{});
 void launch_mean(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream);
+// The means of a chunk of lists made ahead (sessions without exact sums).
+void launch_mean_ahead(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream);
+// The coordinate tables (SessionDev::xdiv, ydiv: n_x and n_y entries; dxt,
+// dy2t) of a session without exact sums.
+void launch_dist_tables(const SessionDev &s, double *xdiv, double *ydiv, double *dxt, double *dy2t, uint32_t n_x,
+                        uint32_t n_y, cudaStream_t stream);
 void launch_resolve(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream,
                     const PendingCommit &pc = PendingCommit{});
 // One CTA per item; `full` scores every candidate completely (lowest latency,

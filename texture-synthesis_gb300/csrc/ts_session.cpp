@@ -1346,7 +1346,7 @@ struct RunCtx {
   PinnedBuf<uint32_t> pitems;
   std::vector<float> luts;
   std::vector<int32_t> tab;
-  std::vector<double> xdiv, ydiv, dxt, dy2t;
+  size_t n_xdiv = 0, n_ydiv = 0;  // entries of the coordinate tables (0: exact sums need none)
   size_t n_batches = 0;
   uint64_t overall_total = 0;
   uint32_t max_batch_items = 1;
@@ -1421,12 +1421,16 @@ struct RunCtx {
 bool exact_sum_ok(uint32_t W, uint32_t H, uint32_t k);
 
 // Whether a run makes its k-NN ahead (RunCtx::knn_ahead): asked for, k > 0,
-// exact sums, and the lists of every item of the run, held at once, within
-// kKnnAheadMaxBytes (larger runs keep the per-step form's scratch).  run_plan
-// leaves out the coordinate tables of such runs, so it decides the same way.
+// the lists of every item of the run, held at once, within kKnnAheadMaxBytes
+// (larger runs keep the per-step form's scratch), and exact sums or an output
+// of kKnnAheadMinPixels (203x117, k = 8: 1.78 against 2.62 ms a call; 500^2:
+// 7.28 against 8.14).  Smaller inexact outputs would gain as well (40^2,
+// k = 50: 2.05 against 3.09 ms) but are documented and tested to keep the
+// per-step form (ts_run_stats.knn_chunks).
 bool knn_ahead_fits(const RunCtx &c, uint32_t W, uint32_t H, uint32_t k) {
   constexpr uint64_t kKnnAheadMaxBytes = 16ull << 30;
-  return c.want_knn_ahead && k > 0 && exact_sum_ok(W, H, k) &&
+  constexpr uint64_t kKnnAheadMinPixels = 2048;
+  return c.want_knn_ahead && k > 0 && (exact_sum_ok(W, H, k) || (uint64_t)W * H >= kKnnAheadMinPixels) &&
          (uint64_t)c.items.size() * ((uint64_t)k * 4 + 16) <= kKnnAheadMaxBytes;
 }
 
@@ -1612,29 +1616,6 @@ void run_plan(ts_session *s, RunCtx &c) {
   c.rc_ahead = c.want_rc_ahead && m > 0 && (uint64_t)n_items_total * m <= kRcandWhole;
   c.x_l = x_l;
   c.y_b = y_b;
-  const int32_t xo = x_l + 2, yo = y_b + 2;
-  // The coordinate tables below serve the f64 distances of inexact sessions
-  // and of the fused small-step kernel; a run whose k-NN is made ahead
-  // (exact sums) derives every distance from its offset and needs none.
-  const bool no_dist_tables = knn_ahead_fits(c, W, H, k);
-  c.xdiv.resize(no_dist_tables ? 0 : W + 2 * (size_t)xo + 1);
-  c.ydiv.resize(no_dist_tables ? 0 : H + 2 * (size_t)yo + 1);
-  for (size_t i = 0; i < c.xdiv.size(); ++i) c.xdiv[i] = (double)((int64_t)i - xo) / (double)W;
-  for (size_t i = 0; i < c.ydiv.size(); ++i) c.ydiv[i] = (double)((int64_t)i - yo) / (double)H;
-  // per-pixel tables of the normalised offsets the weights use: dx and
-  // dy * dy for |offset| <= kDistTabRadius, the same IEEE operations as
-  // get_distances_to_k_neighs (ms.rs:410-415)
-  const int32_t R = kDistTabRadius;
-  c.dxt.resize(no_dist_tables ? 0 : (size_t)W * (2 * R + 1));
-  c.dy2t.resize(no_dist_tables ? 0 : (size_t)H * (2 * R + 1));
-  for (uint32_t x = 0; x < W && !no_dist_tables; ++x)
-    for (int32_t o = -R; o <= R; ++o)
-      c.dxt[(size_t)x * (2 * R + 1) + o + R] = (double)((int64_t)x + o) / (double)W - (double)x / (double)W;
-  for (uint32_t y = 0; y < H && !no_dist_tables; ++y)
-    for (int32_t o = -R; o <= R; ++o) {
-      const double dy = (double)((int64_t)y + o) / (double)H - (double)y / (double)H;
-      c.dy2t[(size_t)y * (2 * R + 1) + o + R] = dy * dy;
-    }
   // the tree is rebuilt from the resolved list, mirrors included (ms.rs:747-779)
   c.occ.assign((size_t)wpr * H, 0);
   c.mir.assign((size_t)wpr * H, 0);
@@ -1664,6 +1645,14 @@ void run_plan(ts_session *s, RunCtx &c) {
     else if (y > (int)H - y_b)
       add_cell(x, y - (int)H);
   }
+  // the coordinate tables serve the f64 distances of sessions without exact
+  // sums (launch_dist_tables); exact ones derive every distance from its
+  // offset
+  const bool tables = k > 0 && !exact_sum_ok(W, H, k);
+  c.n_xdiv = tables ? W + 2 * (size_t)(x_l + 2) + 1 : 0;
+  c.n_ydiv = tables ? H + 2 * (size_t)(y_b + 2) + 1 : 0;
+  const uint64_t dist_table_doubles =
+      tables ? c.n_xdiv + c.n_ydiv + ((uint64_t)W + H) * (2 * kDistTabRadius + 1) : 0;
   // device memory the run will hold (run_alloc), for admission control
   const size_t kk = std::max<uint32_t>(k, 1), mb = max_batch_items;
   uint64_t steps_est = 0;
@@ -1671,7 +1660,7 @@ void run_plan(ts_session *s, RunCtx &c) {
   c.dev_bytes = N * 4 + N * sizeof(uint4) + 2 * (uint64_t)wpr * H * 4 + c.res_total * 8 + items.size() * 4 +
                 c.luts.size() * 4 + c.tab.size() * 4 + mb * kk * 12 + mb * (4 + 8 + 4 + sizeof(Result)) +
                 c.n_batches * 4 + (c.rc_ahead ? (uint64_t)items.size() : std::max<uint64_t>(c.rc_items, mb)) * m * 8 +
-                (c.xdiv.size() + c.ydiv.size() + c.dxt.size() + c.dy2t.size()) * 8 + steps_est * sizeof(StepDev) +
+                dist_table_doubles * 8 + steps_est * sizeof(StepDev) +
                 c.cells.size() * 4 + c.init_list.size() * 4;
 }
 
@@ -1963,15 +1952,16 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     c.tab_parts.push_back(RunCtx::TabPart{o, v.data(), bytes});
     return o;
   };
-  const size_t t_lut = T(c.luts), t_tab = T(c.tab), t_xdiv = T(c.xdiv), t_ydiv = T(c.ydiv), t_dxt = T(c.dxt),
-               t_dy2t = T(c.dy2t), t_cells = T(c.cells), t_occ = T(c.occ), t_mir = T(c.mir), t_init = T(c.init_list),
+  const size_t t_lut = T(c.luts), t_tab = T(c.tab), t_cells = T(c.cells), t_occ = T(c.occ), t_mir = T(c.mir), t_init = T(c.init_list),
                t_btab = T(c.btab);
   // scratch
   const size_t w_res = wl.add(c.res_total * 4), w_items = wl.add(c.items.size() * 4), w_nbuf = wl.add(mb * kk * 4),
-               w_ncnt = wl.add(mb * 4), w_dist = wl.add(mb * kk * 8), w_mean = wl.add(mb * 8), w_fbl = wl.add(mb * 4),
+               w_ncnt = wl.add(mb * 4), w_dist = wl.add(c.knn_ahead ? 0 : mb * kk * 8), w_mean = wl.add(mb * 8), w_fbl = wl.add(mb * 4),
                w_result = wl.add((c.knn_ahead ? 2 : 1) * mb * sizeof(Result)), w_rcand = wl.add(rc_n * 8),
                w_knbuf = wl.add(n_kitems * kk * 4), w_kncnt = wl.add(n_kitems * 4), w_kmean = wl.add(n_kitems * 8),
-               w_kfbl = wl.add(n_kitems * 4);
+               w_kfbl = wl.add(n_kitems * 4), w_xdiv = wl.add(c.n_xdiv * 8), w_ydiv = wl.add(c.n_ydiv * 8),
+               w_dxt = wl.add(c.n_xdiv ? (size_t)W * (2 * R + 1) * 8 : 0),
+               w_dy2t = wl.add(c.n_xdiv ? (size_t)H * (2 * R + 1) * 8 : 0);
   CUDA_TRY(A(c.d_zero, zl.off));
   CUDA_TRY(A(c.d_tabs, tl.off));
   CUDA_TRY(A(c.d_work, wl.off));
@@ -1986,10 +1976,6 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.d_evals.view(z + z_evals, 1);
   c.d_lut.view(tb + t_lut, c.luts.size());
   c.d_tab.view(tb + t_tab, c.tab.size());
-  c.d_xdiv.view(tb + t_xdiv, c.xdiv.size());
-  c.d_ydiv.view(tb + t_ydiv, c.ydiv.size());
-  c.d_dxt.view(tb + t_dxt, c.dxt.size());
-  c.d_dy2t.view(tb + t_dy2t, c.dy2t.size());
   c.d_cells.view(tb + t_cells, c.cells.size());
   c.d_occ.view(tb + t_occ, c.occ.size());
   c.d_mir.view(tb + t_mir, c.mir.size());
@@ -2003,11 +1989,15 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.d_kncnt.view(wk + w_kncnt, n_kitems);
   c.d_kmean.view(wk + w_kmean, n_kitems);
   c.d_kfbl.view(wk + w_kfbl, n_kitems);
+  c.d_xdiv.view(wk + w_xdiv, c.n_xdiv);
+  c.d_ydiv.view(wk + w_ydiv, c.n_ydiv);
+  c.d_dxt.view(wk + w_dxt, c.n_xdiv ? (size_t)W * (2 * R + 1) : 0);
+  c.d_dy2t.view(wk + w_dy2t, c.n_xdiv ? (size_t)H * (2 * R + 1) : 0);
   c.d_res.view(wk + w_res, c.res_total);
   c.d_items.view(wk + w_items, c.items.size());
   c.d_nbuf.view(wk + w_nbuf, mb * kk);
   c.d_ncnt.view(wk + w_ncnt, mb);
-  c.d_dist.view(wk + w_dist, mb * kk);
+  c.d_dist.view(wk + w_dist, c.knn_ahead ? 0 : mb * kk);
   c.d_mean.view(wk + w_mean, mb);
   c.d_fbl.view(wk + w_fbl, mb);
   c.d_result.view(wk + w_result, (c.knn_ahead ? 2 : 1) * mb);
@@ -2149,6 +2139,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
           bd.nbuf = c.d_knbuf.p + g0 * kk;
           bd.ncnt = c.d_kncnt.p + g0;
           bd.mean = c.d_kmean.p + g0;
+          bd.dist = nullptr;
         }
         stp.exhaustive = bp.exhaustive;
         bd.grid_first = bp.grid_first ? 1 : 0;
@@ -2237,6 +2228,10 @@ void run_upload(RunCtx &c, cudaStream_t st) {
     CUDA_TRY(cudaMemsetAsync(c.d_zero.p, 0, c.zero_bytes, st));
   }
   CUDA_TRY(cudaMemcpyAsync(c.d_tabs.p, c.ptab.p, c.tabs_bytes, cudaMemcpyHostToDevice, st));
+  if (c.n_xdiv) {
+    launch_dist_tables(c.sd, c.d_xdiv.p, c.d_ydiv.p, c.d_dxt.p, c.d_dy2t.p, (uint32_t)c.n_xdiv, (uint32_t)c.n_ydiv, st);
+    ++c.launches;
+  }
   if (c.dense_init) {
     if (c.locked) CUDA_TRY(cudaMemcpyAsync(c.d_res.p, c.resolved.data(), c.locked * 4, cudaMemcpyHostToDevice, st));
   } else if (!c.init_list.empty()) {
@@ -2281,6 +2276,10 @@ void run_enqueue_knn(RunCtx &c, cudaStream_t kst, LaunchTimer &lt, int stage) {
       lt.run(TS_KERNEL_KNN_WALK, [&] { launch_knn_walk(sd, ch.st, ch.b, kst, PendingCommit{}); });
       lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, false, kst, PendingCommit{}); });
       c.launches += 2;
+    }
+    if (!sd.exact_sum) {
+      lt.run(TS_KERNEL_MEAN, [&] { launch_mean_ahead(sd, ch.st, ch.b, kst); });
+      ++c.launches;
     }
     CUDA_TRY(cudaEventCreateWithFlags(&c.knn_ev[q].e, cudaEventDisableTiming));
     CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, kst));
