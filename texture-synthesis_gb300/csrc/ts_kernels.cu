@@ -1316,14 +1316,16 @@ __device__ __forceinline__ float candidate0_score(const SessionDev &s, const Sta
 
 // The reference's sequential find_best_match (ms.rs:1184-1221), for stages or
 // items with non-finite or negative costs, where early exit and argmin need
-// its exact comparison sequence.  One thread.
+// its exact comparison sequence.  One thread.  Candidates from n_coh on lie
+// `gap` records further.
 template <bool kG = true>
 __device__ void sequential_best(const SessionDev &s, const StageDev &st, const WarpSmem &w, const float *lc,
-                                const float *lg, uint32_t nk, uint32_t nc, float &best_s, uint32_t &best_i) {
+                                const float *lg, uint32_t nk, uint32_t nc, float &best_s, uint32_t &best_i,
+                                uint32_t n_coh = 0, uint32_t gap = 0) {
   best_s = FLT_MAX;
   best_i = 0;
   for (uint32_t c = 0; c < nc; ++c) {
-    const uint2 cd = w.cand[c];
+    const uint2 cd = w.cand[c < n_coh ? c : c + gap];
     const uint32_t aux = cd.y;
     const uint32_t map = aux & 0x7fffu;
     const bool neg = (aux & kAuxNeg) != 0;
@@ -1370,18 +1372,12 @@ __device__ __forceinline__ void add_cell_point(const SessionDev &s, int x, int y
 __device__ __forceinline__ void commit_item(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t local,
                                             const Result &r, bool count_evals = true) {
   const uint32_t p = r.pixel;
-  if (r.cmap >= s.n_maps || p >= s.W * s.H) {
+  if ((r.flags & kResBad) || p >= s.W * s.H) {
     set_err(s.err, kDevErrIndex);
     return;
   }
-  const MapDesc md = s.maps[r.cmap];
-  const uint32_t sx = r.srcxy & 0xffffu, sy = r.srcxy >> 16;
-  if (sx >= md.w || sy >= md.h) {
-    set_err(s.err, kDevErrIndex);
-    return;
-  }
-  s.state[p] = make_uint4(r.srcxy, r.idp, r.idm, r.cmap);
-  s.color[p] = s.levels[md.off + (size_t)st.level * md.w * md.h + (size_t)sy * md.w + sx];
+  s.state[p] = make_uint4(r.srcxy, r.idp, r.idm, r.idm);
+  s.color[p] = r.color;
   if (count_evals && r.ncand) atomicAdd(s.evals, (unsigned long long)r.ncand);
   if (r.flags & kResAppend) {
     const uint32_t item = b.i0 + local;
@@ -1417,17 +1413,19 @@ __device__ __forceinline__ void emit_result(const SessionDev &s, const StageDev 
     commit_item(s, st, b, local, r, count_evals);
   } else {
     b.res[local] = r;
-    if (b.defer_tag && r.cmap < s.n_maps && r.pixel < s.W * s.H) {
+    if (b.defer_tag && !(r.flags & kResBad) && r.pixel < s.W * s.H) {
       // what the commit will write, for the next step's readers (start_pixel)
-      const MapDesc md = s.maps[r.cmap];
-      const uint32_t sx = r.srcxy & 0xffffu, sy = r.srcxy >> 16;
-      if (sx < md.w && sy < md.h) {
-        const uint32_t col = s.levels[md.off + (size_t)st.level * md.w * md.h + (size_t)sy * md.w + sx];
-        s.shadow[2 * (size_t)r.pixel] = make_uint4(b.defer_tag, col, 0u, 0u);
-        s.shadow[2 * (size_t)r.pixel + 1] = make_uint4(r.srcxy, r.idp, r.idm, r.cmap);
-      }
+      s.shadow[2 * (size_t)r.pixel] = make_uint4(b.defer_tag, r.color, 0u, 0u);
+      s.shadow[2 * (size_t)r.pixel + 1] = make_uint4(r.srcxy, r.idp, r.idm, r.idm);
     }
   }
+}
+
+// The colour of a candidate's centre at the stage's level (its coordinates
+// are valid).
+__device__ __forceinline__ uint32_t centre_colour(const SessionDev &s, const StageDev &st, uint32_t map, uint32_t cxy) {
+  const MapDesc md = s.maps[map];
+  return __ldg(&s.levels[md.off + (size_t)st.level * md.w * md.h + (size_t)(cxy >> 16) * md.w + (cxy & 0xffffu)]);
 }
 
 // The winning candidate as an update (ms.rs:976-1001): source coordinate and
@@ -1456,7 +1454,7 @@ __device__ void write_result(const SessionDev &s, const StageDev &st, const Warp
   r.srcxy = cxy;
   r.idp = idp;
   r.idm = map;
-  r.cmap = map;
+  r.color = centre_colour(s, st, map, cxy);
   r.flags = (is_new ? kResAppend : 0u) | kResMirrors;
   r.score = best_s;
   r.ncand = nc;
@@ -1483,7 +1481,7 @@ __device__ void write_random_result(const SessionDev &s, const StageDev &st, con
   r.srcxy = x | (y << 16);
   r.idp = pixel;
   r.idm = map;
-  r.cmap = map;
+  r.color = centre_colour(s, st, map, r.srcxy);
   r.flags = kResAppend;
   r.score = 0.0f;
   r.ncand = 0;
@@ -1500,8 +1498,8 @@ __device__ void write_bad_result(const SessionDev &s, const StageDev &st, const 
   r.srcxy = 0;
   r.idp = 0;
   r.idm = 0;
-  r.cmap = 0xffffffffu;
-  r.flags = 0;
+  r.color = 0;
+  r.flags = kResBad;
   r.score = 0.0f;
   r.ncand = 0;
   emit_result(s, st, b, local, r);
@@ -2223,9 +2221,11 @@ __global__ void k_pad(const uint32_t *src, uint32_t w, uint32_t h, uint32_t leve
 // then lets the next one launch, whose blocks start and wait in turn while
 // this one's last wave runs.  Kernels launched without the attribute pass
 // both instructions at once.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait();
+  pdl_launch();
 }
 
 // ---------------------------------------------------------------------------
@@ -2552,6 +2552,451 @@ __global__ void __launch_bounds__(T) k_resolve_team_multi(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
   resolve_team_body<T, kFull>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+}
+
+// ---------------------------------------------------------------------------
+// resolve, small steps: a CTA of T threads per item, for steps too small to
+// fill the GPU with warps, where the time of a step is one item's chain of
+// dependent loads, barriers and sums (the plain path runs some 60 to 130 such
+// steps one after another).
+//
+// With its lists and random candidates made ahead (BatchDev::early) nearly all
+// of an item is known before the step it builds on is done: its weights, its
+// target-guide texels, its random candidates and their texels.  All of that
+// runs before griddepcontrol.wait, and the launch lets the next step's launch
+// start before it waits itself, so it overlaps the steps before.  What
+// remains after the wait is one warp's loads of the neighbours' state, the
+// repeat match, one gather of the few different coherence candidates (the
+// random ones' terms are formed while it is in flight), one in-order sum per
+// lane and the argmin.  A step of one item, k = m = 50: 18.8 -> 4.7 us, of
+// which 1.2 from the end of the step before to the wait's return, 1 state and
+// repeats, 1.2 gather and terms, 0.8 sums and argmin, 0.4 commit.
+//
+// F: terms of a random candidate formed at once: all of them while the steps
+// are small; for larger ones (kSmallFirst) only the candidates that are still
+// below the best coherence cost after F terms go on.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kSmallK = 64;      // neighbours one warp takes in two rounds
+constexpr uint32_t kSmallFirst = 8;
+constexpr size_t kSmallMaxSmem = 64 * 1024;
+// Floats per term row: a multiple of 4 whose quarter is odd, so that the lanes'
+// in-order sums read 16 bytes each from different banks.
+__host__ __device__ __forceinline__ uint32_t term_pitch(uint32_t k) { return 4u * (((k + 3u) / 4u) | 1u); }
+// LUTs, records, offsets, patch ids, then per candidate {record, centre,
+// centre colour} and its term row; coherence candidates in slots [0, k),
+// random ones in [k, k + m).
+__host__ __device__ __forceinline__ size_t small_smem_bytes(uint32_t k, uint32_t m, uint32_t n_maps) {
+  return 2048 + kSmallK * 24 + (size_t)n_maps * 16 + (((size_t)(k + m) * 20 + 15) & ~(size_t)15) +
+         (size_t)(k + m) * term_pitch(k) * 4;
+}
+
+template <int T, bool kG>
+__device__ __forceinline__ void resolve_small_body(const SessionDev &s, const StageDev &st, const BatchDev &b,
+                                                   const PendingCommit &pc, uint32_t F) {
+  constexpr int NW = T / kWarp;
+  constexpr int NR = T >= 512 ? 6 : (T >= 256 ? 10 : 4);  // random texels held per thread
+  constexpr int NC = 2;                                   // coherence texels in flight per thread
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ float tab_ff[128];
+  __shared__ float red_s[NW];
+  __shared__ uint32_t red_i[NW];
+  __shared__ uint32_t sh_ncoh, sh_all, sh_bad, sh_live;
+  __shared__ uint2 first[kWarp];
+  __shared__ uint8_t slots[128];
+  float *lc = (float *)smem, *lg = lc + 256;
+  uint4 *nbr = (uint4 *)(smem + 2048);
+  int32_t *offs = (int32_t *)(nbr + kSmallK);
+  uint32_t *pid = (uint32_t *)(offs + kSmallK);
+  uint4 *mt = (uint4 *)(pid + kSmallK);  // {w | mask flag | h << 16, -, texel index of (0, 0) on the padded planes}
+  uint64_t *cen = (uint64_t *)(mt + s.n_maps);
+  uint2 *cand = (uint2 *)(cen + s.k + s.m);
+  uint32_t *ccol = (uint32_t *)(cand + s.k + s.m);
+  float *rows = (float *)(smem + 2048 + kSmallK * 24 + (size_t)s.n_maps * 16 +
+                          align16((size_t)(s.k + s.m) * 20));
+  constexpr uint32_t kMasked = 0x8000u;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t lt = (1u << lane) - 1u, pitch = term_pitch(s.k);
+  const uint32_t nb = b.i1 - b.i0;
+  for (int i = tid; i < (kG ? 512 : 256); i += T) lc[i] = st.lut[i];
+  for (int i = tid; i < 128; i += T) tab_ff[i] = g_exp2_ff[i];
+  for (uint32_t i = tid; i < s.n_maps; i += T) {
+    const MapDesc md = s.maps[i];
+    const uint64_t c0 = padded_centre(md, st.level, 0u);
+    mt[i] = make_uint4(md.w | (md.h << 16) | (md.mask_off >= 0 ? kMasked : 0u), 0u, (uint32_t)c0, (uint32_t)(c0 >> 32));
+  }
+  auto centre_of = [&](uint32_t map, uint32_t cxy) -> uint64_t {
+    const uint4 e = mt[map];
+    return (((uint64_t)e.w << 32) | e.z) + (uint64_t)((cxy >> 16) * s.ppitch + (cxy & 0xffffu));
+  };
+  // texel (and guide texel) of candidate slot c at neighbour j
+  auto fetch = [&](uint32_t c, uint32_t j, bool far, uint32_t &t, uint32_t &g) {
+    if (!far) {
+      const int lin = (int32_t)nbr[j].x;
+      const int64_t at = (int64_t)cen[c] + ((cand[c].y & kAuxNeg) ? -lin : lin);
+      t = __ldg(s.plevels + at);
+      if (kG) g = __ldg(s.pguides + at);
+    } else {
+      const uint2 cd = cand[c];
+      const uint32_t map = cd.y & 0x7fffu;
+      const int sg = (cd.y & kAuxNeg) ? -1 : 1;
+      const int qx = (int)(cd.x & 0xffffu) + sg * off_dx(offs[j]), qy = (int)(cd.x >> 16) + sg * off_dy(offs[j]);
+      const MapDesc md = s.maps[map];
+      t = texel(s.levels + md.off + (size_t)st.level * md.w * md.h, md, qx, qy);
+      if (kG) {
+        const GuideDesc gd = s.gdesc[map];
+        g = kOutside;
+        if ((unsigned)qx < gd.w && (unsigned)qy < gd.h)
+          g = __ldg(&s.guides[gd.off + (size_t)st.level * gd.w * gd.h + (size_t)qy * gd.w + qx]);
+      }
+    }
+  };
+  auto put_term = [&](uint32_t c, uint32_t j, uint32_t t, uint32_t g) {
+    const uint4 nr = nbr[j];
+    float nps = lut4r(lc, __vabsdiffu4(nr.y, t), 0.0f, st.opaque);
+    if (kG) nps = lut4r(lg, __vabsdiffu4(nr.z, g), nps, st.opaque);
+    rows[c * pitch + j] = __fmul_rn(nps, __uint_as_float(nr.w));
+  };
+  // in-order sum of row c over [j, n), from acc (j a multiple of 4)
+  auto row_sum = [&](uint32_t c, uint32_t j, uint32_t n, float acc) -> float {
+    const float *row = rows + c * pitch;
+    for (; j + 8 <= n; j += 8) {  // both loads in flight ahead of their adds
+      const float4 v = *(const float4 *)(row + j), x = *(const float4 *)(row + j + 4);
+      acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+      acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, x.x), x.y), x.z), x.w);
+    }
+    for (; j + 4 <= n; j += 4) {
+      const float4 v = *(const float4 *)(row + j);
+      acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+    }
+    for (; j < n; ++j) acc = __fadd_rn(acc, row[j]);
+    return acc;
+  };
+  // lowest (score, index) over the block; every thread gets it
+  auto block_best = [&](float v, uint32_t i, float &bs, uint32_t &bi) {
+    const float wv = warp_min(v);
+    const uint32_t wi = __reduce_min_sync(0xffffffffu, v == wv ? i : 0xffffffffu);
+    if (lane == 0) {
+      red_s[warp] = wv;
+      red_i[warp] = wi;
+    }
+    __syncthreads();
+    const float qv = lane < NW ? red_s[lane] : __builtin_huge_valf();
+    const uint32_t qi = lane < NW ? red_i[lane] : 0xffffffffu;
+    bs = warp_min(qv);
+    bi = __reduce_min_sync(0xffffffffu, qv == bs ? qi : 0xffffffffu);
+  };
+
+  bool waited = false;
+  uint32_t evals = 0;  // thread 0: candidates of the items committed here
+  auto wait_once = [&]() {
+    if (waited) return;
+    waited = true;
+    pdl_wait();
+    // the previous step's deferred commit, by the last threads first (the
+    // first warp has the chain to run)
+    uint32_t ev = 0;
+    for (uint32_t i = blockIdx.x * T + (T - 1 - tid); i < pc.n; i += gridDim.x * T) {
+      const Result r = pc.b.res[i];
+      ev += r.ncand;
+      commit_item(s, pc.st, pc.b, i, r, false);
+    }
+    if (pc.n) {
+      ev = __reduce_add_sync(0xffffffffu, ev);
+      if (lane == 0 && ev) atomicAdd(s.evals, (unsigned long long)ev);
+    }
+  };
+  if (!b.early) wait_once();  // the lists come from the launches before this one
+
+  for (uint32_t local = blockIdx.x; local < nb; local += gridDim.x) {
+    __syncthreads();  // the tables (first item), the records of the item before
+    const uint32_t item = b.i0 + local;
+    const uint32_t pixel = st.items[item];
+    const uint32_t nk = b.ncnt[local];
+    if (nk == 0) {
+      wait_once();
+      if (tid == 0) write_random_result(s, st, b, local, pixel);
+      continue;
+    }
+    int px, py;
+    pixel_xy(s, pixel, px, py);
+    const double avg = b.mean[local];
+    const FfMean fm = ts_ff_mean(avg);
+    bool nan_w = false;
+    int maxoff = 0;
+    for (uint32_t j = tid; j < nk; j += T) {
+      const int32_t off = b.nbuf[(size_t)local * s.k + j];
+      const int dx = off_dx(off), dy = off_dy(off);
+      maxoff = max(maxoff, max(abs(dx), abs(dy)));
+      uint32_t gpat = 0;
+      if (kG) {
+        const uint32_t p = (uint32_t)wrap1(py + dy, (int)s.H) * s.W + (uint32_t)wrap1(px + dx, (int)s.W);
+        gpat = __ldg(&s.tguide[(size_t)st.level * s.W * s.H + p]);
+      }
+      const float wv = item_weight(s, b, local, nb, px, py, j, off, avg, fm, tab_ff);
+      nan_w |= (wv != wv);
+      nbr[j] = make_uint4((uint32_t)(dy * (int)s.ppitch + dx), 0u, gpat, __float_as_uint(wv));
+      offs[j] = off;
+    }
+    const uint2 *rc = st.rcand + (size_t)item * s.m;
+    for (uint32_t t = tid; t < s.m; t += T) {
+      const uint2 cd = random_candidate(s, rc, t);
+      const uint64_t c = centre_of(cd.y & 0x7fffu, cd.x);
+      cand[s.k + t] = cd;
+      cen[s.k + t] = c;
+      ccol[s.k + t] = __ldg(s.plevels + c);
+    }
+    const bool far = __syncthreads_or(maxoff > kPad) || s.guide_dims_differ;
+    const bool slow = __syncthreads_or(nan_w) || st.slow_lut;
+    // the random candidates' first f texels
+    const uint32_t f = min(F, nk), n_rnd = slow ? 0u : s.m * f;
+    const float rf = __fdividef(1.0f, (float)f);
+    auto split = [&](uint32_t i, float r, uint32_t n, uint32_t &c, uint32_t &j) {
+      c = (uint32_t)(((float)i + 0.5f) * r);  // i / n, exact below 2^20
+      j = i - c * n;
+    };
+    uint32_t tx[NR], gx[NR];
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+      const uint32_t i = tid + (uint32_t)u * T;
+      tx[u] = gx[u] = 0;
+      if (i < n_rnd) {
+        uint32_t c, j;
+        split(i, rf, f, c, j);
+        fetch(s.k + c, j, far, tx[u], gx[u]);
+      }
+    }
+    wait_once();
+    // the neighbours' state: own pattern (ms.rs:1151-1181), coherence
+    // candidates (ms.rs:497-547) without repeats (the same cost as the first
+    // of them; kept where the exact sequential form compares them)
+    if (warp == 0) {
+      uint32_t pat[2], ncoh = 0, all = 0;
+      uint4 sv[2];
+      bool bad = false;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint32_t j = lane + (uint32_t)r * kWarp;
+        pat[r] = 0;
+        sv[r] = make_uint4(0u, 0u, 0u, 0u);
+        if (j < nk) {
+          const int32_t off = offs[j];
+          const uint32_t p = (uint32_t)wrap1(py + off_dy(off), (int)s.H) * s.W + (uint32_t)wrap1(px + off_dx(off), (int)s.W);
+          start_pixel(s, b, p, true, pat[r], sv[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint32_t j = lane + (uint32_t)r * kWarp;
+        if ((uint32_t)r * kWarp >= nk) break;
+        bool valid = false;
+        uint32_t cxy = 0;
+        const uint32_t map = sv[r].z;
+        if (j < nk) {
+          nbr[j].y = pat[r];
+          pid[j] = sv[r].y;
+          if (map >= s.n_maps) {
+            bad = true;
+          } else {
+            const int ccx = (int)(sv[r].x & 0xffffu) - off_dx(offs[j]), ccy = (int)(sv[r].x >> 16) - off_dy(offs[j]);
+            const uint32_t wh = mt[map].x, mw = wh & 0x7fffu;
+            valid = (uint32_t)ccx < mw && (uint32_t)ccy < (wh >> 16);
+            if (valid && (wh & kMasked)) valid = __ldg(&s.masks[s.maps[map].mask_off + (size_t)ccy * mw + ccx]) != 0;
+            cxy = (uint32_t)ccx | ((uint32_t)ccy << 16);
+          }
+        }
+        const uint32_t vm = __ballot_sync(0xffffffffu, valid);
+        bool keep = valid;
+        if (!slow) {
+          uint32_t same;
+          if (s.n_maps <= 16)
+            same = __match_any_sync(0xffffffffu, (cxy & 0x3fffu) | ((cxy >> 16) << 14) | (map << 28));
+          else
+            same = __match_any_sync(0xffffffffu, ((unsigned long long)map << 32) | cxy);
+          if (same & vm & lt) keep = false;
+          // the second round against the first: a table from hashes to lanes
+          // of the first round (the last writer of a slot; what it holds is
+          // compared, so a stale or shared slot only lets a repeat stay)
+          const uint32_t h = ((cxy + map * 0x632be5abu) * 0x9e3779b1u) >> 25;
+          if (r == 0) {
+            first[lane] = make_uint2(cxy, valid ? map : 0xffffffffu);
+            if (valid) slots[h] = (uint8_t)lane;
+          } else {
+            const uint2 c1 = first[slots[h] & 31u];
+            if (c1.x == cxy && c1.y == map) keep = false;
+          }
+        }
+        all += __popc(vm);
+        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const uint32_t slot = ncoh + __popc(bal & lt);
+          cand[slot] = make_uint2(cxy, map | (j << 16));
+          cen[slot] = centre_of(map, cxy);
+        }
+        ncoh += __popc(bal);
+        __syncwarp();
+      }
+      const bool any_bad = __any_sync(0xffffffffu, bad);
+      if (lane == 0) {
+        sh_ncoh = ncoh;
+        sh_all = all;
+        sh_bad = any_bad ? 1u : 0u;
+        sh_live = 0;
+      }
+    }
+    __syncthreads();
+    const uint32_t ncoh = sh_ncoh;
+    if (sh_bad) {
+      // the reference panics on this index; record the error and leave the
+      // pixel untouched (commit skips results with an invalid map)
+      if (tid == 0) write_bad_result(s, st, b, local, pixel);
+      continue;
+    }
+    float best_s = FLT_MAX;
+    uint32_t best_i = 0;
+    if (slow) {
+      WarpSmem w;
+      w.nbr = nbr;
+      w.cand = cand;
+      w.term = nullptr;
+      w.off = offs;
+      if (tid == 0) {
+        sequential_best<kG>(s, st, w, lc, lg, nk, ncoh + s.m, best_s, best_i, ncoh, s.k - ncoh);
+        const uint32_t slot = best_i < ncoh ? best_i : s.k + best_i - ncoh;
+        ccol[slot] = __ldg(s.plevels + cen[slot]);
+      }
+    } else {
+      // the coherence candidates' texels in flight, the random ones' terms
+      // meanwhile
+      const uint32_t n_coh_terms = ncoh * nk;
+      const float rk = __fdividef(1.0f, (float)nk);
+      uint32_t t2[NC], g2[NC], c2[NC], j2[NC], col = 0;
+#pragma unroll
+      for (int u = 0; u < NC; ++u) {
+        const uint32_t i = tid + (uint32_t)u * T;
+        t2[u] = g2[u] = c2[u] = j2[u] = 0;
+        if (i < n_coh_terms) {
+          split(i, rk, nk, c2[u], j2[u]);
+          fetch(c2[u], j2[u], far, t2[u], g2[u]);
+        }
+      }
+      if ((uint32_t)tid < ncoh) col = __ldg(s.plevels + cen[tid]);
+#pragma unroll
+      for (int u = 0; u < NR; ++u) {
+        const uint32_t i = tid + (uint32_t)u * T;
+        if (i < n_rnd) {
+          uint32_t c, j;
+          split(i, rf, f, c, j);
+          put_term(s.k + c, j, tx[u], gx[u]);
+        }
+      }
+      for (uint32_t i = tid + (uint32_t)NR * T; i < n_rnd; i += T) {
+        uint32_t c, j, t, g = 0;
+        split(i, rf, f, c, j);
+        fetch(s.k + c, j, far, t, g);
+        put_term(s.k + c, j, t, g);
+      }
+#pragma unroll
+      for (int u = 0; u < NC; ++u)
+        if (tid + (uint32_t)u * T < n_coh_terms) put_term(c2[u], j2[u], t2[u], g2[u]);
+      if ((uint32_t)tid < ncoh) ccol[tid] = col;
+      for (uint32_t i = tid + (uint32_t)NC * T; i < n_coh_terms; i += T) {
+        uint32_t c, j, t, g = 0;
+        split(i, rk, nk, c, j);
+        fetch(c, j, far, t, g);
+        put_term(c, j, t, g);
+      }
+      for (uint32_t c = tid + T; c < ncoh; c += T) ccol[c] = __ldg(s.plevels + cen[c]);
+      __syncthreads();
+      // sums, one candidate per thread; the first strict minimum
+      float my_s = FLT_MAX;
+      uint32_t my_i = 0xffffffffu;
+      auto offer = [&](float v, uint32_t i) {
+        if (v < my_s || (v == my_s && i < my_i)) {
+          my_s = v;
+          my_i = i;
+        }
+      };
+      if (f == nk) {
+        for (uint32_t q = tid; q < ncoh + s.m; q += T) offer(row_sum(q < ncoh ? q : s.k + q - ncoh, 0, nk, 0.0f), q);
+        block_best(my_s, my_i, best_s, best_i);
+      } else {
+        for (uint32_t q = tid; q < ncoh; q += T) offer(row_sum(q, 0, nk, 0.0f), q);
+        block_best(my_s, my_i, best_s, best_i);
+        // random candidates below that cost after f terms: their other terms
+        uint32_t *live = (uint32_t *)(rows + (size_t)ncoh * pitch);  // the coherence rows from ncoh on are unused
+        const uint32_t live_cap = (s.k - ncoh) * pitch;
+        my_s = best_s;
+        my_i = best_i;
+        for (uint32_t t = tid; t < s.m; t += T) {
+          const float part = row_sum(s.k + t, 0, f, 0.0f);
+          if (part < best_s) {
+            const uint32_t at = atomicAdd(&sh_live, 1u);
+            if (at < live_cap) {
+              live[at] = t;
+              rows[(s.k + t) * pitch] = part;  // the sum so far, in the place of the first terms
+            } else {
+              // no room for the list: this thread scores the rest itself
+              float acc = part;
+              for (uint32_t j = f; j < nk; ++j) {
+                uint32_t tt, gg = 0;
+                fetch(s.k + t, j, far, tt, gg);
+                put_term(s.k + t, j, tt, gg);
+                acc = __fadd_rn(acc, rows[(s.k + t) * pitch + j]);
+              }
+              offer(acc, ncoh + t);
+            }
+          }
+        }
+        __syncthreads();
+        const uint32_t n_live = min(sh_live, live_cap), rest = nk - f;
+        const float rr = __fdividef(1.0f, (float)rest);
+        for (uint32_t i = tid; i < n_live * rest; i += T) {
+          uint32_t c, j, t, g = 0;
+          split(i, rr, rest, c, j);
+          const uint32_t slot = s.k + live[c];
+          fetch(slot, f + j, far, t, g);
+          put_term(slot, f + j, t, g);
+        }
+        __syncthreads();
+        for (uint32_t c = tid; c < n_live; c += T) {
+          const uint32_t t = live[c];
+          offer(row_sum(s.k + t, f, nk, rows[(s.k + t) * pitch]), ncoh + t);
+        }
+        if (sh_live) block_best(my_s, my_i, best_s, best_i);
+      }
+      if (best_i == 0xffffffffu) {  // no score below f32::MAX: the reference keeps candidate 0
+        best_s = FLT_MAX;
+        best_i = 0;
+      }
+    }
+    if (tid == 0) {
+      const uint32_t slot = best_i < ncoh ? best_i : s.k + best_i - ncoh;
+      const uint2 cd = cand[slot];
+      const uint32_t map = cd.y & 0x7fffu;
+      Result r;
+      r.pixel = pixel;
+      r.srcxy = cd.x;
+      r.idp = (cd.y & kAuxNeg) ? (cd.x >> 16) * (mt[map].x & 0x7fffu) + (cd.x & 0xffffu) : pid[cd.y >> 16];
+      r.idm = map;
+      r.color = ccol[slot];
+      r.flags = (item >= st.redo ? kResAppend : 0u) | kResMirrors;
+      r.score = best_s;
+      r.ncand = sh_all + s.m;
+      emit_result(s, st, b, local, r, false);
+      evals += r.ncand;
+    }
+  }
+  wait_once();
+  // (a batch left to a later commit is counted there)
+  if (b.fused_commit && tid == 0 && evals) atomicAdd(s.evals, (unsigned long long)evals);
+}
+
+template <int T, bool kG>
+__global__ void __launch_bounds__(T, 1024 / T)
+    k_resolve_small(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+                    const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc, uint32_t F) {
+  pdl_launch();
+  resolve_small_body<T, kG>(s, st, b, pc, F);
 }
 
 // One step of a batch of new items whose neighbours the exhaustive k-NN
@@ -2898,7 +3343,7 @@ static cudaError_t raise_smem(K *kernel, size_t bytes) {
   return e;
 }
 
-cudaError_t configure_kernels(uint32_t k, uint32_t m) {
+cudaError_t configure_kernels(uint32_t k, uint32_t m, uint32_t n_maps) {
   cudaError_t e = raise_smem(k_resolve, resolve_smem_bytes(k, m));
   if (e != cudaSuccess) return e;
   e = raise_smem(k_resolve_lean, resolve_smem_bytes(k, m));
@@ -2911,6 +3356,14 @@ cudaError_t configure_kernels(uint32_t k, uint32_t m) {
   if (e != cudaSuccess) return e;
   e = raise_smem(k_resolve_team<kTeamThreads, false>, team_smem_bytes(k, m));
   if (e != cudaSuccess) return e;
+  if (k > 0 && k <= kSmallK && small_smem_bytes(k, m, n_maps) <= kSmallMaxSmem) {
+    const size_t b = small_smem_bytes(k, m, n_maps);
+    for (auto kernel : {k_resolve_small<512, false>, k_resolve_small<512, true>, k_resolve_small<256, false>,
+                        k_resolve_small<256, true>, k_resolve_small<128, false>, k_resolve_small<128, true>}) {
+      e = raise_smem(kernel, b);
+      if (e != cudaSuccess) return e;
+    }
+  }
   const size_t fsm = team_full_smem_bytes(k, m);
   if (fsm <= kTeamFullMaxSmem) {
     e = raise_smem(k_resolve_team<kTeamFullThreads, true>, fsm);
@@ -3103,10 +3556,47 @@ void launch_resolve(const SessionDev &s, const StageDev &st, const BatchDev &b, 
     launch_pdl(k_resolve_lean, grid, kResolveWarps * kWarp, smem, stream, s, st, b, pc);
 }
 
+// The small-step form: up to kSmallK neighbours, the term rows within
+// kSmallMaxSmem.
+static bool small_fits(const SessionDev &s) {
+  return s.k > 0 && s.k <= kSmallK && small_smem_bytes(s.k, s.m, s.n_maps) <= kSmallMaxSmem;
+}
+
+template <int T>
+static void launch_small_t(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t F, cudaStream_t stream,
+                           const PendingCommit &pc) {
+  const uint32_t grid = std::max(1u, b.i1 - b.i0);
+  const size_t smem = small_smem_bytes(s.k, s.m, s.n_maps);
+  if (s.guided)
+    launch_pdl(k_resolve_small<T, true>, grid, T, smem, stream, s, st, b, pc, F);
+  else
+    launch_pdl(k_resolve_small<T, false>, grid, T, smem, stream, s, st, b, pc, F);
+}
+
+// Threads per item by the step's items: 512 while every item has an SM, 256
+// while the items are resident together, else 128.  F: see k_resolve_small.
+static void launch_small(const SessionDev &s, const StageDev &st, const BatchDev &b, bool full, cudaStream_t stream,
+                         const PendingCommit &pc) {
+  const uint32_t n = b.i1 - b.i0;
+  if (full && n <= 152u)
+    launch_small_t<512>(s, st, b, s.k, stream, pc);
+  else if (full)
+    launch_small_t<256>(s, st, b, s.k, stream, pc);
+  else
+    launch_small_t<128>(s, st, b, kSmallFirst, stream, pc);
+}
+
 void launch_resolve_team(const SessionDev &s, const StageDev &st, const BatchDev &b, bool full,
                          cudaStream_t stream, const PendingCommit &pc) {
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 && pc.n == 0) return;
+  // larger steps of more than one round of neighbours are bound by work per
+  // item, not its latency: the early-exit form below (k = m = 50: 2.49
+  // against 2.60 ms a 256^2 call; k = m = 8: 1.40 against 1.33)
+  if (small_fits(s) && (full || s.k <= kWarp)) {
+    launch_small(s, st, b, full, stream, pc);
+    return;
+  }
   uint32_t grid = n < 152u * 16u ? n : 152u * 16u;
   grid = std::max(grid, std::min(152u * 16u, cdiv(pc.n, kTeamThreads)));
   if (full && team_full_smem_bytes(s.k, s.m) <= kTeamFullMaxSmem && n <= 152u && pc.n == 0)

@@ -38,11 +38,11 @@ struct GuideDesc {
   uint64_t off;
 };
 
-enum : uint32_t { kResAppend = 1u, kResMirrors = 2u };
+enum : uint32_t { kResAppend = 1u, kResMirrors = 2u, kResBad = 4u };  // kResBad: an invalid map id was met
 
 struct Result {
-  uint32_t pixel, srcxy, idp, idm;
-  uint32_t cmap, flags;
+  uint32_t pixel, srcxy, idp, idm;  // idm: the map, for the id and the coordinate map alike
+  uint32_t color, flags;
   float score;
   uint32_t ncand;
 };
@@ -166,6 +166,10 @@ struct BatchDev {
   // tag) commits them while it runs (PendingCommit) and reads a tagged
   // pixel's batch-start colour and state from the shadow instead of the image
   uint32_t defer_tag, prev_tag;
+  // the neighbour lists, means and random candidates were made on other
+  // streams that the chain waited for before this batch's stage or chunk: a
+  // launch may read them before the launches ahead of it are done
+  int early;
   // warp resolve of the plain path: kWorkCtrs counters (zeroed), kWorkCtrStride
   // words apart, from which the warps of a resident grid take items after
   // their first, so that no warp waits for its block's slowest item; null:
@@ -343,7 +347,8 @@ void launch_pad(const uint32_t *src, uint32_t w, uint32_t h, uint32_t levels, ui
 
 // Bytes of dynamic shared memory the resolve kernel needs per CTA.
 size_t resolve_smem_bytes(uint32_t k, uint32_t m);
-// Per-device kernel attributes for a (k, m) session (current device).
-cudaError_t configure_kernels(uint32_t k, uint32_t m);
+// Per-device kernel attributes for a session of (k, m) and n_maps maps
+// (current device).
+cudaError_t configure_kernels(uint32_t k, uint32_t m, uint32_t n_maps);
 
 }  // namespace ts

@@ -1036,7 +1036,7 @@ extern "C" int ts_builder_build(ts_builder *b, ts_session **out) {
     StreamGuard sg;
     CUDA_TRY(cudaStreamCreateWithFlags(&sg.s, cudaStreamNonBlocking));
     const cudaStream_t st = sg.s;
-    CUDA_TRY(configure_kernels(p.k, (uint32_t)p.m));
+    CUDA_TRY(configure_kernels(p.k, (uint32_t)p.m, (uint32_t)input_count));
     // the target guide at the output size (session.rs:258-266), then the
     // inputs at their final sizes (Example::resolve, lib.rs:564-603);
     // examples without a guide get the automatic one (lib.rs:575-582)
@@ -1365,7 +1365,6 @@ struct RunCtx {
   bool want_knn_ahead = false, knn_ahead = false;
   std::vector<KnnChunk> knn_chunks;
   std::vector<EventHandle> knn_ev;  // per chunk: its k-NN is done
-  std::vector<EventHandle> items_ev;  // per stage: its items are on the device
   std::vector<uint2> btab;          // every batch: {first stage item, tree length at its start}
   // knn_ahead: a batch step whose commit the next step's resolve launch
   // makes (its results in one of two result buffers, alternating)
@@ -2140,6 +2139,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
           bd.ncnt = c.d_kncnt.p + g0;
           bd.mean = c.d_kmean.p + g0;
           bd.dist = nullptr;
+          bd.early = c.rc_ahead ? 1 : 0;
         }
         stp.exhaustive = bp.exhaustive;
         bd.grid_first = bp.grid_first ? 1 : 0;
@@ -2620,8 +2620,11 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
       launch_rank_init(c.sd, (uint32_t)c.locked, st);
       if (c.locked) ++c.launches;
       CUDA_TRY(side_stream(s->prm.device, prio_low, &kg.s));
+      EventHandle ready;
+      CUDA_TRY(cudaEventCreateWithFlags(&ready.e, cudaEventDisableTiming));
+      CUDA_TRY(cudaEventRecord(ready.e, st));
+      CUDA_TRY(cudaStreamWaitEvent(kg.s, ready.e, 0));
       c.knn_ev.resize(c.knn_chunks.size());
-      c.items_ev.resize(c.plan.size());
     }
     CUDA_TRY(cudaEventRecord(ev_up.a, st));
     LaunchTimer lt;
@@ -2661,16 +2664,18 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
       }
       pick_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - p0).count();
       const StagePlan &sp = c.plan[si];
+      // With the k-NN made ahead the items go up on its stream, where they
+      // wait for nothing of the step chain: the lists of a stage are made
+      // while the stages before it run (a first chunk that waited for the
+      // stage before it held the chain up for 25 to 55 us).  The chain reads
+      // a stage's items after its first chunk's event.
+      const cudaStream_t ist = c.knn_ahead ? kg.s : st;
       if (sp.n_items) {
         memcpy(pitems.p + sp.items_off, c.items.data() + sp.items_off, (size_t)sp.n_items * 4);
         CUDA_TRY(cudaMemcpyAsync(c.d_items.p + sp.items_off, pitems.p + sp.items_off, (size_t)sp.n_items * 4,
-                                 cudaMemcpyHostToDevice, st));
+                                 cudaMemcpyHostToDevice, ist));
       }
       if (c.knn_ahead) {
-        // the stage's neighbour lists on the k-NN stream, from its items on
-        CUDA_TRY(cudaEventCreateWithFlags(&c.items_ev[si].e, cudaEventDisableTiming));
-        CUDA_TRY(cudaEventRecord(c.items_ev[si].e, st));
-        CUDA_TRY(cudaStreamWaitEvent(kg.s, c.items_ev[si].e, 0));
         lt.stage = sp.p_stage;
         run_enqueue_knn(c, kg.s, lt, (int)si);
       }
