@@ -128,7 +128,7 @@ __device__ __forceinline__ bool in_tree(const SessionDev &s, uint32_t p, uint32_
 __device__ __forceinline__ bool occupied_n(const SessionDev &s, int x, int y, uint32_t n) {
   if (!occupied(s, x, y)) return false;
   if (!s.rank) return true;
-  const int xs = modi(x, (int)s.W), ys = modi(y, (int)s.H);  // a mirror stands for its wrapped pixel
+  const int xs = wrap1(x, (int)s.W), ys = wrap1(y, (int)s.H);  // a mirror stands for its wrapped pixel
   return in_tree(s, (uint32_t)ys * s.W + (uint32_t)xs, n);
 }
 
@@ -282,7 +282,6 @@ __device__ __forceinline__ unsigned long long nb_key(uint32_t d2, int x, int y) 
 constexpr int kWinRows = 2 * kKnnTabRadius + 1;
 constexpr int kWinWords = (2 * kKnnTabRadius + 1 + 31) / 32;
 constexpr uint32_t kWalkDirect = 128;  // expected entries still to scan above which the window is built
-constexpr size_t kWalkWinBytes = (size_t)kWalkWarps * kWinRows * kWinWords * 4;  // dynamic shared memory
 
 // Bits of bitmap row `row` for x in [x0, x0 + 32) (bit i = x0 + i), zero
 // outside [0, W).
@@ -330,99 +329,196 @@ __device__ __forceinline__ uint32_t window_word(const SessionDev &s, int x0, int
   return (ys >= 0 && ys > s.y_t) ? row_bits(s.mir + (size_t)ys * s.wpr, x0, s) : 0u;
 }
 
-// kWin: small (latency-bound) steps, whose sparse items switch to a
+// Bound on |dx| and |dy| of the first c table entries: a disc of radius r holds
+// at least pi (r - 0.71)^2 lattice points.
+__device__ __forceinline__ int walk_reach(uint32_t c) {
+  return min(kKnnTabRadius, (int)(sqrtf((float)c * 0.31830989f) + 0.71f) + 1);
+}
+
+constexpr int kWalkPend = 3 * kWarp;  // hits of a window walk waiting for their tree check
+constexpr size_t kWalkWinBytes = (size_t)kWalkWarps * (kWinRows * kWinWords + kWalkPend) * 4;  // dynamic shared memory
+// A warp takes a run of consecutive items (as many as spread the launch over
+// its warps, at most 32): their pixels are one load, their batch follows from
+// the one before, and their means are divided together at the end, one per
+// lane (the 64-bit integer division is some 300 instructions, whatever the
+// active lanes).  A round looks 64 table entries up, two per lane.  Items
+// whose round stays inside the image, nearly all of them, need no bounds or
+// wrapping: with the k-NN made ahead one load and one comparison of the tree
+// position per entry, else one bitmap word.  The last stage of a 2048^2 output
+// (2^22 items, beside its resolves): 11.6 -> 6.3 ms.
+//
+// kWin: small (latency-bound) launches, whose sparse items switch to a
 // window in dynamic shared memory (kWalkWinBytes) once the hits so far say
-// more than two further rounds are needed.
+// more than two further rounds are needed.  With the k-NN made ahead the
+// window holds later points too: its hits wait in a list and are checked 32
+// at a time, so that a round without a full list waits for no load.
 template <bool kWin>
 __device__ __forceinline__ void knn_walk_body(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t vb,
                                               uint32_t vg) {
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t nb = b.i1 - b.i0;
-  for (uint32_t local = vb * kWalkWarps + (threadIdx.x >> 5); local < nb; local += vg * kWalkWarps) {
-    const uint32_t pixel = st.items[b.i0 + local];
-    int px, py;
-    pixel_xy(s, pixel, px, py);
-    int32_t *nbo = b.nbuf + (size_t)local * s.k;
-    const uint32_t n_tree = item_nres(b, b.i0 + local);
-    uint32_t count = 0;
-    const uint32_t tab_n = b.grid_first ? 0u : s.knn_tab_n;
-    // 64 table entries per round, two per lane, both looked up before either
-    // is used; `hit` answers membership for an offset
-    auto round = [&](uint32_t c, auto &&hit) {
-      const uint32_t i0 = c + lane, i1 = c + kWarp + lane;
-      const int32_t o0 = i0 < tab_n ? __ldg(&s.knn_tab[i0]) : 0;
-      const int32_t o1 = i1 < tab_n ? __ldg(&s.knn_tab[i1]) : 0;
-      const bool h0 = i0 < tab_n && hit(off_dx(o0), off_dy(o0));
-      const bool h1 = i1 < tab_n && hit(off_dx(o1), off_dy(o1));
-      const uint32_t b0 = __ballot_sync(0xffffffffu, h0);
-      const uint32_t b1 = __ballot_sync(0xffffffffu, h1);
-      const uint32_t r0 = count + __popc(b0 & lt), r1 = count + __popc(b0) + __popc(b1 & lt);
-      if (h0 && r0 < s.k) nbo[r0] = o0;
-      if (h1 && r1 < s.k) nbo[r1] = o1;
-      count += __popc(b0) + __popc(b1);
-    };
-    // rounds look the bitmap up directly while the hits so far say that
-    // two more rounds or fewer will do (dense steps end here)
-    uint32_t c = 0;
-    while (c < tab_n) {
-      round(c, [&](int dx, int dy) { return occupied_n(s, px + dx, py + dy, n_tree); });
-      c += 2 * kWarp;
-      if (count >= s.k) break;
-      if (kWin && (count == 0 || (uint64_t)(s.k - count) * c > (uint64_t)count * kWalkDirect)) break;
-    }
-    if (kWin && count < s.k && c < tab_n) {
-      // sparse: the membership bits of the whole table's square, built in
-      // one pass of independent loads, then the rest of the walk from
-      // shared memory
-      extern __shared__ uint32_t walk_win[];
-      uint32_t *win = walk_win + (threadIdx.x >> 5) * (kWinRows * kWinWords);
-      for (uint32_t wi = lane; wi < kWinRows * kWinWords; wi += kWarp) {
-        const int row = (int)(wi / kWinWords), word = (int)(wi - row * kWinWords);
-        win[wi] = window_word(s, px - kKnnTabRadius + 32 * word, py - kKnnTabRadius + row);
-      }
-      __syncwarp();
-      for (; c < tab_n; c += 2 * kWarp) {
-        round(c, [&](int dx, int dy) {
-          const int i = dx + kKnnTabRadius;
-          // (a set bit of a later point fails its tree check)
-          return ((win[(dy + kKnnTabRadius) * kWinWords + (i >> 5)] >> (i & 31)) & 1u) != 0u &&
-                 (!s.rank || occupied_n(s, px + dx, py + dy, n_tree));
-        });
-        if (count >= s.k) break;
-      }
-      __syncwarp();  // the window is rebuilt for the warp's next item
-    }
-    if (count >= s.k) {
-      // the distances once the k offsets are known, 32 per f64 warp
-      // instruction (an f64 instruction costs the same whatever its active
-      // lanes, and GB300's f64 pipe is narrow)
-      __syncwarp();
-      // (sessions with exact sums store no distances: the resolve derives
-      // each one from its offset, exact_dist;
-      // nor do lists made ahead: k_mean_ahead and the resolve derive them
-      // from the coordinate tables)
-      unsigned long long part = 0;
-      for (uint32_t j = lane; j < (s.exact_sum || b.dist ? s.k : 0u); j += kWarp) {
-        const int32_t o = nbo[j];
-        if (s.exact_sum)
-          part += exact_units(s, off_dx(o), off_dy(o));
+  const uint32_t nb = b.i1 - b.i0, warps = vg * kWalkWarps;
+  const uint32_t per = min(32u, (nb + warps - 1) / warps);
+  const uint32_t tab_n = b.grid_first ? 0u : s.knn_tab_n;
+  const bool ahead = s.rank != nullptr;
+  int32_t head[4];  // the first two rounds' entries
+#pragma unroll
+  for (int u = 0; u < 4; ++u) head[u] = (uint32_t)(u * kWarp + lane) < tab_n ? __ldg(&s.knn_tab[u * kWarp + lane]) : 0;
+  for (uint32_t base = (vb * kWalkWarps + (threadIdx.x >> 5)) * per; base < nb; base += warps * per) {
+    const uint32_t n = min(per, nb - base);
+    const uint32_t pixels = (uint32_t)lane < n ? st.items[b.i0 + base + lane] : 0u;
+    uint64_t my_units = 0;  // lane q: the units of item base + q, when its list is complete
+    bool mine = false;
+    uint32_t n_tree = b.n_res, bt = 0, bt_end = 0xffffffffu;  // item base + q's tree, its batch, the batch's last item + 1
+    if (b.btab) {
+      uint32_t hi = b.nbt;
+      while (hi - bt > 1) {
+        const uint32_t mid = (bt + hi) >> 1;
+        if (__ldg(&b.btab[mid].x) <= b.i0 + base)
+          bt = mid;
         else
-          b.dist[(size_t)j * nb + local] = neighbour_dist_near(s, px, py, off_dx(o), off_dy(o));
+          hi = mid;
       }
-      if (s.exact_sum) {
-        part = warp_sum_units(part);
-        if (lane == 0) b.mean[local] = exact_mean(s, part, s.k);
-      }
+      n_tree = __ldg(&b.btab[bt].y);
+      bt_end = bt + 1 < b.nbt ? __ldg(&b.btab[bt + 1].x) : 0xffffffffu;
     }
-    if (lane == 0) {
+    for (uint32_t q = 0; q < n; ++q) {
+      const uint32_t local = base + q, pixel = __shfl_sync(0xffffffffu, pixels, q);
+      while (b.i0 + local >= bt_end) {
+        ++bt;
+        n_tree = __ldg(&b.btab[bt].y);
+        bt_end = bt + 1 < b.nbt ? __ldg(&b.btab[bt + 1].x) : 0xffffffffu;
+      }
+      int px, py;
+      pixel_xy(s, pixel, px, py);
+      int32_t *nbo = b.nbuf + (size_t)local * s.k;
+      uint32_t count = 0, ux = 0, uy = 0;  // hits; the sums of dx^2 and dy^2 over this lane's kept hits
+      auto keep = [&](bool h, uint32_t r, int32_t o) {
+        if (h && r < s.k) {
+          nbo[r] = o;
+          ux += (uint32_t)(off_dx(o) * off_dx(o));
+          uy += (uint32_t)(off_dy(o) * off_dy(o));
+        }
+      };
+      auto take = [&](bool h0, bool h1, int32_t o0, int32_t o1) {
+        const uint32_t b0 = __ballot_sync(0xffffffffu, h0), b1 = __ballot_sync(0xffffffffu, h1);
+        keep(h0, count + __popc(b0 & lt), o0);
+        keep(h1, count + __popc(b0) + __popc(b1 & lt), o1);
+        count += __popc(b0) + __popc(b1);
+      };
+      // rounds look the tree up directly while the hits so far say that two
+      // more rounds or fewer will do (dense steps end here)
+      uint32_t c = 0;
+      while (c < tab_n) {
+        const uint32_t i0 = c + lane, i1 = i0 + kWarp;
+        const bool on0 = i0 < tab_n, on1 = i1 < tab_n;
+        const int32_t o0 = c == 0 ? head[0] : (c == 2 * kWarp ? head[2] : (on0 ? __ldg(&s.knn_tab[i0]) : 0));
+        const int32_t o1 = c == 0 ? head[1] : (c == 2 * kWarp ? head[3] : (on1 ? __ldg(&s.knn_tab[i1]) : 0));
+        const int reach = walk_reach(c + 2 * kWarp);
+        const bool inside = px >= reach && py >= reach && px + reach < (int)s.W && py + reach < (int)s.H;
+        bool h0, h1;
+        if (inside) {
+          if (ahead) {
+            const uint32_t r0 = __ldg(&s.rank[pixel + (uint32_t)(off_dy(o0) * (int)s.W + off_dx(o0))]);
+            const uint32_t r1 = __ldg(&s.rank[pixel + (uint32_t)(off_dy(o1) * (int)s.W + off_dx(o1))]);
+            h0 = on0 && r0 - 1u < n_tree;
+            h1 = on1 && r1 - 1u < n_tree;
+          } else {
+            const int x0 = px + off_dx(o0), x1 = px + off_dx(o1);
+            const uint32_t w0 = __ldg(&s.occ[(uint32_t)(py + off_dy(o0)) * s.wpr + (uint32_t)(x0 >> 5)]);
+            const uint32_t w1 = __ldg(&s.occ[(uint32_t)(py + off_dy(o1)) * s.wpr + (uint32_t)(x1 >> 5)]);
+            h0 = on0 && ((w0 >> (x0 & 31)) & 1u);
+            h1 = on1 && ((w1 >> (x1 & 31)) & 1u);
+          }
+        } else {
+          h0 = on0 && occupied_n(s, px + off_dx(o0), py + off_dy(o0), n_tree);
+          h1 = on1 && occupied_n(s, px + off_dx(o1), py + off_dy(o1), n_tree);
+        }
+        take(h0, h1, o0, o1);
+        c += 2 * kWarp;
+        if (count >= s.k) break;
+        if (kWin && (count == 0 || (uint64_t)(s.k - count) * c > (uint64_t)count * kWalkDirect)) break;
+      }
+      if (kWin && count < s.k && c < tab_n) {
+        // sparse: the membership bits of the whole table's square, built in
+        // one pass of independent loads, then the rest of the walk from
+        // shared memory
+        extern __shared__ uint32_t walk_win[];
+        uint32_t *win = walk_win + (threadIdx.x >> 5) * (kWinRows * kWinWords + kWalkPend);
+        int32_t *pend = (int32_t *)(win + kWinRows * kWinWords);
+        uint32_t n_pend = 0;
+        for (uint32_t wi = lane; wi < kWinRows * kWinWords; wi += kWarp) {
+          const int row = (int)(wi / kWinWords), word = (int)(wi - row * kWinWords);
+          win[wi] = window_word(s, px - kKnnTabRadius + 32 * word, py - kKnnTabRadius + row);
+        }
+        __syncwarp();
+        auto bit = [&](int32_t o) {
+          const int i = off_dx(o) + kKnnTabRadius;
+          return ((win[(off_dy(o) + kKnnTabRadius) * kWinWords + (i >> 5)] >> (i & 31)) & 1u) != 0u;
+        };
+        // the first 32 waiting hits (or all, at the end) against the tree
+        auto check = [&]() {
+          const bool on = (uint32_t)lane < n_pend;
+          const int32_t o = on ? pend[lane] : 0;
+          const uint32_t p = (uint32_t)wrap1(py + off_dy(o), (int)s.H) * s.W + (uint32_t)wrap1(px + off_dx(o), (int)s.W);
+          const bool h = on && __ldg(&s.rank[p]) - 1u < n_tree;
+          const uint32_t bal = __ballot_sync(0xffffffffu, h);
+          keep(h, count + __popc(bal & lt), o);
+          count += __popc(bal);
+          const int32_t m0 = pend[kWarp + lane], m1 = pend[2 * kWarp + lane];
+          __syncwarp();
+          pend[lane] = m0;
+          pend[kWarp + lane] = m1;
+          n_pend -= min(n_pend, (uint32_t)kWarp);
+          __syncwarp();
+        };
+        for (; c < tab_n && count < s.k; c += 2 * kWarp) {
+          const uint32_t i0 = c + lane, i1 = i0 + kWarp;
+          const int32_t o0 = i0 < tab_n ? __ldg(&s.knn_tab[i0]) : 0, o1 = i1 < tab_n ? __ldg(&s.knn_tab[i1]) : 0;
+          const bool h0 = i0 < tab_n && bit(o0), h1 = i1 < tab_n && bit(o1);
+          if (!ahead) {
+            take(h0, h1, o0, o1);
+            continue;
+          }
+          const uint32_t b0 = __ballot_sync(0xffffffffu, h0), b1 = __ballot_sync(0xffffffffu, h1);
+          if (h0) pend[n_pend + __popc(b0 & lt)] = o0;
+          if (h1) pend[n_pend + __popc(b0) + __popc(b1 & lt)] = o1;
+          n_pend += __popc(b0) + __popc(b1);
+          __syncwarp();
+          while (n_pend >= kWarp && count < s.k) check();
+        }
+        while (n_pend && count < s.k) check();
+        __syncwarp();  // the window is rebuilt for the warp's next item
+      }
       if (count >= s.k) {
-        b.ncnt[local] = s.k;
-      } else {
-        const uint32_t slot = atomicAdd(b.fb_count, 1u);
-        b.fb_list[slot] = local;
+        if (s.exact_sum) {
+          // (sessions with exact sums store no distances: the resolve derives
+          // each one from its offset, exact_dist)
+          const uint64_t units = ((uint64_t)__reduce_add_sync(0xffffffffu, ux) << s.exact_sx) +
+                                 ((uint64_t)__reduce_add_sync(0xffffffffu, uy) << s.exact_sy);
+          if ((uint32_t)lane == q) {
+            my_units = units;
+            mine = true;
+          }
+        } else if (b.dist) {
+          // the distances once the k offsets are known, 32 per f64 warp
+          // instruction (lists made ahead leave them to k_mean_ahead and the
+          // resolve)
+          __syncwarp();
+          for (uint32_t j = lane; j < s.k; j += kWarp) {
+            const int32_t o = nbo[j];
+            b.dist[(size_t)j * nb + local] = neighbour_dist_near(s, px, py, off_dx(o), off_dy(o));
+          }
+        }
+      }
+      if (lane == 0) {
+        if (count >= s.k)
+          b.ncnt[local] = s.k;
+        else
+          b.fb_list[atomicAdd(b.fb_count, 1u)] = local;
       }
     }
+    if (mine) b.mean[base + lane] = exact_mean(s, my_units, s.k);
   }
 }
 
@@ -570,103 +666,229 @@ __device__ __forceinline__ const unsigned long long *sort_first(unsigned long lo
   return keys;
 }
 
+// Radix select over keys[0, total), total > k: the cut D such that at least k
+// keys have d2 <= D, in digits of up to 8 bits from the highest significant
+// bit of any d2 (`bits`) down, until no more than `fit` keys lie at or below
+// the selected digit's range or the digits are used up (for points spread
+// over an area d2 is near uniform, so the first digit usually suffices).
+// Whole CTA; every thread gets D.
+__device__ uint32_t block_cut(const unsigned long long *keys, uint32_t total, uint32_t k, int bits, uint32_t fit,
+                              ExhShared &sh) {
+  const int lane = threadIdx.x & 31;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    sh.prefix = 0;
+    sh.rank = k;
+    sh.below = 0;
+  }
+  int hi = bits;  // the bits at and above hi are fixed by the prefix
+  for (;;) {
+    const int lo = max(hi - 8, 0);
+    const uint32_t dmask = (1u << (hi - lo)) - 1u;
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.hist[i] = 0;
+    __syncthreads();
+    const uint32_t prefix = sh.prefix;
+    for (uint32_t i0 = 0; i0 < total; i0 += blockDim.x) {
+      const uint32_t i = i0 + threadIdx.x;
+      uint32_t bin = 0xffffffffu;
+      if (i < total) {
+        const uint32_t d2 = (uint32_t)(keys[i] >> 32);
+        if (hi >= 32 || (d2 >> hi) == (prefix >> hi)) bin = (d2 >> lo) & dmask;
+      }
+      // one shared atomic per distinct digit of the warp
+      const uint32_t peers = __match_any_sync(0xffffffffu, bin);
+      if (bin != 0xffffffffu && lane == __ffs(peers) - 1) atomicAdd(&sh.hist[bin], (uint32_t)__popc(peers));
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      // warp 0: inclusive scan of 256 bins, 8 per lane
+      uint32_t v[8], acc = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        acc += sh.hist[lane * 8 + q];
+        v[q] = acc;
+      }
+      uint32_t off = acc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, off, o);
+        if (lane >= o) off += t;
+      }
+      off -= acc;  // exclusive prefix of this lane's 8 bins
+      const uint32_t rank = sh.rank, below = sh.below;
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const uint32_t lo_c = off + (q ? v[q - 1] : 0u), hi_c = off + v[q];
+        if (lo_c < rank && rank <= hi_c) {
+          sh.prefix = prefix | ((uint32_t)(lane * 8 + q) << lo);
+          sh.rank = rank - lo_c;
+          sh.le = below + hi_c;  // keys at or below the digit's range
+          sh.below = below + lo_c;
+        }
+      }
+    }
+    __syncthreads();
+    if (lo == 0 || sh.le <= fit) return sh.prefix | ((1u << lo) - 1u);
+    hi = lo;
+  }
+}
+
 // The points of the cells in rings around the item's cell, as keys in
 // all[], until k keys lie below the rings' reach: after rings 0..r every
 // point with d2 < (r * kCell + 1)^2 has been seen (the cells beyond are that
 // far away in x or y), so the k smallest collected keys are then the k
 // nearest points under the tie rule; a ring wholly outside the grid means
 // every point has been seen.  The cells of consecutive rings are numbered
-// 0, 1.. (ring r starts at 4r(r-1) + 1) and taken blockDim.x at a time; the
-// bound is tested after each such round for the last ring it completed.
-// Leaves the count in sh.total (above kExhAllKeys: the buffer overflowed)
-// and the OR of the d2 in sh.prefix.
+// 0, 1.. (ring r starts at 4r(r-1) + 1) and taken up to blockDim.x at a time,
+// as many as surely fit the buffer; the bound is tested after each such round
+// for the last ring it completed.  Once kCutFrom keys are held only the ones
+// up to the k-th smallest's cut stay, and no point beyond it enters: an item
+// in a hole of a dense image meets thousands of points per ring at its rim
+// (before, they overflowed the buffer and sent it to five passes over the
+// whole resolved list; 2756 such items of a 512^2 inpainting: 3.4 -> 0.19 ms).
+// Leaves the count in sh.total (above cap: the buffer overflowed) and the OR
+// of the d2 in sh.prefix.
 __device__ __forceinline__ uint32_t ring_base(uint32_t r) { return r == 0 ? 0u : 4u * r * (r - 1u) + 1u; }
+constexpr uint32_t kCutFrom = 512;
 
 __device__ void grid_collect(const SessionDev &s, int px, int py, uint32_t k, uint32_t n_tree, ExhShared &sh,
                              unsigned long long *all, uint32_t cap) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     sh.total = 0;
-    sh.prefix = 0;
-    sh.flag = 0;
     sh.cnt = 0;
   }
+  uint32_t dor = 0, cut = 0xffffffffu;
   __syncthreads();
   const int qcx = (px - s.cox) / kCell, qcy = (py - s.coy) / kCell;
   // rings wholly outside the grid start beyond the farthest grid edge
   const uint32_t r_max = (uint32_t)max(max(qcx, (int)s.cgw - 1 - qcx), max(qcy, (int)s.cgh - 1 - qcy));
   const uint32_t f_end_all = ring_base(r_max + 1);
-  for (uint32_t f0 = 0; f0 < f_end_all; f0 += blockDim.x) {
+  for (uint32_t f0 = 0; f0 < f_end_all;) {
     const uint32_t f = f0 + threadIdx.x;
-    uint32_t dor = 0;
+    const uint32_t held = sh.total;
+    int gx = -1, gy = -1;
+    uint32_t cnt = 0;
     if (f < f_end_all) {
       // ring r of cell number f: 4r(r-1) + 1 <= f < 4r(r+1) + 1
       uint32_t r = f == 0 ? 0u : (uint32_t)(sqrtf((float)(f - 1) * 0.25f + 0.25f) + 0.5f);
       while (r > 0 && ring_base(r) > f) --r;
       while (ring_base(r + 1) <= f) ++r;
-      int gx, gy;
       ring_cell((int)r, (int)(f - ring_base(r)), gx, gy);
       gx += qcx;
       gy += qcy;
-      const uint32_t cnt =
-          ((unsigned)gx < s.cgw && (unsigned)gy < s.cgh) ? __ldg(&s.cells[(size_t)gy * s.cgw + gx]) : 0u;
-      if (cnt) {
-        const int x0 = s.cox + gx * kCell, y0 = s.coy + gy * kCell;
-        uint32_t found = 0;
-        for (int yy = 0; yy < kCell && found < cnt; ++yy) {
-          const int y = y0 + yy, dy = y - py;
-          uint32_t bits;
-          if ((unsigned)y < s.H && x0 >= 0 && x0 + kCell <= (int)s.W) {
-            const uint32_t wi = (uint32_t)x0 >> 5, sh5 = (uint32_t)x0 & 31u;
-            const uint32_t *row = s.occ + (size_t)y * s.wpr;
-            uint64_t wv = __ldg(&row[wi]);
-            if (sh5 + kCell > 32) wv |= (uint64_t)__ldg(&row[wi + 1]) << 32;
-            bits = (uint32_t)(wv >> sh5) & ((1u << kCell) - 1u);
-            if (s.rank)  // set bits of later points (k-NN made ahead) do not count
-              for (uint32_t t = bits; t;) {
-                const int bp = __ffs(t) - 1;
-                t &= t - 1u;
-                if (!in_tree(s, (uint32_t)y * s.W + (uint32_t)(x0 + bp), n_tree)) bits &= ~(1u << bp);
-              }
-          } else {
-            bits = 0;
-            for (int xx = 0; xx < kCell; ++xx)
-              if (occupied_n(s, x0 + xx, y, n_tree)) bits |= 1u << xx;
+      cnt = ((unsigned)gx < s.cgw && (unsigned)gy < s.cgh) ? __ldg(&s.cells[(size_t)gy * s.cgw + gx]) : 0u;
+    }
+    // the round's cells: the first ones whose points fit beside the held keys
+    // (all of them once a cut keeps most points out)
+    uint32_t f1 = min(f0 + blockDim.x, f_end_all);
+    if (cut == 0xffffffffu) {
+      uint32_t incl = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) sh.hist[warp] = incl;
+      if (threadIdx.x == 0) sh.flag = 0;
+      __syncthreads();
+      for (int q = 0; q < warp; ++q) incl += sh.hist[q];
+      const uint32_t fits = __ballot_sync(0xffffffffu, held + incl <= cap);
+      if (lane == 0 && fits) atomicMax(&sh.flag, (uint32_t)(warp * kWarp + 32 - __clz(fits)));
+      __syncthreads();
+      f1 = min(f1, f0 + max(1u, sh.flag));
+    }
+    if (f < f1 && cnt) {
+      const int x0 = s.cox + gx * kCell, y0 = s.coy + gy * kCell;
+      uint32_t found = 0;
+      for (int yy = 0; yy < kCell && found < cnt; ++yy) {
+        const int y = y0 + yy, dy = y - py;
+        uint32_t bits;
+        if ((unsigned)y < s.H && x0 >= 0 && x0 + kCell <= (int)s.W) {
+          const uint32_t wi = (uint32_t)x0 >> 5, sh5 = (uint32_t)x0 & 31u;
+          const uint32_t *row = s.occ + (size_t)y * s.wpr;
+          uint64_t wv = __ldg(&row[wi]);
+          if (sh5 + kCell > 32) wv |= (uint64_t)__ldg(&row[wi + 1]) << 32;
+          bits = (uint32_t)(wv >> sh5) & ((1u << kCell) - 1u);
+          found += __popc(bits);
+          for (uint32_t t = bits; t;) {
+            const int bp = __ffs(t) - 1;
+            t &= t - 1u;
+            const int dx = x0 + bp - px;
+            // beyond the cut, or (k-NN made ahead) a later point
+            if ((uint32_t)(dx * dx + dy * dy) > cut || !in_tree(s, (uint32_t)y * s.W + (uint32_t)(x0 + bp), n_tree))
+              bits &= ~(1u << bp);
           }
-          while (bits) {
-            const int bp = __ffs(bits) - 1;
-            bits &= bits - 1u;
-            const int x = x0 + bp, dx = x - px;
-            const uint32_t d2 = (uint32_t)(dx * dx + dy * dy);
-            dor |= d2;
-            const uint32_t slot = atomicAdd(&sh.total, 1u);
-            if (slot < cap) all[slot] = nb_key(d2, x, y);
-            ++found;
-          }
+        } else {
+          bits = 0;
+          for (int xx = 0; xx < kCell; ++xx)
+            if (occupied_n(s, x0 + xx, y, n_tree)) bits |= 1u << xx;
+          found += __popc(bits);
+        }
+        while (bits) {
+          const int bp = __ffs(bits) - 1;
+          bits &= bits - 1u;
+          const int x = x0 + bp, dx = x - px;
+          const uint32_t d2 = (uint32_t)(dx * dx + dy * dy);
+          if (d2 > cut) continue;
+          dor |= d2;
+          const uint32_t slot = atomicAdd(&sh.total, 1u);
+          if (slot < cap) all[slot] = nb_key(d2, x, y);
         }
       }
     }
-    if (dor) atomicOr(&sh.prefix, dor);
     __syncthreads();
     const uint32_t n = sh.total;
     if (n > cap) break;
     // the last ring this round completed
-    const uint32_t f_done = min(f0 + blockDim.x, f_end_all);
+    const uint32_t f_done = f1;
+    f0 = f1;
     uint32_t r_done = 0;
     while (ring_base(r_done + 2) <= f_done) ++r_done;
-    if (ring_base(r_done + 1) > f_done) continue;  // not even ring 0 complete (cannot happen)
-    const uint32_t lim = (uint32_t)(r_done * kCell + 1) * (uint32_t)(r_done * kCell + 1);
+    const uint32_t lim = ring_base(r_done + 1) > f_done ? 0u : (uint32_t)(r_done * kCell + 1) * (uint32_t)(r_done * kCell + 1);
     uint32_t c = 0;
     for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) c += (uint32_t)(all[e] >> 32) < lim ? 1u : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&sh.cnt, c);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0 && c) atomicAdd(&sh.cnt, c);
     __syncthreads();
-    const uint32_t lt = sh.cnt;
+    const uint32_t below = sh.cnt;
     __syncthreads();  // every thread has read cnt
-    if (lt >= k) break;
+    if (below >= k) break;
     if (threadIdx.x == 0) sh.cnt = 0;
+    if (n >= kCutFrom && n > k) {
+      // the keys up to the k-th smallest's cut, compacted in place
+      // (the points seen lie within r_done + 2 cells in x and y)
+      const uint32_t far = (r_done + 2) * kCell;
+      cut = min(cut, block_cut(all, n, k, 32 - __clz(2 * far * far), max(k, kCutFrom / 2), sh));
+      uint32_t kept = 0;
+      for (uint32_t e0 = 0; e0 < n; e0 += blockDim.x) {
+        const uint32_t e = e0 + threadIdx.x;
+        const unsigned long long key = e < n ? all[e] : ~0ull;
+        const bool in = (uint32_t)(key >> 32) <= cut && e < n;
+        const uint32_t bal = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) sh.hist[warp] = __popc(bal);
+        __syncthreads();
+        uint32_t at = kept + __popc(bal & ((1u << lane) - 1u)), all_in = 0;
+        for (uint32_t q = 0; q < blockDim.x / kWarp; ++q) {
+          if (q < (uint32_t)warp) at += sh.hist[q];
+          all_in += sh.hist[q];
+        }
+        if (in) all[at] = key;  // (at <= e: every key of this round has been read)
+        kept += all_in;
+        __syncthreads();
+      }
+      if (threadIdx.x == 0) sh.total = kept;
+    }
     __syncthreads();
   }
+  // the OR of the keys' d2 (an upper bound on their bits)
+  __syncthreads();
+  if (threadIdx.x == 0) sh.prefix = 0;
+  __syncthreads();
+  dor = __reduce_or_sync(0xffffffffu, dor);
+  if (lane == 0 && dor) atomicOr(&sh.prefix, dor);
+  __syncthreads();
 }
 
 __device__ uint32_t knn_exhaustive_item(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t local,
@@ -764,68 +986,8 @@ __device__ uint32_t knn_exhaustive_item(const SessionDev &s, const StageDev &st,
     // keys are sorted whole
     const uint32_t dor_all = sh.prefix;
     const int bits = dor_all ? 32 - __clz(dor_all) : 1;
-    uint32_t D = 0xffffffffu;
     if (total > k && total > (uint32_t)kExhSortAll) {
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        sh.prefix = 0;
-        sh.rank = k;
-        sh.below = 0;
-      }
-      int hi = bits;  // the bits at and above hi are fixed by the prefix
-      for (;;) {
-        const int lo = max(hi - 8, 0);
-        const uint32_t dmask = (1u << (hi - lo)) - 1u;
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.hist[i] = 0;
-        __syncthreads();
-        const uint32_t prefix = sh.prefix;
-        for (uint32_t i0 = 0; i0 < total; i0 += blockDim.x) {
-          const uint32_t i = i0 + threadIdx.x;
-          uint32_t bin = 0xffffffffu;
-          if (i < total) {
-            const uint32_t d2 = (uint32_t)(all[i] >> 32);
-            if (hi >= 32 || (d2 >> hi) == (prefix >> hi)) bin = (d2 >> lo) & dmask;
-          }
-          // one shared atomic per distinct digit of the warp
-          const uint32_t peers = __match_any_sync(0xffffffffu, bin);
-          if (bin != 0xffffffffu && lane == __ffs(peers) - 1) atomicAdd(&sh.hist[bin], (uint32_t)__popc(peers));
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) {
-          // warp 0: inclusive scan of 256 bins, 8 per lane
-          uint32_t v[8], acc = 0;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            acc += sh.hist[lane * 8 + q];
-            v[q] = acc;
-          }
-          uint32_t off = acc;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, off, o);
-            if (lane >= o) off += t;
-          }
-          off -= acc;  // exclusive prefix of this lane's 8 bins
-          const uint32_t rank = sh.rank, below = sh.below;
-          __syncwarp();
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const uint32_t lo_c = off + (q ? v[q - 1] : 0u), hi_c = off + v[q];
-            if (lo_c < rank && rank <= hi_c) {
-              sh.prefix = prefix | ((uint32_t)(lane * 8 + q) << lo);
-              sh.rank = rank - lo_c;
-              sh.le = below + hi_c;  // keys at or below the digit's range
-              sh.below = below + lo_c;
-            }
-          }
-        }
-        __syncthreads();
-        if (lo == 0 || sh.le <= (uint32_t)kExhCap) {
-          D = sh.prefix | ((1u << lo) - 1u);
-          break;
-        }
-        hi = lo;
-      }
+      const uint32_t D = block_cut(all, total, k, bits, (uint32_t)kExhCap, sh);
       // keys at or below the cut, into the small buffer
       if (threadIdx.x == 0) sh.nkeys = 0;
       __syncthreads();
@@ -3413,7 +3575,7 @@ uint32_t multi_blocks(int phase, uint32_t n, uint32_t cap) {
   switch (phase) {
     case kPhaseLevelSwitch: b = cdiv(n, 256); break;
     case kPhaseRandom: b = cdiv(n, 128); break;
-    case kPhaseWalk: b = cdiv(n, kWalkWarps); break;
+    case kPhaseWalk: b = cdiv(n, kWalkWarps * std::min(8u, std::max(1u, n / 4096u))); break;
     case kPhaseExhaustive: b = n; break;
     case kPhaseMean: b = cdiv(n, 128); break;
     case kPhaseResolve: b = cdiv(n, kResolveWarps); break;
@@ -3471,11 +3633,16 @@ void launch_random_candidates(const SessionDev &s, const StageDev &st, cudaStrea
   launch_pdl(k_random_candidates, cdiv(st.n_items, 128), 128, 0, stream, s, st);
 }
 
+// Items per warp of a walk over n items: one while a warp per item fits the
+// GPU, then as many as keep its warps (152 SMs x 32) busy some four times
+// over.
+static uint32_t walk_items(uint32_t n) { return std::min(32u, std::max(1u, n / (152u * 32u * 4u))); }
+
 void launch_knn_walk(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream,
                      const PendingCommit &pc) {
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 && pc.n == 0) return;
-  const uint32_t grid = std::max(cdiv(n, kWalkWarps), cdiv(pc.n, kWalkWarps * kWarp));
+  const uint32_t grid = std::max(cdiv(n, kWalkWarps * walk_items(n)), cdiv(pc.n, kWalkWarps * kWarp));
   if (b.walk_window)
     launch_pdl(k_knn_walk<true>, grid, kWalkWarps * kWarp, kWalkWinBytes, stream, s, st, b, pc);
   else

@@ -1911,13 +1911,16 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   std::vector<std::pair<uint32_t, uint32_t>> chunk_batches;  // [first, last) batch of each chunk
   std::vector<uint32_t> stage_bt_base(plan.size(), 0);        // each stage's first batch
   if (c.knn_ahead) {
-    constexpr uint32_t kChunkMinItems = 64;
+    // the first stage's chunks start small, its first steps wait for them;
+    // later stages' lists are made while the stages before them run, where a
+    // launch's fixed time counts
+    constexpr uint32_t kChunkMinItems = 64, kChunkMinLater = 8192;
     for (size_t si = 0; si < plan.size(); ++si) {
       const StagePlan &sp = plan[si];
       const uint32_t bt_base = stage_bt_base[si] = (uint32_t)c.btab.size();
       for (const BatchPlan &bp : sp.batches) c.btab.push_back(make_uint2(bp.i0, bp.n_res));
       auto form = [&](const BatchPlan &bp) {
-        return (bp.exhaustive ? 1 : 0) | (bp.grid_first ? 2 : 0) | ((bp.i1 - bp.i0) <= p.walk_window_max ? 4 : 0);
+        return (bp.exhaustive ? 1 : 0) | (bp.grid_first ? 2 : 0);
       };
       uint32_t covered = 0;
       size_t j = 0;
@@ -1925,7 +1928,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
         const size_t j0 = j;
         uint32_t items = 0;
         while (j < sp.batches.size() && form(sp.batches[j]) == form(sp.batches[j0]) &&
-               (j == j0 || items < std::max(kChunkMinItems, covered))) {
+               (j == j0 || items < std::max(si == 0 ? kChunkMinItems : kChunkMinLater, covered))) {
           items += sp.batches[j].i1 - sp.batches[j].i0;
           ++j;
         }
