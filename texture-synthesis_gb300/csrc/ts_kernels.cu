@@ -1114,6 +1114,118 @@ __device__ uint32_t knn_exhaustive_item(const SessionDev &s, const StageDev &st,
 }
 
 // ---------------------------------------------------------------------------
+// k-NN over a short resolved list (the sparse first steps, up to kListMax
+// points), lists made ahead: a warp per item.  One pass over the tree's points
+// keeps the keys within a squared radius chosen from the density so that some
+// 1.5 k points are expected; too few or too many and the radius is bisected
+// (the count grows with it).  The keys' ranks among each other are their
+// places.  A CTA per item with a radix select over every key (the exhaustive
+// form, which still takes the items whose radius does not settle and those
+// the walk could not finish) took 74 us for a launch of a few thousand items
+// and held the first stage's steps up; this one takes 30.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kListWarps = 4;
+constexpr uint32_t kListMax = 4096;
+__host__ __device__ __forceinline__ uint32_t list_cap(uint32_t k) { return 2u * k + 96u; }
+
+__device__ __forceinline__ void knn_list_body(const SessionDev &s, const StageDev &st, const BatchDev &b) {
+  extern __shared__ unsigned long long list_keys[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u, cap = list_cap(s.k), nb = b.i1 - b.i0;
+  unsigned long long *keys = list_keys + (size_t)warp * cap;
+  for (uint32_t local = blockIdx.x * kListWarps + warp; local < nb; local += gridDim.x * kListWarps) {
+    const uint32_t pixel = st.items[b.i0 + local], n_tree = item_nres(b, b.i0 + local);
+    int px, py;
+    pixel_xy(s, pixel, px, py);
+    // squared radius of a disc that holds 1.5 k + 8 of n points spread over the image
+    const float want = 1.5f * (float)s.k + 8.0f;
+    const float r2 = want * (float)s.W * (float)s.H / (3.1415927f * (float)max(n_tree, 1u));
+    uint32_t lo = 0, hi = 0xffffffffu;  // counts: at lo (if > 0) below k, at hi (if found) above cap
+    uint32_t lim = r2 < 2.0e9f ? (uint32_t)r2 : 2000000000u;
+    if (n_tree <= s.k) lim = 0xfffffffeu;
+    uint32_t n = 0;
+    bool settled = false;
+    for (int pass = 0; pass < 24 && !settled; ++pass) {
+      n = 0;
+      auto add = [&](bool in, int x, int y) {
+        const int dx = x - px, dy = y - py;
+        const uint32_t d2 = (uint32_t)(dx * dx + dy * dy);
+        in = in && d2 <= lim;
+        const uint32_t bal = __ballot_sync(0xffffffffu, in);
+        const uint32_t at = n + __popc(bal & lt);
+        if (in && at < cap) keys[at] = nb_key(d2, x, y);
+        n += __popc(bal);
+      };
+      for (uint32_t e0 = 0; e0 < n_tree; e0 += 4 * kWarp) {
+        uint32_t pt[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t e = e0 + (uint32_t)u * kWarp + lane;
+          pt[u] = e < n_tree ? __ldg(&s.resolved[e]) : 0xffffffffu;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const bool on = pt[u] != 0xffffffffu;
+          int x = 0, y = 0;
+          if (on) pixel_xy(s, pt[u], x, y);
+          add(on, x, y);
+          if (s.tiling) {
+            // its mirrors (flush_resolved, ms.rs:306-328)
+            const int mx = x < s.x_l ? (int)s.W : (x > s.x_r ? -(int)s.W : 0);
+            const int my = y < s.y_b ? (int)s.H : (y > s.y_t ? -(int)s.H : 0);
+            const bool mb = on && (mx | my) != 0 && mir_bit(s, (uint32_t)x, (uint32_t)y);
+            if (__any_sync(0xffffffffu, mb)) {
+              add(mb && mx != 0, x + mx, y);
+              add(mb && my != 0, x, y + my);
+            }
+          }
+        }
+      }
+      if (n > cap) {
+        hi = lim;
+        if (hi - lo <= 1) break;  // more points at one distance than there is room for
+        lim = lo + (hi - lo) / 2;
+      } else if (n < s.k && lim < 0xfffffffeu && hi - lo > 1) {
+        lo = lim;
+        // grow the area; between a too small and a too large one, halve
+        lim = hi == 0xffffffffu ? (lim < 1000000000u ? lim * 2u + 2u : 0xfffffffeu) : lo + (hi - lo) / 2;
+      } else {
+        settled = n >= s.k || lim == 0xfffffffeu;
+        if (!settled) break;
+      }
+    }
+    __syncwarp();
+    if (!settled) {
+      if (lane == 0) b.fb_list[atomicAdd(b.fb_count, 1u)] = local;
+      continue;
+    }
+    // each key's place: the number of smaller ones (keys are distinct)
+    const uint32_t nout = min(n, s.k);
+    int32_t *nbo = b.nbuf + (size_t)local * s.k;
+    uint32_t ux = 0, uy = 0;
+    for (uint32_t e0 = 0; e0 < n; e0 += kWarp) {
+      const uint32_t e = e0 + lane;
+      const unsigned long long key = e < n ? keys[e] : ~0ull;
+      uint32_t r = 0;
+#pragma unroll 4
+      for (uint32_t q = 0; q < n; ++q) r += keys[q] < key ? 1u : 0u;
+      if (e < n && r < nout) {
+        const int dx = (int)(key & 0xffffu) - 32768 - px, dy = (int)((key >> 16) & 0xffffu) - 32768 - py;
+        nbo[r] = pack_off(dx, dy);
+        ux += (uint32_t)(dx * dx);
+        uy += (uint32_t)(dy * dy);
+      }
+    }
+    if (s.exact_sum) {
+      const unsigned long long units = (warp_sum_units(ux) << s.exact_sx) + (warp_sum_units(uy) << s.exact_sy);
+      if (lane == 0 && nout) b.mean[local] = exact_mean(s, units, nout);
+    }
+    if (lane == 0) b.ncnt[local] = nout;
+    __syncwarp();  // the keys are rebuilt for the warp's next item
+  }
+}
+
+// ---------------------------------------------------------------------------
 // mean: thread per item (get_distances_to_k_neighs, ms.rs:417-423): the sum
 // of the 4x-duplicated distance list in order, then / (4k).
 // ---------------------------------------------------------------------------
@@ -2500,6 +2612,13 @@ __global__ void __launch_bounds__(kWalkWarps *kWarp, 4) k_knn_walk_multi(MultiLa
   knn_walk_body<false>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
 }
 
+__global__ void __launch_bounds__(kListWarps *kWarp)
+    k_knn_list(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+               const __grid_constant__ BatchDev b) {
+  pdl_enter();
+  knn_list_body(s, st, b);
+}
+
 __global__ void __launch_bounds__(kExhThreads) k_knn_exhaustive(SessionDev s, StageDev st, BatchDev b, uint32_t cap,
                                                                  int all_items,
                                                                  const __grid_constant__ PendingCommit pc) {
@@ -2590,8 +2709,12 @@ __global__ void __launch_bounds__(kMeanThreads) k_mean_staged(SessionDev s, Stag
 // the FP64 pipe busy (an f64 warp instruction takes it 18 cycles whatever its
 // active lanes), so every lane of a warp carries an item; the launches run on
 // the side stream, off the step chain.
+// Four threads per item form the distances, four at a time each (chained
+// loads and f64 operations: with one thread and one distance at a time a
+// launch over far neighbours took 81 us).
 constexpr uint32_t kMeanPitch = kMeanThreads + 1;
-__global__ void __launch_bounds__(kMeanThreads)
+constexpr uint32_t kMeanAheadThreads = 4 * kMeanThreads;
+__global__ void __launch_bounds__(kMeanAheadThreads)
     k_mean_ahead(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
                  const __grid_constant__ BatchDev b) {
   pdl_enter();
@@ -2600,24 +2723,33 @@ __global__ void __launch_bounds__(kMeanThreads)
   __shared__ uint32_t cnt[kMeanThreads];
   const uint32_t first = blockIdx.x * kMeanThreads, n = min(kMeanThreads, b.i1 - b.i0 - first);
   const uint32_t tid = threadIdx.x;
-  cnt[tid] = 0;
-  if (tid < n) {
-    pixel_xy(s, st.items[b.i0 + first + tid], xs[tid], ys[tid]);
-    cnt[tid] = b.ncnt[first + tid];
+  if (tid < kMeanThreads) {
+    cnt[tid] = 0;
+    xs[tid] = ys[tid] = 0;  // (the entries past the last item look up pixel 0's tables)
+    if (tid < n) {
+      pixel_xy(s, st.items[b.i0 + first + tid], xs[tid], ys[tid]);
+      cnt[tid] = b.ncnt[first + tid];
+    }
   }
   __syncthreads();
   const int32_t *nbo = b.nbuf + (size_t)first * s.k;
-  uint32_t i = tid / s.k, j = tid - i * s.k;
-  for (uint32_t e = tid; e < n * s.k; e += kMeanThreads) {
-    if (j < cnt[i]) {
-      const int32_t off = nbo[e];
-      md[j * kMeanPitch + i] = neighbour_dist(s, xs[i], ys[i], off_dx(off), off_dy(off));
+  constexpr int kPer = 4;
+  for (uint32_t e0 = tid; e0 < n * s.k; e0 += kPer * kMeanAheadThreads) {
+    uint32_t it[kPer], jt[kPer];
+    int32_t off[kPer];
+    double d[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const uint32_t e = e0 + (uint32_t)u * kMeanAheadThreads;
+      it[u] = min(e / s.k, kMeanThreads - 1u);
+      jt[u] = e - it[u] * s.k;
+      off[u] = e < n * s.k && jt[u] < cnt[it[u]] ? __ldg(&nbo[e]) : 0;
     }
-    j += kMeanThreads;
-    while (j >= s.k) {
-      j -= s.k;
-      ++i;
-    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) d[u] = neighbour_dist(s, xs[it[u]], ys[it[u]], off_dx(off[u]), off_dy(off[u]));
+#pragma unroll
+    for (int u = 0; u < kPer; ++u)
+      if (e0 + (uint32_t)u * kMeanAheadThreads < n * s.k && jt[u] < cnt[it[u]]) md[jt[u] * kMeanPitch + it[u]] = d[u];
   }
   __syncthreads();
   if (tid >= n || cnt[tid] == 0) return;
@@ -3667,6 +3799,15 @@ void launch_knn_exhaustive(const SessionDev &s, const StageDev &st, const BatchD
   launch_pdl(k_knn_exhaustive, grid, kExhThreads, (size_t)cap * 8, stream, s, st, b, cap, all_items ? 1 : 0, pc);
 }
 
+bool knn_list_fits(const SessionDev &s, const BatchDev &b) { return s.rank != nullptr && b.n_res <= kListMax; }
+
+void launch_knn_list(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream) {
+  const uint32_t n = b.i1 - b.i0;
+  if (n == 0) return;
+  launch_pdl(k_knn_list, cdiv(n, kListWarps), kListWarps * kWarp, (size_t)kListWarps * list_cap(s.k) * 8, stream, s, st,
+             b);
+}
+
 void launch_mean(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream) {
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 || s.k == 0) return;
@@ -3676,7 +3817,7 @@ void launch_mean(const SessionDev &s, const StageDev &st, const BatchDev &b, cud
 void launch_mean_ahead(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream) {
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 || s.k == 0) return;
-  launch_pdl(k_mean_ahead, cdiv(n, kMeanThreads), kMeanThreads, (size_t)s.k * kMeanPitch * 8, stream, s, st, b);
+  launch_pdl(k_mean_ahead, cdiv(n, kMeanThreads), kMeanAheadThreads, (size_t)s.k * kMeanPitch * 8, stream, s, st, b);
 }
 
 void launch_dist_tables(const SessionDev &s, double *xdiv, double *ydiv, double *dxt, double *dy2t, uint32_t n_x,

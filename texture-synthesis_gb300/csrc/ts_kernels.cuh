@@ -266,6 +266,10 @@ void launch_knn_walk(const SessionDev &s, const StageDev &st, const BatchDev &b,
 // the walk left in fb_list.
 void launch_knn_exhaustive(const SessionDev &s, const StageDev &st, const BatchDev &b, bool all_items,
                            cudaStream_t stream, const PendingCommit &pc = PendingCommit{});
+// Lists made ahead over a short resolved list (knn_list_fits: b.n_res points
+// at most), a warp per item; items it cannot settle go to fb_list.
+bool knn_list_fits(const SessionDev &s, const BatchDev &b);
+void launch_knn_list(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream);
 void launch_mean(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream);
 // The means of a chunk of lists made ahead (sessions without exact sums).
 void launch_mean_ahead(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream);

@@ -2259,8 +2259,8 @@ bool can_defer_commit(const RunCtx &c, const Step &stp, const Step *next) {
 
 // k-NN ahead: the chunks of stage `stage` on the k-NN stream kst, once its
 // items are up: each chunk's tree entries, then its neighbour lists and
-// means, then its event.
-void run_enqueue_knn(RunCtx &c, cudaStream_t kst, LaunchTimer &lt, int stage) {
+// means (inexact ones on the stream mst), then its event.
+void run_enqueue_knn(RunCtx &c, cudaStream_t kst, cudaStream_t mst, LaunchTimer &lt, int stage) {
   const SessionDev &sd = c.sd;
   const cudaStream_t main_st = lt.st;
   lt.st = kst;
@@ -2272,20 +2272,36 @@ void run_enqueue_knn(RunCtx &c, cudaStream_t kst, LaunchTimer &lt, int stage) {
       lt.run(TS_KERNEL_COMMIT, [&] { launch_tree_append(sd, ch.st, ch.a0, ch.a1, ch.pos0, ch.nomir_end, kst); });
       ++c.launches;
     }
-    if (ch.all_exhaustive) {
+    const bool list = ch.all_exhaustive && knn_list_fits(sd, ch.b);
+    if (ch.all_exhaustive && !list) {
       lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, true, kst, PendingCommit{}); });
       ++c.launches;
     } else {
-      lt.run(TS_KERNEL_KNN_WALK, [&] { launch_knn_walk(sd, ch.st, ch.b, kst, PendingCommit{}); });
+      lt.run(TS_KERNEL_KNN_WALK, [&] {
+        if (list)
+          launch_knn_list(sd, ch.st, ch.b, kst);
+        else
+          launch_knn_walk(sd, ch.st, ch.b, kst, PendingCommit{});
+      });
       lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, false, kst, PendingCommit{}); });
       c.launches += 2;
     }
-    if (!sd.exact_sum) {
-      lt.run(TS_KERNEL_MEAN, [&] { launch_mean_ahead(sd, ch.st, ch.b, kst); });
-      ++c.launches;
-    }
     CUDA_TRY(cudaEventCreateWithFlags(&c.knn_ev[q].e, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, kst));
+    if (!sd.exact_sum) {
+      // on a stream of their own: the f64 chains (6.6 us at least) overlap
+      // the next chunk's lists
+      EventHandle lists;
+      CUDA_TRY(cudaEventCreateWithFlags(&lists.e, cudaEventDisableTiming));
+      CUDA_TRY(cudaEventRecord(lists.e, kst));
+      CUDA_TRY(cudaStreamWaitEvent(mst, lists.e, 0));
+      lt.st = mst;
+      lt.run(TS_KERNEL_MEAN, [&] { launch_mean_ahead(sd, ch.st, ch.b, mst); });
+      lt.st = kst;
+      ++c.launches;
+      CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, mst));
+    } else {
+      CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, kst));
+    }
   }
   lt.st = main_st;
 }
@@ -2542,6 +2558,7 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
   StreamGuard sg;  // declared first: the run's pool buffers are freed on it before it goes
   StreamGuard rg;  // side stream of the random candidates made ahead
   StreamGuard kg;  // k-NN stream (knn_ahead)
+  StreamGuard mg;  // the means of inexact lists
   // the items go up stage by stage from pinned memory, so that the device
   // runs a stage while the host picks the next one
   PinnedBuf<uint32_t> pitems;
@@ -2623,6 +2640,7 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
       launch_rank_init(c.sd, (uint32_t)c.locked, st);
       if (c.locked) ++c.launches;
       CUDA_TRY(side_stream(s->prm.device, prio_low, &kg.s));
+      if (!c.sd.exact_sum) CUDA_TRY(side_stream(s->prm.device, prio_low, &mg.s));
       EventHandle ready;
       CUDA_TRY(cudaEventCreateWithFlags(&ready.e, cudaEventDisableTiming));
       CUDA_TRY(cudaEventRecord(ready.e, st));
@@ -2680,7 +2698,7 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
       }
       if (c.knn_ahead) {
         lt.stage = sp.p_stage;
-        run_enqueue_knn(c, kg.s, lt, (int)si);
+        run_enqueue_knn(c, kg.s, mg.s, lt, (int)si);
       }
       run_enqueue_plain(c, st, lt, progress, user, (int)si);
     }
@@ -2711,6 +2729,7 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
   } catch (const Failure &f) {
     // nothing of the run may be in flight when its buffers go
     if (kg.s) cudaStreamSynchronize(kg.s);
+    if (mg.s) cudaStreamSynchronize(mg.s);
     if (rg.s) cudaStreamSynchronize(rg.s);
     if (sg.s) cudaStreamSynchronize(sg.s);
     s->err = f.msg;
