@@ -157,10 +157,10 @@ typedef struct ts_run_stats {
   /* Device time of the initial uploads and of reading the results back
    * (CUDA events; part of gpu_ms). */
   double upload_ms, readback_ms;
-  /* Parts of host_enqueue_ms: waiting for the pick chain
-   * (pick_random_unresolved, on its own host thread) to finish a stage, and
-   * the rest (uploads, launches and stream-order calls, and the read-back
-   * copies, which wait for the device). */
+  /* Parts of host_enqueue_ms: the pick chain (pick_random_unresolved) where
+   * the host makes it (0: the device does), and the rest (uploads, launches
+   * and stream-order calls, and the read-back copies, which wait for the
+   * device). */
   double host_pick_ms, host_launch_ms;
   /* Chunks of batches whose neighbour lists were made ahead on a side
    * stream (k > 0; power-of-two outputs, others from 2048 pixels on); 0 when

@@ -291,6 +291,24 @@ void launch_step_team_full(const SessionDev &s, const StageDev &st, const BatchD
 void launch_commit(const SessionDev &s, const StageDev &st, const BatchDev &b, cudaStream_t stream);
 void launch_level_switch(const SessionDev &s, uint32_t level, uint32_t n_res, cudaStream_t stream);
 
+// A stage of the pick chain on the device (pick_random_unresolved,
+// ms.rs:380-389).  un: the unresolved list at its start (len0 entries), un_next
+// receives the one after it (len0 - n_new); items [0, redo) are copied from
+// redo_from, the new ones go to items[redo..] and on to the resolved list.
+// head (len0 entries, zeroed), next and draw (n_new): scratch.
+struct PickStage {
+  uint64_t seed;
+  uint32_t redo, n_new, len0;
+  int append_redo;  // k = 0: the redo items enter the resolved list again, before the new ones
+  const uint32_t *redo_from;
+  uint32_t *items, *resolved;
+  const uint32_t *un;
+  uint32_t *un_next, *head, *next, *draw;
+};
+void launch_picks(const PickStage &ps, cudaStream_t stream);
+// un = 0, 1, .., n - 1, then un[over[2i]] = over[2i + 1] for i < n_over.
+void launch_pick_init(uint32_t *un, uint32_t n, const uint32_t *over, uint32_t n_over, cudaStream_t stream);
+
 // Initial state of the pixels set before the first stage (random init):
 // list[6i..6i+6] = {pixel, colour, state.x, state.y, state.z, state.w};
 // res[i] = pixel (the resolved list starts with them, in list order).

@@ -56,7 +56,7 @@ constexpr uint64_t kRcandBudget = 64ull << 20;  // random-candidate entries held
 constexpr uint32_t kWalkWindowItems = 4096;
 // Runs whose random candidates for every stage fit this many entries make
 // them all ahead, on a side stream, while the first stages run.
-constexpr uint64_t kRcandWhole = 256ull << 20;
+constexpr uint64_t kRcandWhole = 1024ull << 20;
 
 struct Image {
   std::vector<uint8_t> px;  // RGBA8
@@ -1341,9 +1341,7 @@ struct RunCtx {
   // as {pixel, colour, state.x, state.y, state.z, state.w}
   bool dense_init = false;
   std::vector<uint32_t> init_list;
-  // items_async: the caller uploads the items from pitems itself
-  bool items_async = false;
-  PinnedBuf<uint32_t> pitems;
+  PinnedBuf<uint32_t> pitems;  // the served form's items
   std::vector<float> luts;
   std::vector<int32_t> tab;
   size_t n_xdiv = 0, n_ydiv = 0;  // entries of the coordinate tables (0: exact sums need none)
@@ -1375,9 +1373,15 @@ struct RunCtx {
   uint32_t pend_n = 0, defer_parity = 0;
   size_t res_total = 0;                // resolved-list length at the end of the run
   std::vector<uint32_t> unresolved;    // pixels not yet picked (the pick chain's state)
+  // dev_picks: the pick chain runs on the device (run_enqueue_picks).  The
+  // unresolved list starts as `unresolved` (inpainting) or as 0, 1, .. with
+  // the entries un_over {position, pixel} that the random init's picks left
+  bool want_dev_picks = false, dev_picks = false;
+  size_t n_unresolved = 0, n_items = 0;
+  size_t pick_len = 0;       // entries of the device's unresolved list after the stages enqueued so far
+  uint32_t pick_parity = 0;  // which of d_un holds it
+  std::vector<uint32_t> un_over;
   size_t picked_stages = 0;            // stages whose items are known
-  bool parallel_picks = false;         // draws of large stages on the shared host pool (single-session runs)
-  std::vector<uint64_t> draws;         // a stage's random indices, before the swap-removes
   int32_t x_l = 0, y_b = 0;
   uint64_t dev_bytes = 0;  // device memory run_alloc takes
   // device state
@@ -1394,6 +1398,7 @@ struct RunCtx {
   PinnedBuf<uint8_t> ptab;
   DevBuf<uint32_t> d_color, d_occ, d_mir, d_res, d_items, d_ncnt, d_fbl, d_fbc, d_cells, d_init;
   DevBuf<uint32_t> d_rank, d_kncnt, d_kfbl, d_kfbc;  // knn_ahead
+  DevBuf<uint32_t> d_un[2], d_phead, d_pnext, d_pdraw, d_over;  // dev_picks
   DevBuf<uint32_t> d_wctr;  // per batch: the warp resolve's item counters (BatchDev::work_ctr)
   DevBuf<int32_t> d_knbuf;
   DevBuf<double> d_kmean;
@@ -1430,7 +1435,7 @@ bool knn_ahead_fits(const RunCtx &c, uint32_t W, uint32_t H, uint32_t k) {
   constexpr uint64_t kKnnAheadMaxBytes = 16ull << 30;
   constexpr uint64_t kKnnAheadMinPixels = 2048;
   return c.want_knn_ahead && k > 0 && (exact_sum_ok(W, H, k) || (uint64_t)W * H >= kKnnAheadMinPixels) &&
-         (uint64_t)c.items.size() * ((uint64_t)k * 4 + 16) <= kKnnAheadMaxBytes;
+         (uint64_t)c.n_items * ((uint64_t)k * 4 + 16) <= kKnnAheadMaxBytes;
 }
 
 // Host schedule of Generator::resolve (ms.rs:702-1051) and the device
@@ -1477,13 +1482,30 @@ void run_plan(ts_session *s, RunCtx &c) {
       }
     }
     locked = resolved.size();
-  } else {
+  }
+  size_t n_un = s->inpaint ? unresolved.size() : N;
+  c.dev_picks = c.want_dev_picks;
+  // the list is identity where nothing was picked: on the device it starts
+  // so, and the few entries that the random init's swap-removes change are
+  // kept in a map
+  const bool sparse = c.dev_picks && !s->inpaint;
+  std::unordered_map<uint64_t, uint32_t> moved;
+  if (!s->inpaint && !sparse) {
     unresolved.resize(N);
     for (size_t i = 0; i < N; ++i) unresolved[i] = (uint32_t)i;
   }
   auto pick = [&](uint64_t seed) -> uint32_t {
     Pcg32 r = pcg_from_u64(seed);
-    const uint64_t idx = gen_range_u64(r, unresolved.size());
+    const uint64_t idx = gen_range_u64(r, n_un--);
+    if (sparse) {
+      auto at = [&](uint64_t i) {
+        const auto it = moved.find(i);
+        return it == moved.end() ? (uint32_t)i : it->second;
+      };
+      const uint32_t v = at(idx);
+      moved[idx] = at(n_un);
+      return v;
+    }
     const uint32_t v = unresolved[idx];
     unresolved[idx] = unresolved.back();
     unresolved.pop_back();
@@ -1491,7 +1513,7 @@ void run_plan(ts_session *s, RunCtx &c) {
   };
   // ---- random init (session.rs:42-52, ms.rs:427-475): all examples ----
   if (p.has_random_init) {
-    if (p.random_init > unresolved.size())
+    if (p.random_init > n_un)
       throw Failure{TS_ERR_INVALID_RANGE, "random_init exceeds the number of pixels to synthesise"};
     for (uint64_t i = 0; i < p.random_init; ++i) {
       const uint32_t px = pick(p.seed + i);
@@ -1512,7 +1534,10 @@ void run_plan(ts_session *s, RunCtx &c) {
     locked += p.random_init;
   }
   c.locked = locked;
-  const size_t total = unresolved.size();
+  const size_t total = c.n_unresolved = n_un;
+  c.un_over.clear();
+  for (const auto &e : moved)
+    if (e.first < n_un) c.un_over.insert(c.un_over.end(), {(uint32_t)e.first, e.second});
   // ---- the schedule of Generator::resolve ----
   const int32_t x_l = (int32_t)((float)W * kTilingBoundary), y_b = (int32_t)((float)H * kTilingBoundary);
   const float sig2 = p.cauchy * p.cauchy;
@@ -1527,7 +1552,7 @@ void run_plan(ts_session *s, RunCtx &c) {
   std::vector<uint32_t> &items = c.items;
   std::vector<float> &luts = c.luts;
   size_t n_res = resolved.size();
-  size_t n_unresolved = unresolved.size();
+  size_t n_unresolved = n_un;
   size_t n_items_total = 0;
   int32_t pyramid_level = 0;
   uint32_t max_batch_items = 1, max_stage_items = 1;
@@ -1602,10 +1627,14 @@ void run_plan(ts_session *s, RunCtx &c) {
     max_stage_items = std::max<uint32_t>(max_stage_items, (uint32_t)P_eff);
     plan.push_back(std::move(sp));
   }
-  // the items themselves come from the pick chain, stage by stage (run_pick)
-  items.assign(n_items_total, 0);
+  // the items themselves come from the pick chain, stage by stage (run_pick,
+  // or on the device)
+  c.n_items = n_items_total;
   c.res_total = n_res;
-  resolved.reserve(n_res);  // the picks append without moving the locked entries
+  if (!c.dev_picks) {
+    items.assign(n_items_total, 0);
+    resolved.reserve(n_res);  // the picks append without moving the locked entries
+  }
   c.picked_stages = 0;
   // ---- host tables ----
   const uint32_t wpr = (W + 31) / 32;
@@ -1656,91 +1685,19 @@ void run_plan(ts_session *s, RunCtx &c) {
   const size_t kk = std::max<uint32_t>(k, 1), mb = max_batch_items;
   uint64_t steps_est = 0;
   for (auto &sp : plan) steps_est += sp.batches.size() + 1;
-  c.dev_bytes = N * 4 + N * sizeof(uint4) + 2 * (uint64_t)wpr * H * 4 + c.res_total * 8 + items.size() * 4 +
+  c.dev_bytes = N * 4 + N * sizeof(uint4) + 2 * (uint64_t)wpr * H * 4 + c.res_total * 8 + c.n_items * 4 +
+                (c.dev_picks ? c.n_unresolved * 20 : 0) +
                 c.luts.size() * 4 + c.tab.size() * 4 + mb * kk * 12 + mb * (4 + 8 + 4 + sizeof(Result)) +
-                c.n_batches * 4 + (c.rc_ahead ? (uint64_t)items.size() : std::max<uint64_t>(c.rc_items, mb)) * m * 8 +
+                c.n_batches * 4 + (c.rc_ahead ? (uint64_t)c.n_items : std::max<uint64_t>(c.rc_items, mb)) * m * 8 +
                 dist_table_doubles * 8 + steps_est * sizeof(StepDev) +
                 c.cells.size() * 4 + c.init_list.size() * 4;
 }
 
-// A small pool of host threads shared by every single-session run: it
-// computes the random draws of the large stages of the pick chain.  One job
-// at a time (runs that find it busy compute their draws themselves).
-class DrawPool {
- public:
-  static DrawPool &get() {
-    static DrawPool *pool = new DrawPool();  // never destroyed: its threads sleep on it until exit
-    return *pool;
-  }
-  // fn(a, b) over [0, n) in chunks of `grain`, on the pool and the caller;
-  // false (nothing done) when another run holds the pool
-  bool run(size_t n, size_t grain, const std::function<void(size_t, size_t)> &fn) {
-    std::unique_lock<std::mutex> job(job_mu_, std::try_to_lock);
-    if (!job.owns_lock() || workers_.empty()) return false;
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      fn_ = &fn;
-      n_ = n;
-      grain_ = grain;
-      next_ = 0;
-      left_ = (n + grain - 1) / grain;
-    }
-    cv_.notify_all();
-    work();
-    std::unique_lock<std::mutex> lk(mu_);
-    done_cv_.wait(lk, [&] { return left_ == 0; });
-    fn_ = nullptr;
-    return true;
-  }
-
- private:
-  DrawPool() {
-    const unsigned hc = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nw = std::min(7u, hc > 2 ? hc - 2 : 0u);
-    for (unsigned i = 0; i < nw; ++i) workers_.emplace_back([this] { loop(); });
-    for (auto &t : workers_) t.detach();  // they sleep until the process exits
-  }
-  void loop() {
-    for (;;) {
-      {
-        std::unique_lock<std::mutex> lk(mu_);
-        cv_.wait(lk, [&] { return fn_ != nullptr && next_ * grain_ < n_; });
-      }
-      work();
-    }
-  }
-  // Chunks are claimed under the mutex, so a claim always belongs to the
-  // job that is current when it is made.
-  void work() {
-    for (;;) {
-      const std::function<void(size_t, size_t)> *fn;
-      size_t a, b;
-      {
-        std::lock_guard<std::mutex> lk(mu_);
-        if (!fn_ || next_ * grain_ >= n_) return;
-        fn = fn_;
-        a = next_ * grain_;
-        b = std::min(n_, a + grain_);
-        ++next_;
-      }
-      (*fn)(a, b);
-      std::lock_guard<std::mutex> lk(mu_);
-      if (--left_ == 0) done_cv_.notify_all();
-    }
-  }
-  std::mutex job_mu_, mu_;
-  std::condition_variable cv_, done_cv_;
-  std::vector<std::thread> workers_;
-  const std::function<void(size_t, size_t)> *fn_ = nullptr;
-  size_t n_ = 0, grain_ = 1, next_ = 0, left_ = 0;
-};
-
 // pick_random_unresolved (ms.rs:380-389) for a stage's items: redo item i
 // is resolved[i + locked]; new item i swap-removes
 // Pcg32::seed_from_u64(seed + i).gen_range(0..len) from the unresolved list.
-// len is known in advance (the list shrinks by one per new item), so the
-// draws are independent of one another and of the list; only the
-// swap-removes that consume them run in order.
+// The served form's chain; the other forms pick on the device
+// (run_enqueue_picks).
 void run_pick(RunCtx &c) {
   const StagePlan &sp = c.plan[c.picked_stages++];
   std::vector<uint32_t> &unresolved = c.unresolved;
@@ -1749,30 +1706,17 @@ void run_pick(RunCtx &c) {
   for (uint32_t i = 0; i < redo; ++i) it[i] = c.resolved[i + c.locked];
   const size_t n_new = sp.n_items - redo, len0 = unresolved.size();
   if (n_new > len0) throw Failure{TS_ERR_INVALID_RANGE, "more new items than unresolved pixels"};
-  c.draws.resize(n_new);
-  uint64_t *dr = c.draws.data();
-  const std::function<void(size_t, size_t)> draw = [&](size_t a, size_t b) {
-    for (size_t q = a; q < b; ++q) {
-      Pcg32 r = pcg_from_u64(sp.seed + (uint64_t)(redo + q));
-      dr[q] = gen_range_u64(r, len0 - q);
-    }
-  };
-  constexpr size_t kGrain = 8192;
-  if (!(c.parallel_picks && n_new >= 4 * kGrain && DrawPool::get().run(n_new, kGrain, draw))) draw(0, n_new);
   uint32_t *un = unresolved.data();
   size_t len = len0;
   for (size_t q = 0; q < n_new; ++q) {
-    const uint64_t idx = dr[q];
+    Pcg32 r = pcg_from_u64(sp.seed + (uint64_t)(redo + q));
+    const uint64_t idx = gen_range_u64(r, len);
     it[redo + q] = un[idx];
     un[idx] = un[--len];
   }
   unresolved.resize(len);
   for (const BatchPlan &bp : sp.batches)
     for (uint32_t t = bp.append_from; t < bp.i1; ++t) c.resolved.push_back(it[t]);
-}
-
-void run_pick_all(RunCtx &c) {
-  while (c.picked_stages < c.plan.size()) run_pick(c);
 }
 
 // Let the device's default stream-ordered pool keep freed memory (by
@@ -1900,7 +1844,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     }
   } zl, tl, wl;
   const size_t kk = std::max<uint32_t>(k, 1), mb = max_batch_items;
-  const size_t rc_n = c.rc_ahead ? c.items.size() * m : (size_t)std::max<uint64_t>(rc_items, mb) * m;
+  const size_t rc_n = c.rc_ahead ? c.n_items * m : (size_t)std::max<uint64_t>(rc_items, mb) * m;
   // k-NN ahead: the batch table and the chunks (consecutive batches of a
   // stage with one k-NN form, each at least as large as the stage's items
   // before it, so that a chunk's k-NN overlaps the resolves of the ones
@@ -1940,7 +1884,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
       }
     }
   }
-  const size_t n_chunks = c.knn_chunks.size(), n_kitems = c.knn_ahead ? c.items.size() : 0;
+  const size_t n_chunks = c.knn_chunks.size(), n_kitems = c.knn_ahead ? c.n_items : 0;
   // zeroed: colour and state first (uploaded instead when dense_init)
   const size_t z_color = zl.add(N * 4), z_state = zl.add(N * sizeof(uint4)), z_rscore = zl.add(c.res_total * 4),
                z_fbc = zl.add(c.n_batches * 4), z_err = zl.add(sizeof(int)), z_evals = zl.add(8),
@@ -1955,15 +1899,18 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     return o;
   };
   const size_t t_lut = T(c.luts), t_tab = T(c.tab), t_cells = T(c.cells), t_occ = T(c.occ), t_mir = T(c.mir), t_init = T(c.init_list),
-               t_btab = T(c.btab);
+               t_btab = T(c.btab), t_over = T(c.un_over);
   // scratch
-  const size_t w_res = wl.add(c.res_total * 4), w_items = wl.add(c.items.size() * 4), w_nbuf = wl.add(mb * kk * 4),
+  const size_t w_res = wl.add(c.res_total * 4), w_items = wl.add(c.n_items * 4), w_nbuf = wl.add(mb * kk * 4),
                w_ncnt = wl.add(mb * 4), w_dist = wl.add(c.knn_ahead ? 0 : mb * kk * 8), w_mean = wl.add(mb * 8), w_fbl = wl.add(mb * 4),
                w_result = wl.add((c.knn_ahead ? 2 : 1) * mb * sizeof(Result)), w_rcand = wl.add(rc_n * 8),
                w_knbuf = wl.add(n_kitems * kk * 4), w_kncnt = wl.add(n_kitems * 4), w_kmean = wl.add(n_kitems * 8),
                w_kfbl = wl.add(n_kitems * 4), w_xdiv = wl.add(c.n_xdiv * 8), w_ydiv = wl.add(c.n_ydiv * 8),
                w_dxt = wl.add(c.n_xdiv ? (size_t)W * (2 * R + 1) * 8 : 0),
                w_dy2t = wl.add(c.n_xdiv ? (size_t)H * (2 * R + 1) * 8 : 0);
+  const size_t n_un = c.dev_picks ? c.n_unresolved : 0;
+  const size_t w_un0 = wl.add(n_un * 4), w_un1 = wl.add(n_un * 4), w_phead = wl.add(n_un * 4),
+               w_pnext = wl.add(n_un * 4), w_pdraw = wl.add(n_un * 4);
   CUDA_TRY(A(c.d_zero, zl.off));
   CUDA_TRY(A(c.d_tabs, tl.off));
   CUDA_TRY(A(c.d_work, wl.off));
@@ -1991,12 +1938,18 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.d_kncnt.view(wk + w_kncnt, n_kitems);
   c.d_kmean.view(wk + w_kmean, n_kitems);
   c.d_kfbl.view(wk + w_kfbl, n_kitems);
+  c.d_un[0].view(wk + w_un0, n_un);
+  c.d_un[1].view(wk + w_un1, n_un);
+  c.d_phead.view(wk + w_phead, n_un);
+  c.d_pnext.view(wk + w_pnext, n_un);
+  c.d_pdraw.view(wk + w_pdraw, n_un);
+  c.d_over.view(tb + t_over, c.un_over.size());
   c.d_xdiv.view(wk + w_xdiv, c.n_xdiv);
   c.d_ydiv.view(wk + w_ydiv, c.n_ydiv);
   c.d_dxt.view(wk + w_dxt, c.n_xdiv ? (size_t)W * (2 * R + 1) : 0);
   c.d_dy2t.view(wk + w_dy2t, c.n_xdiv ? (size_t)H * (2 * R + 1) : 0);
   c.d_res.view(wk + w_res, c.res_total);
-  c.d_items.view(wk + w_items, c.items.size());
+  c.d_items.view(wk + w_items, c.n_items);
   c.d_nbuf.view(wk + w_nbuf, mb * kk);
   c.d_ncnt.view(wk + w_ncnt, mb);
   c.d_dist.view(wk + w_dist, c.knn_ahead ? 0 : mb * kk);
@@ -2219,7 +2172,7 @@ void run_stage_tables(RunCtx &c) {
 
 // Uploads of the initial state, enqueued on st: one zero fill, one copy of
 // the tables (colour and state too when dense_init), the random-init
-// pixels; the items unless the caller sends them (items_async).
+// pixels.
 void run_upload(RunCtx &c, cudaStream_t st) {
   run_stage_tables(c);
   if (c.dense_init) {
@@ -2237,13 +2190,51 @@ void run_upload(RunCtx &c, cudaStream_t st) {
   }
   if (c.dense_init) {
     if (c.locked) CUDA_TRY(cudaMemcpyAsync(c.d_res.p, c.resolved.data(), c.locked * 4, cudaMemcpyHostToDevice, st));
+    if (c.dev_picks && c.n_unresolved)  // here, not with the picks: those may be captured into a graph
+      CUDA_TRY(cudaMemcpyAsync(c.d_un[0].p, c.unresolved.data(), c.n_unresolved * 4, cudaMemcpyHostToDevice, st));
   } else if (!c.init_list.empty()) {
     // the resolved list starts with the random-init pixels, in list order
     launch_scatter_init(c.d_init.p, (uint32_t)(c.init_list.size() / 6), c.d_color.p, c.d_state.p, c.d_res.p, st);
     ++c.launches;
   }
-  if (!c.items_async && !c.items.empty() && c.picked_stages == c.plan.size())
-    CUDA_TRY(cudaMemcpyAsync(c.d_items.p, c.items.data(), c.items.size() * 4, cudaMemcpyHostToDevice, st));
+}
+
+// The pick chain on the device (dev_picks): the unresolved list's start, then
+// a stage at a time, in stage order, on one stream.
+void run_enqueue_picks_init(RunCtx &c, cudaStream_t st) {
+  c.pick_len = c.n_unresolved;
+  if (c.n_unresolved == 0) return;
+  if (c.s->inpaint) return;  // run_upload copied it
+  launch_pick_init(c.d_un[0].p, (uint32_t)c.n_unresolved, c.d_over.p, (uint32_t)(c.un_over.size() / 2), st);
+  ++c.launches;
+}
+
+void run_enqueue_picks(RunCtx &c, cudaStream_t st) {
+  const size_t q = c.picked_stages++;
+  const StagePlan &sp = c.plan[q];
+  if (sp.n_items == 0) return;
+  PickStage ps{};
+  ps.seed = sp.seed;
+  ps.redo = std::min(sp.redo, sp.n_items);
+  ps.n_new = sp.n_items - ps.redo;
+  if (ps.n_new > c.pick_len) throw Failure{TS_ERR_INVALID_RANGE, "more new items than unresolved pixels"};
+  ps.len0 = (uint32_t)c.pick_len;
+  ps.redo_from = c.d_res.p + c.locked;
+  ps.items = c.d_items.p + sp.items_off;
+  ps.resolved = c.d_res.p + sp.n_res_start;
+  ps.append_redo = c.k == 0;
+  ps.un = c.d_un[c.pick_parity].p;
+  ps.un_next = c.d_un[c.pick_parity ^ 1u].p;
+  ps.head = c.d_phead.p;
+  ps.next = c.d_pnext.p;
+  ps.draw = c.d_pdraw.p;
+  if (ps.n_new) {
+    CUDA_TRY(cudaMemsetAsync(c.d_phead.p, 0, c.pick_len * 4, st));
+    c.pick_parity ^= 1u;
+    c.pick_len -= ps.n_new;
+  }
+  launch_picks(ps, st);
+  c.launches += 2;
 }
 
 // Whether the commit of step `stp` can be left to the first k-NN launch of
@@ -2559,28 +2550,7 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
   StreamGuard rg;  // side stream of the random candidates made ahead
   StreamGuard kg;  // k-NN stream (knn_ahead)
   StreamGuard mg;  // the means of inexact lists
-  // the items go up stage by stage from pinned memory, so that the device
-  // runs a stage while the host picks the next one
-  PinnedBuf<uint32_t> pitems;
   RunCtx c;
-  // The pick chain (pick_random_unresolved, ms.rs:380-389) on its own host
-  // thread from the plan on, stage after stage, so that a stage's picks
-  // never wait behind the launches of the one before; the launching thread
-  // takes each stage once it is picked.  Declared after c: it is joined
-  // before c goes.
-  struct PickThread {
-    std::thread th;
-    std::mutex mu;
-    std::condition_variable cv;
-    size_t done = 0;  // stages picked
-    bool failed = false;
-    Failure fail{};
-    std::atomic<bool> stop{false};
-    ~PickThread() {
-      stop = true;
-      if (th.joinable()) th.join();
-    }
-  } pk;
   try {
     CUDA_TRY(cudaSetDevice(s->prm.device));
     keep_pool(s->prm.device);
@@ -2601,32 +2571,10 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
     };
     c.want_rc_ahead = true;
     c.want_knn_ahead = true;
-    c.parallel_picks = true;
+    c.want_dev_picks = true;
     run_plan(s, c);
-    c.items_async = true;  // each stage's items go up once the pick thread has them
-    pk.th = std::thread([&c, &pk] {
-      try {
-        for (size_t q = 0; q < c.plan.size() && !pk.stop; ++q) {
-          run_pick(c);
-          std::lock_guard<std::mutex> lk(pk.mu);
-          pk.done = q + 1;
-          pk.cv.notify_one();
-        }
-      } catch (const Failure &f) {
-        std::lock_guard<std::mutex> lk(pk.mu);
-        pk.failed = true;
-        pk.fail = f;
-        pk.cv.notify_one();
-      } catch (...) {
-        std::lock_guard<std::mutex> lk(pk.mu);
-        pk.failed = true;
-        pk.fail = Failure{TS_ERR_OUT_OF_MEMORY, "out of host memory"};
-        pk.cv.notify_one();
-      }
-    });
     const double plan_ms = lap();
     run_alloc(c, st);
-    CUDA_TRY(pitems.alloc(c.items.size()));
     run_stage_tables(c);  // its pinned block too, before the device clock starts
     const double alloc_ms = lap();
     EventPair ev, ev_up, ev_rb;
@@ -2675,27 +2623,16 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
       }
     }
     lt.st = st;
-    double pick_ms = 0.0;
+    // With the k-NN made ahead the picks run on its stream, where they wait
+    // for nothing of the step chain: the lists of a stage are made while the
+    // stages before it run (a first chunk that waited for the stage before it
+    // held the chain up for 25 to 55 us).  The chain reads a stage's items
+    // after its first chunk's event.
+    const cudaStream_t pick_st = c.knn_ahead ? kg.s : st;
+    run_enqueue_picks_init(c, pick_st);
     for (size_t si = 0; si < c.plan.size(); ++si) {
-      const auto p0 = std::chrono::steady_clock::now();
-      {
-        std::unique_lock<std::mutex> lk(pk.mu);
-        pk.cv.wait(lk, [&] { return pk.done > si || pk.failed; });
-        if (pk.done <= si) throw pk.fail;
-      }
-      pick_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - p0).count();
       const StagePlan &sp = c.plan[si];
-      // With the k-NN made ahead the items go up on its stream, where they
-      // wait for nothing of the step chain: the lists of a stage are made
-      // while the stages before it run (a first chunk that waited for the
-      // stage before it held the chain up for 25 to 55 us).  The chain reads
-      // a stage's items after its first chunk's event.
-      const cudaStream_t ist = c.knn_ahead ? kg.s : st;
-      if (sp.n_items) {
-        memcpy(pitems.p + sp.items_off, c.items.data() + sp.items_off, (size_t)sp.n_items * 4);
-        CUDA_TRY(cudaMemcpyAsync(c.d_items.p + sp.items_off, pitems.p + sp.items_off, (size_t)sp.n_items * 4,
-                                 cudaMemcpyHostToDevice, ist));
-      }
+      run_enqueue_picks(c, pick_st);
       if (c.knn_ahead) {
         lt.stage = sp.p_stage;
         run_enqueue_knn(c, kg.s, mg.s, lt, (int)si);
@@ -2712,8 +2649,8 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
     c.g->stats.host_plan_ms = plan_ms;
     c.g->stats.host_alloc_ms = alloc_ms;
     c.g->stats.host_enqueue_ms = enqueue_ms;
-    c.g->stats.host_pick_ms = pick_ms;
-    c.g->stats.host_launch_ms = enqueue_ms - pick_ms;
+    c.g->stats.host_pick_ms = 0.0;  // the device picks
+    c.g->stats.host_launch_ms = enqueue_ms;
     c.g->stats.knn_chunks = c.knn_chunks.size();
     c.g->stats.host_wait_ms = wait_ms;
     c.g->stats.host_finish_ms = lap();
@@ -2962,8 +2899,8 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
           try {
             ctx[j].reset(new RunCtx());
             ctx[j]->want_rc_ahead = true;
+            ctx[j]->want_dev_picks = true;
             run_plan(sessions[j], *ctx[j]);
-            run_pick_all(*ctx[j]);
             run_alloc(*ctx[j], nullptr);
             RunCtx &c = *ctx[j];
             run_stage_tables(c);
@@ -2973,9 +2910,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
             c.stv.resize(c.N);
             c.g->resolved.resize(c.res_total);
             c.g->scores.resize(c.res_total);
-            if (cudaSuccess != c.pitems.alloc(c.items.size())) throw Failure{TS_ERR_CUDA, "pinned host memory"};
-            memcpy(c.pitems.p, c.items.data(), c.items.size() * 4);
-            c.items_async = true;
+
           } catch (const Failure &f) {
             fails[j] = f;
           } catch (const std::bad_alloc &) {
@@ -3206,16 +3141,14 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     CUDA_TRY(cudaEventCreateWithFlags(&fork.e, cudaEventDisableTiming));
     CUDA_TRY(cudaEventCreateWithFlags(&side_done.e, cudaEventDisableTiming));
     for (auto &e : items_ev) CUDA_TRY(cudaEventCreateWithFlags(&e.e, cudaEventDisableTiming));
-    // the items of stage 0 (part 0) and of the later stages (part 1), every
-    // session's, from its pinned copy
-    auto upload_items = [&](int part) {
+    // the picks of stage 0 (part 0) and of the later stages (part 1), every
+    // session's
+    auto pick_items = [&](int part) {
       for (size_t j = 0; j < n; ++j) {
         RunCtx &c = *ctx[j];
-        if (c.items.empty()) continue;
-        const size_t split = c.plan.size() > 1 ? c.plan[1].items_off : c.items.size();
-        const size_t a = part == 0 ? 0 : split, e = part == 0 ? split : c.items.size();
-        if (e > a)
-          CUDA_TRY(cudaMemcpyAsync(c.d_items.p + a, c.pitems.p + a, (e - a) * 4, cudaMemcpyHostToDevice, rg.s));
+        if (part == 0) run_enqueue_picks_init(c, rg.s);
+        for (size_t q = part == 0 ? 0 : 1; q < (part == 0 ? std::min<size_t>(1, c.plan.size()) : c.plan.size()); ++q)
+          run_enqueue_picks(c, rg.s);
       }
       CUDA_TRY(cudaEventRecord(items_ev[part].e, rg.s));
     };
@@ -3238,10 +3171,10 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       // first steps run
       CUDA_TRY(cudaEventRecord(fork.e, s));
       CUDA_TRY(cudaStreamWaitEvent(rg.s, fork.e, 0));
-      upload_items(0);
+      pick_items(0);
       size_t rci = 0;
       if (!rc_launches.empty() && rc_pos[0] == 0) launch_rc(rci++);
-      upload_items(1);
+      pick_items(1);
       for (; rci < rc_launches.size(); ++rci) launch_rc(rci);
       CUDA_TRY(cudaEventRecord(side_done.e, rg.s));
       for (size_t li = 0; li < launches.size(); ++li) {
@@ -3956,7 +3889,6 @@ int ts_server_submit(ts_server *S, ts_session *s, uint64_t *ticket) {
   try {
     RunCtx &c = *r->c;
     run_plan(r->s, c);  // host schedule, on the caller's thread
-    c.items_async = true;
     if (cudaSuccess != c.pitems.alloc(c.items.size())) throw Failure{TS_ERR_CUDA, "pinned host memory"};
     if (!c.plan.empty()) server_pick_stage(*r);  // stage 0 here, the rest on a picker thread
   } catch (const Failure &f) {
