@@ -1641,6 +1641,21 @@ __device__ __forceinline__ void add_cell_point(const SessionDev &s, int x, int y
   atomicAdd(&s.cells[(size_t)((y - s.coy) / kCell) * s.cgw + (x - s.cox) / kCell], 1u);
 }
 
+// A tree point in the cell counts, with its mirror copies where it has them
+// (flush_resolved, ms.rs:306-328).
+__device__ __forceinline__ void add_cells(const SessionDev &s, int x, int y, bool mirrors) {
+  add_cell_point(s, x, y);
+  if (!mirrors) return;
+  if (x < s.x_l)
+    add_cell_point(s, x + (int)s.W, y);
+  else if (x > s.x_r)
+    add_cell_point(s, x - (int)s.W, y);
+  if (y < s.y_b)
+    add_cell_point(s, x, y + (int)s.H);
+  else if (y > s.y_t)
+    add_cell_point(s, x, y - (int)s.H);
+}
+
 // update + flush_resolved of one item (ms.rs:296-377): its colour and state,
 // its place in the resolved list, the bitmap, mirrors and cell counts.
 __device__ __forceinline__ void commit_item(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t local,
@@ -1662,19 +1677,9 @@ __device__ __forceinline__ void commit_item(const SessionDev &s, const StageDev 
     int x, y;
     pixel_xy(s, p, x, y);
     atomicOr(&s.occ[(size_t)y * s.wpr + (x >> 5)], 1u << (x & 31));
-    add_cell_point(s, x, y);
-    if (s.tiling && (r.flags & kResMirrors)) {
-      atomicOr(&s.mir[(size_t)y * s.wpr + (x >> 5)], 1u << (x & 31));
-      // the tree's mirror copies (flush_resolved, ms.rs:306-328)
-      if ((int)x < s.x_l)
-        add_cell_point(s, (int)x + (int)s.W, (int)y);
-      else if ((int)x > s.x_r)
-        add_cell_point(s, (int)x - (int)s.W, (int)y);
-      if ((int)y < s.y_b)
-        add_cell_point(s, (int)x, (int)y + (int)s.H);
-      else if ((int)y > s.y_t)
-        add_cell_point(s, (int)x, (int)y - (int)s.H);
-    }
+    const bool mirrors = s.tiling && (r.flags & kResMirrors);
+    if (mirrors) atomicOr(&s.mir[(size_t)y * s.wpr + (x >> 5)], 1u << (x & 31));
+    add_cells(s, x, y, mirrors);
   }
 }
 
@@ -2279,6 +2284,33 @@ __global__ void k_scatter_init(const uint32_t *list, uint32_t n, uint32_t *color
   color[e[0]] = e[1];
   state[e[0]] = make_uint4(e[2], e[3], e[4], e[5]);
   res[i] = e[0];
+}
+
+// Initial state of an inpainting run (Generator::new_from_inpaint,
+// ms.rs:236-293), a warp per 32 pixels of a row: a locked pixel's state, its
+// place in the resolved list and the tree, and the others' place in the
+// unresolved list (both in pixel order; un null: the host keeps that list).  in.before counts the pixels to synthesise before
+// each word.  The host's loops and the upload of colours and states took 1.5 ms
+// of a 512^2 run.
+__global__ void k_inpaint_init(const __grid_constant__ SessionDev s, const __grid_constant__ InpaintDev in) {
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+  if (w >= s.wpr * s.H) return;
+  const uint32_t y = w / s.wpr, x = (w - y * s.wpr) * 32u + lane;
+  const uint32_t open = in.open[w], locked = __ballot_sync(0xffffffffu, x < s.W) & ~open;
+  if (lane == 0 && locked) {
+    s.occ[w] |= locked;  // beside the random init's bits
+    if (s.tiling) s.mir[w] |= locked;
+  }
+  if (x >= s.W) return;
+  const uint32_t p = y * s.W + x, rank = in.before[w] + (uint32_t)__popc(open & ((1u << lane) - 1u));
+  if ((open >> lane) & 1u) {
+    s.state[p] = make_uint4(0, 0, 0, 0);
+    if (in.un && rank < in.n_un) in.un[rank] = p;
+  } else {
+    s.state[p] = make_uint4(x | (y << 16), 0, 0, in.map);
+    s.resolved[p - rank] = p;
+    add_cells(s, (int)x, (int)y, s.tiling);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -4028,6 +4060,11 @@ void launch_tree_append(const SessionDev &s, const StageDev &st, uint32_t a0, ui
 void launch_rank_init(const SessionDev &s, uint32_t n, cudaStream_t stream) {
   if (n == 0) return;
   k_rank_init<<<cdiv(n, 256), 256, 0, stream>>>(s, n);
+}
+
+void launch_inpaint_init(const SessionDev &s, const InpaintDev &in, cudaStream_t stream) {
+  const uint32_t words = s.wpr * s.H;
+  if (words) k_inpaint_init<<<(words + 7) / 8, 256, 0, stream>>>(s, in);
 }
 
 void launch_scatter_init(const uint32_t *list, uint32_t n, uint32_t *color, uint4 *state, uint32_t *res,

@@ -309,6 +309,16 @@ void launch_picks(const PickStage &ps, cudaStream_t stream);
 // un = 0, 1, .., n - 1, then un[over[2i]] = over[2i + 1] for i < n_over.
 void launch_pick_init(uint32_t *un, uint32_t n, const uint32_t *over, uint32_t n_over, cudaStream_t stream);
 
+// Initial state of an inpainting run.  open: a bit per pixel to synthesise, a
+// row's words as in SessionDev::occ; before: such pixels before each word; un (null: not wanted): their list, n_un entries of
+// it; map: the inpainting example.
+struct InpaintDev {
+  const uint32_t *open, *before;
+  uint32_t *un;
+  uint32_t n_un, map;
+};
+void launch_inpaint_init(const SessionDev &s, const InpaintDev &in, cudaStream_t stream);
+
 // Initial state of the pixels set before the first stage (random init):
 // list[6i..6i+6] = {pixel, colour, state.x, state.y, state.z, state.w};
 // res[i] = pixel (the resolved list starts with them, in list order).

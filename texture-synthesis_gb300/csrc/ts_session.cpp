@@ -613,8 +613,9 @@ struct ts_session {
   std::vector<Image> bottoms;                // every example at its loaded size (random init)
   bool inpaint = false;
   uint32_t inpaint_index = 0;
-  Image inpaint_colors;
-  std::vector<uint8_t> inpaint_mask;         // W*H: 1 = to synthesise
+  std::vector<uint32_t> inpaint_open;        // a bit per pixel to synthesise, rows of (W + 31) / 32 words
+  std::vector<uint32_t> inpaint_before;      // such pixels before each word
+  uint32_t inpaint_n = 0;                    // such pixels
   DevBuf<uint32_t> levels, guides, tguide, plevels, pguides;
   bool guide_dims_differ = false;
   DevBuf<uint8_t> masks;
@@ -1079,9 +1080,18 @@ extern "C" int ts_builder_build(ts_builder *b, ts_session **out) {
       } else {
         mask = load_image(b->inpaint.mask, true, W, H, st);
       }
-      s->inpaint_mask.resize((size_t)W * H);
-      for (size_t i = 0; i < (size_t)W * H; ++i) s->inpaint_mask[i] = mask.px[4 * i] < 255 ? 1 : 0;
-      s->inpaint_colors = imgs[s->inpaint_index];
+      const size_t wpr = (W + 31) / 32;
+      s->inpaint_open.resize(wpr * H);
+      s->inpaint_before.resize(wpr * H);
+      for (size_t q = 0; q < wpr * H; ++q) {
+        const size_t y = q / wpr, x0 = (q - y * wpr) * 32, nx = std::min<size_t>(32, W - x0);
+        const uint8_t *px = &mask.px[4 * (y * W + x0)];
+        uint32_t open = 0;
+        for (size_t i = 0; i < nx; ++i) open |= (px[4 * i] < 255 ? 1u : 0u) << i;
+        s->inpaint_open[q] = open;
+        s->inpaint_before[q] = s->inpaint_n;
+        s->inpaint_n += (uint32_t)__builtin_popcount(open);
+      }
     }
     // filtered maps and their device pyramids
     uint64_t texels = 0, ptexels = 0, mask_bytes = 0;
@@ -1332,14 +1342,12 @@ struct RunCtx {
   std::vector<StagePlan> plan;
   std::vector<Step> steps;
   // host data uploaded at the start of the run
-  std::vector<uint32_t> color, resolved, items, occ, mir, cells;
+  std::vector<uint32_t> resolved, items, occ, mir, cells;
   int32_t cox = 0, coy = 0;
   uint32_t cgw = 0, cgh = 0;
-  std::vector<uint4> state;
-  // dense_init: colour and state are uploaded whole (inpainting); otherwise
-  // both start zeroed on the device and init_list holds the few set pixels
-  // as {pixel, colour, state.x, state.y, state.z, state.w}
-  bool dense_init = false;
+  InpaintDev inpaint{};
+  // colour and state start zeroed on the device (inpainting: from the image
+  // and the mask, InpaintDev); init_list holds the pixels that the random init sets
   std::vector<uint32_t> init_list;
   PinnedBuf<uint32_t> pitems;  // the served form's items
   std::vector<float> luts;
@@ -1450,45 +1458,29 @@ void run_plan(ts_session *s, RunCtx &c) {
   c.g.reset(new (std::nothrow) ts_generated());
   if (!c.g) throw Failure{TS_ERR_OUT_OF_MEMORY, "out of host memory"};
   // ---- initial state (Generator::new / new_from_inpaint) ----
-  std::vector<uint32_t> &color = c.color;
-  std::vector<uint4> &state = c.state;
   std::vector<uint32_t> &resolved = c.resolved;
-  c.dense_init = s->inpaint;
   c.init_list.clear();
-  if (c.dense_init) {
-    color.assign(N, 0);
-    state.assign(N, make_uint4(0, 0, 0, 0));
-  }
   auto put = [&](uint32_t px, uint32_t col, uint4 sv) {
-    if (c.dense_init) {
-      color[px] = col;
-      state[px] = sv;
-    } else {
-      c.init_list.insert(c.init_list.end(), {px, col, sv.x, sv.y, sv.z, sv.w});
-    }
+    c.init_list.insert(c.init_list.end(), {px, col, sv.x, sv.y, sv.z, sv.w});
   };
   std::vector<uint32_t> &unresolved = c.unresolved;
   unresolved.clear();
-  size_t locked = 0;
-  if (s->inpaint) {
-    for (size_t i = 0; i < N; ++i) {
-      const uint8_t *cc = &s->inpaint_colors.px[4 * i];
-      color[i] = (uint32_t)cc[0] | ((uint32_t)cc[1] << 8) | ((uint32_t)cc[2] << 16) | ((uint32_t)cc[3] << 24);
-      if (s->inpaint_mask[i]) {
-        unresolved.push_back((uint32_t)i);
-      } else {
-        resolved.push_back((uint32_t)i);
-        state[i] = make_uint4((uint32_t)(i % W) | ((uint32_t)(i / W) << 16), 0, 0, s->inpaint_index);
-      }
-    }
-    locked = resolved.size();
-  }
-  size_t n_un = s->inpaint ? unresolved.size() : N;
   c.dev_picks = c.want_dev_picks;
-  // the list is identity where nothing was picked: on the device it starts
-  // so, and the few entries that the random init's swap-removes change are
-  // kept in a map
-  const bool sparse = c.dev_picks && !s->inpaint;
+  // the colours, states and lists of inpainting are made on the device
+  // (k_inpaint_init); the host needs the pixels to synthesise where it picks
+  if (s->inpaint && (!c.dev_picks || p.has_random_init)) {
+    const size_t wpr = (W + 31) / 32;
+    unresolved.reserve(s->inpaint_n);
+    for (size_t q = 0; q < s->inpaint_open.size(); ++q)
+      for (uint32_t open = s->inpaint_open[q]; open; open &= open - 1)
+        unresolved.push_back((uint32_t)((q / wpr) * W + (q % wpr) * 32) + (uint32_t)__builtin_ctz(open));
+  }
+  size_t locked = s->inpaint ? N - s->inpaint_n : 0;
+  if (!c.dev_picks) resolved.resize(locked);  // run_pick reads the entries after them
+  size_t n_un = N - locked;
+  // on the device the list starts as it was before the random init, and the
+  // few entries that the swap-removes change are kept in a map
+  const bool sparse = c.dev_picks;
   std::unordered_map<uint64_t, uint32_t> moved;
   if (!s->inpaint && !sparse) {
     unresolved.resize(N);
@@ -1500,7 +1492,7 @@ void run_plan(ts_session *s, RunCtx &c) {
     if (sparse) {
       auto at = [&](uint64_t i) {
         const auto it = moved.find(i);
-        return it == moved.end() ? (uint32_t)i : it->second;
+        return it != moved.end() ? it->second : s->inpaint ? unresolved[i] : (uint32_t)i;
       };
       const uint32_t v = at(idx);
       moved[idx] = at(n_un);
@@ -1529,7 +1521,7 @@ void run_plan(ts_session *s, RunCtx &c) {
       const uint8_t *cc = &im.px[((size_t)y * im.w + x) * 4];
       put(px, (uint32_t)cc[0] | ((uint32_t)cc[1] << 8) | ((uint32_t)cc[2] << 16) | ((uint32_t)cc[3] << 24),
           make_uint4(x | (y << 16), px, map, map));
-      resolved.push_back(px);
+      if (!c.dev_picks) resolved.push_back(px);
     }
     locked += p.random_init;
   }
@@ -1551,7 +1543,7 @@ void run_plan(ts_session *s, RunCtx &c) {
   std::vector<StagePlan> &plan = c.plan;
   std::vector<uint32_t> &items = c.items;
   std::vector<float> &luts = c.luts;
-  size_t n_res = resolved.size();
+  size_t n_res = locked;
   size_t n_unresolved = n_un;
   size_t n_items_total = 0;
   int32_t pyramid_level = 0;
@@ -1647,8 +1639,8 @@ void run_plan(ts_session *s, RunCtx &c) {
   // the tree is rebuilt from the resolved list, mirrors included (ms.rs:747-779)
   c.occ.assign((size_t)wpr * H, 0);
   c.mir.assign((size_t)wpr * H, 0);
-  for (size_t i = 0; i < locked; ++i) {
-    const uint32_t q = resolved[i];
+  for (size_t i = 0; i < c.init_list.size(); i += 6) {
+    const uint32_t q = c.init_list[i];
     c.occ[(size_t)(q / W) * wpr + (q % W) / 32] |= 1u << ((q % W) & 31);
     if (p.tiling) c.mir[(size_t)(q / W) * wpr + (q % W) / 32] |= 1u << ((q % W) & 31);
   }
@@ -1660,8 +1652,8 @@ void run_plan(ts_session *s, RunCtx &c) {
   c.cgh = (H + (p.tiling ? 2 * (uint32_t)y_b : 0) + kCell - 1) / kCell;
   c.cells.assign((size_t)c.cgw * c.cgh, 0);
   auto add_cell = [&](int x, int y) { c.cells[(size_t)((y - c.coy) / kCell) * c.cgw + (x - c.cox) / kCell] += 1; };
-  for (size_t i = 0; i < locked; ++i) {
-    const int x = (int)(resolved[i] % W), y = (int)(resolved[i] / W);
+  for (size_t i = 0; i < c.init_list.size(); i += 6) {
+    const int x = (int)(c.init_list[i] % W), y = (int)(c.init_list[i] / W);
     add_cell(x, y);
     if (!p.tiling || !((c.mir[(size_t)y * wpr + x / 32] >> (x & 31)) & 1u)) continue;
     if (x < x_l)
@@ -1690,7 +1682,7 @@ void run_plan(ts_session *s, RunCtx &c) {
                 c.luts.size() * 4 + c.tab.size() * 4 + mb * kk * 12 + mb * (4 + 8 + 4 + sizeof(Result)) +
                 c.n_batches * 4 + (c.rc_ahead ? (uint64_t)c.n_items : std::max<uint64_t>(c.rc_items, mb)) * m * 8 +
                 dist_table_doubles * 8 + steps_est * sizeof(StepDev) +
-                c.cells.size() * 4 + c.init_list.size() * 4;
+                c.cells.size() * 4 + c.init_list.size() * 4 + (s->inpaint ? 2 * (uint64_t)wpr * H * 4 : 0);
 }
 
 // pick_random_unresolved (ms.rs:380-389) for a stage's items: redo item i
@@ -1885,7 +1877,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     }
   }
   const size_t n_chunks = c.knn_chunks.size(), n_kitems = c.knn_ahead ? c.n_items : 0;
-  // zeroed: colour and state first (uploaded instead when dense_init)
+  // zeroed: colour and state first (inpainting writes them whole instead)
   const size_t z_color = zl.add(N * 4), z_state = zl.add(N * sizeof(uint4)), z_rscore = zl.add(c.res_total * 4),
                z_fbc = zl.add(c.n_batches * 4), z_err = zl.add(sizeof(int)), z_evals = zl.add(8),
                z_rank = zl.add(c.knn_ahead ? N * 4 : 0), z_kfbc = zl.add(n_chunks * 4),
@@ -1899,7 +1891,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     return o;
   };
   const size_t t_lut = T(c.luts), t_tab = T(c.tab), t_cells = T(c.cells), t_occ = T(c.occ), t_mir = T(c.mir), t_init = T(c.init_list),
-               t_btab = T(c.btab), t_over = T(c.un_over);
+               t_btab = T(c.btab), t_over = T(c.un_over), t_open = T(s->inpaint_open), t_before = T(s->inpaint_before);
   // scratch
   const size_t w_res = wl.add(c.res_total * 4), w_items = wl.add(c.n_items * 4), w_nbuf = wl.add(mb * kk * 4),
                w_ncnt = wl.add(mb * 4), w_dist = wl.add(c.knn_ahead ? 0 : mb * kk * 8), w_mean = wl.add(mb * 8), w_fbl = wl.add(mb * 4),
@@ -1944,6 +1936,14 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.d_pnext.view(wk + w_pnext, n_un);
   c.d_pdraw.view(wk + w_pdraw, n_un);
   c.d_over.view(tb + t_over, c.un_over.size());
+  c.inpaint = InpaintDev{};
+  if (s->inpaint) {
+    c.inpaint.open = (const uint32_t *)(tb + t_open);
+    c.inpaint.before = (const uint32_t *)(tb + t_before);
+    c.inpaint.un = c.dev_picks ? c.d_un[0].p : nullptr;
+    c.inpaint.n_un = (uint32_t)n_un;
+    c.inpaint.map = s->inpaint_index;
+  }
   c.d_xdiv.view(wk + w_xdiv, c.n_xdiv);
   c.d_ydiv.view(wk + w_ydiv, c.n_ydiv);
   c.d_dxt.view(wk + w_dxt, c.n_xdiv ? (size_t)W * (2 * R + 1) : 0);
@@ -2171,30 +2171,28 @@ void run_stage_tables(RunCtx &c) {
 }
 
 // Uploads of the initial state, enqueued on st: one zero fill, one copy of
-// the tables (colour and state too when dense_init), the random-init
-// pixels.
+// the tables, inpainting's colours, the locked and the random-init pixels.
 void run_upload(RunCtx &c, cudaStream_t st) {
   run_stage_tables(c);
-  if (c.dense_init) {
-    const size_t cs = (size_t)((uint8_t *)c.d_rscore.p - c.d_zero.p);
-    CUDA_TRY(cudaMemcpyAsync(c.d_color.p, c.color.data(), c.N * 4, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(c.d_state.p, c.state.data(), c.N * sizeof(uint4), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemsetAsync(c.d_zero.p + cs, 0, c.zero_bytes - cs, st));
-  } else {
-    CUDA_TRY(cudaMemsetAsync(c.d_zero.p, 0, c.zero_bytes, st));
-  }
+  const size_t cs = c.s->inpaint ? (size_t)((uint8_t *)c.d_rscore.p - c.d_zero.p) : 0;
+  CUDA_TRY(cudaMemsetAsync(c.d_zero.p + cs, 0, c.zero_bytes - cs, st));
   CUDA_TRY(cudaMemcpyAsync(c.d_tabs.p, c.ptab.p, c.tabs_bytes, cudaMemcpyHostToDevice, st));
   if (c.n_xdiv) {
     launch_dist_tables(c.sd, c.d_xdiv.p, c.d_ydiv.p, c.d_dxt.p, c.d_dy2t.p, (uint32_t)c.n_xdiv, (uint32_t)c.n_ydiv, st);
     ++c.launches;
   }
-  if (c.dense_init) {
-    if (c.locked) CUDA_TRY(cudaMemcpyAsync(c.d_res.p, c.resolved.data(), c.locked * 4, cudaMemcpyHostToDevice, st));
-    if (c.dev_picks && c.n_unresolved)  // here, not with the picks: those may be captured into a graph
-      CUDA_TRY(cudaMemcpyAsync(c.d_un[0].p, c.unresolved.data(), c.n_unresolved * 4, cudaMemcpyHostToDevice, st));
-  } else if (!c.init_list.empty()) {
-    // the resolved list starts with the random-init pixels, in list order
-    launch_scatter_init(c.d_init.p, (uint32_t)(c.init_list.size() / 6), c.d_color.p, c.d_state.p, c.d_res.p, st);
+  size_t n_res = 0;
+  if (c.s->inpaint) {
+    CUDA_TRY(cudaMemcpyAsync(c.d_color.p, c.s->bottoms[c.s->inpaint_index].px.data(), c.N * 4, cudaMemcpyHostToDevice,
+                             st));
+    launch_inpaint_init(c.sd, c.inpaint, st);
+    n_res = c.N - c.s->inpaint_n;
+    ++c.launches;
+  }
+  if (!c.init_list.empty()) {
+    // the resolved list goes on with the random-init pixels, in list order
+    launch_scatter_init(c.d_init.p, (uint32_t)(c.init_list.size() / 6), c.d_color.p, c.d_state.p, c.d_res.p + n_res,
+                        st);
     ++c.launches;
   }
 }
@@ -2203,9 +2201,9 @@ void run_upload(RunCtx &c, cudaStream_t st) {
 // a stage at a time, in stage order, on one stream.
 void run_enqueue_picks_init(RunCtx &c, cudaStream_t st) {
   c.pick_len = c.n_unresolved;
-  if (c.n_unresolved == 0) return;
-  if (c.s->inpaint) return;  // run_upload copied it
-  launch_pick_init(c.d_un[0].p, (uint32_t)c.n_unresolved, c.d_over.p, (uint32_t)(c.un_over.size() / 2), st);
+  // (run_upload made inpainting's list)
+  launch_pick_init(c.d_un[0].p, c.s->inpaint ? 0 : (uint32_t)c.n_unresolved, c.d_over.p,
+                   (uint32_t)(c.un_over.size() / 2), st);
   ++c.launches;
 }
 
