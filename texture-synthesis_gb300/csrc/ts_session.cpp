@@ -55,8 +55,11 @@ constexpr uint64_t kRcandBudget = 64ull << 20;  // random-candidate entries held
 // ts_builder_tuning sets it per session).
 constexpr uint32_t kWalkWindowItems = 4096;
 // Runs whose random candidates for every stage fit this many entries make
-// them all ahead, on a side stream, while the first stages run.
-constexpr uint64_t kRcandWhole = 1024ull << 20;
+// them all ahead, on a side stream, while the first stages run.  From
+// kRcandWholeSmall entries (2 GB) on only a run by itself does, and only where
+// the device has four times the room, so that many large runs side by side
+// still fit.
+constexpr uint64_t kRcandWhole = 1024ull << 20, kRcandWholeSmall = 256ull << 20;
 
 struct Image {
   std::vector<uint8_t> px;  // RGBA8
@@ -1369,6 +1372,9 @@ struct RunCtx {
   // each batch start); the resolves wait for their chunk's event.  Plain
   // path, k > 0, exact distance sums.
   bool want_knn_ahead = false, knn_ahead = false;
+  // multi: the steps go out as multi-session launches (batch, server), which
+  // commit in launches of their own and take one item per warp
+  bool multi = false;
   std::vector<KnnChunk> knn_chunks;
   std::vector<EventHandle> knn_ev;  // per chunk: its k-NN is done
   std::vector<uint2> btab;          // every batch: {first stage item, tree length at its start}
@@ -1444,6 +1450,24 @@ bool knn_ahead_fits(const RunCtx &c, uint32_t W, uint32_t H, uint32_t k) {
   constexpr uint64_t kKnnAheadMinPixels = 2048;
   return c.want_knn_ahead && k > 0 && (exact_sum_ok(W, H, k) || (uint64_t)W * H >= kKnnAheadMinPixels) &&
          (uint64_t)c.n_items * ((uint64_t)k * 4 + 16) <= kKnnAheadMaxBytes;
+}
+
+// Bytes the k-NN ahead adds to a run's buffers (run_alloc).
+uint64_t knn_ahead_bytes(const RunCtx &c) {
+  return (uint64_t)c.n_items * ((uint64_t)c.k * 4 + 16) + (uint64_t)c.N * 4;
+}
+
+// Device memory that the stream-ordered pool can still hand out.
+uint64_t device_room(int dev) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+  cudaMemPool_t pool;
+  uint64_t reserved = 0, used = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+    free_b += reserved - used;
+  return free_b;
 }
 
 // Host schedule of Generator::resolve (ms.rs:702-1051) and the device
@@ -1633,7 +1657,10 @@ void run_plan(ts_session *s, RunCtx &c) {
   for (auto &sp : plan) c.n_batches += sp.batches.size();
   c.max_batch_items = max_batch_items;
   c.rc_items = std::max<uint64_t>(1, std::min<uint64_t>(max_stage_items, kRcandBudget / std::max(m, 1u)));
-  c.rc_ahead = c.want_rc_ahead && m > 0 && (uint64_t)n_items_total * m <= kRcandWhole;
+  const uint64_t rc_all = (uint64_t)n_items_total * m;
+  c.rc_ahead = c.want_rc_ahead && m > 0 &&
+               (rc_all <= kRcandWholeSmall ||
+                (!c.multi && rc_all <= kRcandWhole && device_room(s->prm.device) >= 4 * rc_all * 8));
   c.x_l = x_l;
   c.y_b = y_b;
   // the tree is rebuilt from the resolved list, mirrors included (ms.rs:747-779)
@@ -1877,11 +1904,14 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     }
   }
   const size_t n_chunks = c.knn_chunks.size(), n_kitems = c.knn_ahead ? c.n_items : 0;
+  const size_t n_wctr = c.multi ? 0 : c.n_batches * kWorkCtrs * kWorkCtrStride;
+  const size_t n_result = (c.knn_ahead && !c.multi ? 2 : 1) * mb;
   // zeroed: colour and state first (inpainting writes them whole instead)
   const size_t z_color = zl.add(N * 4), z_state = zl.add(N * sizeof(uint4)), z_rscore = zl.add(c.res_total * 4),
                z_fbc = zl.add(c.n_batches * 4), z_err = zl.add(sizeof(int)), z_evals = zl.add(8),
                z_rank = zl.add(c.knn_ahead ? N * 4 : 0), z_kfbc = zl.add(n_chunks * 4),
-               z_shadow = zl.add(c.knn_ahead ? 2 * N * sizeof(uint4) : 0), z_wctr = zl.add(c.n_batches * kWorkCtrs * kWorkCtrStride * 4);
+               z_shadow = zl.add(c.knn_ahead && !c.multi ? 2 * N * sizeof(uint4) : 0),
+               z_wctr = zl.add(n_wctr * 4);
   // uploaded tables
   c.tab_parts.clear();
   auto T = [&](const auto &v) {
@@ -1895,7 +1925,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   // scratch
   const size_t w_res = wl.add(c.res_total * 4), w_items = wl.add(c.n_items * 4), w_nbuf = wl.add(mb * kk * 4),
                w_ncnt = wl.add(mb * 4), w_dist = wl.add(c.knn_ahead ? 0 : mb * kk * 8), w_mean = wl.add(mb * 8), w_fbl = wl.add(mb * 4),
-               w_result = wl.add((c.knn_ahead ? 2 : 1) * mb * sizeof(Result)), w_rcand = wl.add(rc_n * 8),
+               w_result = wl.add(n_result * sizeof(Result)), w_rcand = wl.add(rc_n * 8),
                w_knbuf = wl.add(n_kitems * kk * 4), w_kncnt = wl.add(n_kitems * 4), w_kmean = wl.add(n_kitems * 8),
                w_kfbl = wl.add(n_kitems * 4), w_xdiv = wl.add(c.n_xdiv * 8), w_ydiv = wl.add(c.n_ydiv * 8),
                w_dxt = wl.add(c.n_xdiv ? (size_t)W * (2 * R + 1) * 8 : 0),
@@ -1923,8 +1953,8 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.d_init.view(tb + t_init, c.init_list.size());
   c.d_btab.view(tb + t_btab, c.btab.size());
   c.d_rank.view(z + z_rank, c.knn_ahead ? N : 0);
-  c.d_shadow.view(z + z_shadow, c.knn_ahead ? 2 * N : 0);
-  c.d_wctr.view(z + z_wctr, c.n_batches * kWorkCtrs * kWorkCtrStride);
+  c.d_shadow.view(z + z_shadow, c.knn_ahead && !c.multi ? 2 * N : 0);
+  c.d_wctr.view(z + z_wctr, n_wctr);
   c.d_kfbc.view(z + z_kfbc, n_chunks);
   c.d_knbuf.view(wk + w_knbuf, n_kitems * kk);
   c.d_kncnt.view(wk + w_kncnt, n_kitems);
@@ -1955,7 +1985,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.d_dist.view(wk + w_dist, c.knn_ahead ? 0 : mb * kk);
   c.d_mean.view(wk + w_mean, mb);
   c.d_fbl.view(wk + w_fbl, mb);
-  c.d_result.view(wk + w_result, (c.knn_ahead ? 2 : 1) * mb);
+  c.d_result.view(wk + w_result, n_result);
   c.d_rcand.view(wk + w_rcand, rc_n);
   const std::vector<int32_t> &tab = c.tab;
 
@@ -2087,7 +2117,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
         bd.res = c.d_result.p;
         stp.n = bp.i1 - bp.i0;
         stp.stage_i0 = bp.i0;
-        if (c.want_knn_ahead) bd.work_ctr = c.d_wctr.p + (size_t)bidx * kWorkCtrs * kWorkCtrStride;  // plain runs (ts_session_run) only
+        if (!c.multi) bd.work_ctr = c.d_wctr.p + (size_t)bidx * kWorkCtrs * kWorkCtrStride;
         stp.bidx = bidx++;
         if (c.knn_ahead) {  // the chunk's lists, made ahead on the k-NN stream
           const size_t g0 = (size_t)sp.items_off + bp.i0;
@@ -2246,52 +2276,54 @@ bool can_defer_commit(const RunCtx &c, const Step &stp, const Step *next) {
   return !(next->exhaustive && next->resolve == kPhaseTeamFull && team_full_fits(c.sd.k, c.sd.m));
 }
 
-// k-NN ahead: the chunks of stage `stage` on the k-NN stream kst, once its
-// items are up: each chunk's tree entries, then its neighbour lists and
-// means (inexact ones on the stream mst), then its event.
-void run_enqueue_knn(RunCtx &c, cudaStream_t kst, cudaStream_t mst, LaunchTimer &lt, int stage) {
+// k-NN ahead: chunk q on the k-NN stream kst, once its stage's items are up:
+// its tree entries, then its neighbour lists and means (inexact ones on the
+// stream mst), then its event.
+void run_enqueue_chunk(RunCtx &c, size_t q, cudaStream_t kst, cudaStream_t mst, LaunchTimer &lt) {
   const SessionDev &sd = c.sd;
-  const cudaStream_t main_st = lt.st;
+  const KnnChunk &ch = c.knn_chunks[q];
   lt.st = kst;
-  for (size_t q = 0; q < c.knn_chunks.size(); ++q) {
-    const KnnChunk &ch = c.knn_chunks[q];
-    if (ch.stage != stage) continue;
-    lt.items = ch.b.i1 - ch.b.i0;
-    if (ch.a1 > ch.a0) {
-      lt.run(TS_KERNEL_COMMIT, [&] { launch_tree_append(sd, ch.st, ch.a0, ch.a1, ch.pos0, ch.nomir_end, kst); });
-      ++c.launches;
-    }
-    const bool list = ch.all_exhaustive && knn_list_fits(sd, ch.b);
-    if (ch.all_exhaustive && !list) {
-      lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, true, kst, PendingCommit{}); });
-      ++c.launches;
-    } else {
-      lt.run(TS_KERNEL_KNN_WALK, [&] {
-        if (list)
-          launch_knn_list(sd, ch.st, ch.b, kst);
-        else
-          launch_knn_walk(sd, ch.st, ch.b, kst, PendingCommit{});
-      });
-      lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, false, kst, PendingCommit{}); });
-      c.launches += 2;
-    }
-    CUDA_TRY(cudaEventCreateWithFlags(&c.knn_ev[q].e, cudaEventDisableTiming));
-    if (!sd.exact_sum) {
+  lt.items = ch.b.i1 - ch.b.i0;
+  if (ch.a1 > ch.a0) {
+    lt.run(TS_KERNEL_COMMIT, [&] { launch_tree_append(sd, ch.st, ch.a0, ch.a1, ch.pos0, ch.nomir_end, kst); });
+    ++c.launches;
+  }
+  const bool list = ch.all_exhaustive && knn_list_fits(sd, ch.b);
+  if (ch.all_exhaustive && !list) {
+    lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, true, kst, PendingCommit{}); });
+    ++c.launches;
+  } else {
+    lt.run(TS_KERNEL_KNN_WALK, [&] {
+      if (list)
+        launch_knn_list(sd, ch.st, ch.b, kst);
+      else
+        launch_knn_walk(sd, ch.st, ch.b, kst, PendingCommit{});
+    });
+    lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, ch.st, ch.b, false, kst, PendingCommit{}); });
+    c.launches += 2;
+  }
+  CUDA_TRY(cudaEventCreateWithFlags(&c.knn_ev[q].e, cudaEventDisableTiming));
+  if (!sd.exact_sum) {
+    if (mst != kst) {
       // on a stream of their own: the f64 chains (6.6 us at least) overlap
       // the next chunk's lists
       EventHandle lists;
       CUDA_TRY(cudaEventCreateWithFlags(&lists.e, cudaEventDisableTiming));
       CUDA_TRY(cudaEventRecord(lists.e, kst));
       CUDA_TRY(cudaStreamWaitEvent(mst, lists.e, 0));
-      lt.st = mst;
-      lt.run(TS_KERNEL_MEAN, [&] { launch_mean_ahead(sd, ch.st, ch.b, mst); });
-      lt.st = kst;
-      ++c.launches;
-      CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, mst));
-    } else {
-      CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, kst));
     }
+    lt.st = mst;
+    lt.run(TS_KERNEL_MEAN, [&] { launch_mean_ahead(sd, ch.st, ch.b, mst); });
+    ++c.launches;
   }
+  CUDA_TRY(cudaEventRecord(c.knn_ev[q].e, sd.exact_sum ? kst : mst));
+}
+
+// The chunks of stage `stage`.
+void run_enqueue_knn(RunCtx &c, cudaStream_t kst, cudaStream_t mst, LaunchTimer &lt, int stage) {
+  const cudaStream_t main_st = lt.st;
+  for (size_t q = 0; q < c.knn_chunks.size(); ++q)
+    if (c.knn_chunks[q].stage == stage) run_enqueue_chunk(c, q, kst, mst, lt);
   lt.st = main_st;
 }
 
@@ -2585,8 +2617,10 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
       // the initial tree's positions; the k-NN stream starts after them
       launch_rank_init(c.sd, (uint32_t)c.locked, st);
       if (c.locked) ++c.launches;
-      CUDA_TRY(side_stream(s->prm.device, prio_low, &kg.s));
-      if (!c.sd.exact_sum) CUDA_TRY(side_stream(s->prm.device, prio_low, &mg.s));
+      // before the random candidates, whose blocks would fill the GPU ahead of
+      // the first lists (2048^2: 39.6 ms, so 38.4)
+      CUDA_TRY(side_stream(s->prm.device, prio_low - 1, &kg.s));
+      if (!c.sd.exact_sum) CUDA_TRY(side_stream(s->prm.device, prio_low - 1, &mg.s));
       EventHandle ready;
       CUDA_TRY(cudaEventCreateWithFlags(&ready.e, cudaEventDisableTiming));
       CUDA_TRY(cudaEventRecord(ready.e, st));
@@ -2741,7 +2775,7 @@ namespace {
 
 // Units a session's step hands to a phase (0 = no segment).
 uint32_t phase_units(const Step &stp, const RunCtx &c, int phase) {
-  const bool knn = stp.batch && c.k > 0;
+  const bool knn = stp.batch && c.k > 0 && !c.knn_ahead;
   switch (phase) {
     case kPhaseLevelSwitch: return stp.ls ? stp.ls_n_res : 0;
     case kPhaseRandom: return (stp.rc && c.m > 0 && !c.rc_ahead) ? stp.rc_st.n_items : 0;
@@ -2776,8 +2810,19 @@ struct PlannedLaunch {
   uint32_t n_lean = 0, lean_blocks = 0;  // resolve: leading segments of sessions without guides
   uint32_t key_cap = 0;                  // exhaustive: keys in shared memory (largest over the steps)
   int wait_rc = -1;  // first wait for the side stream's random candidates up to this launch of them
-  int wait_items = -1;  // first wait for the side stream's item uploads up to this part
+  int wait_items = -1;  // first wait for the side stream's picks up to this part
+  int first_of = -1;    // the batch step whose first launch this is
 };
+
+// The batch's k-NN ahead: the sessions' chunks go to kBatchKnnStreams streams,
+// in the order of the steps that need them and kBatchAheadSteps steps early (a
+// chunk of the first stage covers some six).  Each session's own launches
+// take the steps' walk, fallback and mean out of the chain: 24 sessions,
+// 10.8 M items: 80.5 -> 64 ms a run, with 4 streams 65, with 10 or 60 steps
+// the same within 1%.  Their buffers take at most kBatchAheadMaxBytes.
+constexpr size_t kBatchKnnStreams = 8, kBatchAheadSteps = 24;
+constexpr uint64_t kBatchAheadMaxBytes = 48ull << 30;
+constexpr uint64_t kBatchPoolKeep = 16ull << 30;
 
 // Blocks of the exhaustive k-NN's fallback pool (three 64 KB CTAs per SM).
 constexpr uint32_t kFallbackPool = 152u * 3u;
@@ -2868,17 +2913,29 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       for (ts_session *s : v) delete s;
     }
   } owned{sessions};
-  // main stream, side stream (item uploads, random candidates made ahead)
+  // what the batch's buffers leave in the device's pool above kBatchPoolKeep
+  // goes back to the device
+  struct Trim {
+    int dev;
+    ~Trim() {
+      cudaMemPool_t pool;
+      if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) cudaMemPoolTrimTo(pool, kBatchPoolKeep);
+    }
+  } trim{b->device};
+  // main stream, side stream (picks, random candidates made ahead)
   // and copy stream (read-backs); outside the try so that a failure can
   // drain them before the sessions' buffers go
   StreamGuard sg, rg, cg;
+  std::vector<StreamGuard> ks(kBatchKnnStreams);
   std::vector<std::unique_ptr<RunCtx>> ctx(n);
   size_t current = 0;
   try {
     CUDA_TRY(cudaSetDevice(b->device));
-    // the step chain on the highest priority, the side stream's work on the
-    // lowest and (unless the launches are captured into a graph) on the
-    // green context that leaves SMs to the chain (side_stream)
+    // the step chain on the highest priority, the random candidates on the
+    // lowest and (unless the launches are captured into a graph) on the green
+    // context that leaves SMs to the chain (side_stream), the neighbour lists
+    // made ahead between the two: behind the candidates the first steps of 24
+    // sessions waited 3.5 ms for theirs
     int prio_low = 0, prio_high = 0;
     CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
     CUDA_TRY(cudaStreamCreateWithPriority(&sg.s, cudaStreamNonBlocking, prio_high));
@@ -2889,32 +2946,71 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       // sessions plan independently: host threads take them in turn
       unsigned nt = b->plan_threads ? b->plan_threads : std::min(32u, std::max(1u, std::thread::hardware_concurrency()));
       nt = (unsigned)std::min<size_t>(nt, n);
-      std::atomic<size_t> next{0};
+      std::atomic<size_t> next{0}, next_alloc{0};
       std::vector<Failure> fails(n, Failure{TS_OK, ""});
+      auto guarded = [&](size_t j, auto &&f) {
+        try {
+          f();
+        } catch (const Failure &e) {
+          fails[j] = e;
+        } catch (const std::bad_alloc &) {
+          fails[j] = Failure{TS_ERR_OUT_OF_MEMORY, "out of host memory"};
+        }
+      };
+      // Which sessions make their k-NN ahead: in order, while the lists fit
+      // kBatchAheadMaxBytes and half of what the sessions' other buffers
+      // leave free.  Captured launches keep their steps' own k-NN.
+      auto choose_ahead = [&] {
+        uint64_t base = 0;
+        for (size_t j = 0; j < n; ++j)
+          if (ctx[j]) base += ctx[j]->dev_bytes;
+        const uint64_t room = device_room(b->device);
+        uint64_t left = std::min<uint64_t>(kBatchAheadMaxBytes, room > base ? (room - base) / 2 : 0);
+        for (size_t j = 0; j < n; ++j) {
+          if (!ctx[j] || b->graph) continue;
+          const uint64_t need = knn_ahead_bytes(*ctx[j]);
+          if (need > left) continue;
+          ctx[j]->want_knn_ahead = true;
+          left -= need;
+        }
+      };
+      std::mutex mu;
+      std::condition_variable cv;
+      unsigned planned = 0;
       auto work = [&] {
-        if (cudaSetDevice(b->device) != cudaSuccess) return;
-        for (size_t j = next++; j < n; j = next++) {
-          try {
-            ctx[j].reset(new RunCtx());
-            ctx[j]->want_rc_ahead = true;
-            ctx[j]->want_dev_picks = true;
-            run_plan(sessions[j], *ctx[j]);
-            run_alloc(*ctx[j], nullptr);
-            RunCtx &c = *ctx[j];
-            run_stage_tables(c);
-            // touch the read-back destinations here, in parallel, rather
-            // than in the copies at the end of the run
-            c.col.resize(c.N);
-            c.stv.resize(c.N);
-            c.g->resolved.resize(c.res_total);
-            c.g->scores.resize(c.res_total);
-
-          } catch (const Failure &f) {
-            fails[j] = f;
-          } catch (const std::bad_alloc &) {
-            fails[j] = Failure{TS_ERR_OUT_OF_MEMORY, "out of host memory"};
+        const bool ok = cudaSetDevice(b->device) == cudaSuccess;
+        for (size_t j = next++; j < n; j = next++)
+          guarded(j, [&] {
+            if (!ok) throw Failure{TS_ERR_CUDA, "cannot select the device"};
+            std::unique_ptr<RunCtx> c(new RunCtx());
+            c->multi = true;
+            c->want_rc_ahead = true;
+            c->want_dev_picks = true;
+            run_plan(sessions[j], *c);
+            ctx[j] = std::move(c);
+          });
+        {
+          std::unique_lock<std::mutex> lk(mu);
+          if (++planned == nt) {
+            choose_ahead();
+            cv.notify_all();
+          } else {
+            cv.wait(lk, [&] { return planned == nt; });
           }
         }
+        for (size_t j = next_alloc++; j < n; j = next_alloc++)
+          if (ctx[j])
+            guarded(j, [&] {
+              RunCtx &c = *ctx[j];
+              run_alloc(c, st);
+              run_stage_tables(c);
+              // touch the read-back destinations here, in parallel, rather
+              // than in the copies at the end of the run
+              c.col.resize(c.N);
+              c.stv.resize(c.N);
+              c.g->resolved.resize(c.res_total);
+              c.g->scores.resize(c.res_total);
+            });
       };
       std::vector<std::thread> pool;
       for (unsigned i = 1; i < nt; ++i) pool.emplace_back(work);
@@ -2922,7 +3018,6 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       for (auto &t : pool) t.join();
       for (current = 0; current < n; ++current) {
         if (fails[current].status != TS_OK) throw fails[current];
-        if (!ctx[current]) throw Failure{TS_ERR_CUDA, "cannot select the device"};
         max_steps = std::max(max_steps, ctx[current]->steps.size());
       }
     }
@@ -2994,6 +3089,16 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
         rc_launches.push_back(pl);
       }
     }
+    // the chunks of neighbour lists made ahead, by the step that needs them
+    struct AheadChunk {
+      size_t step, session, chunk;
+    };
+    std::vector<AheadChunk> ahead;
+    for (size_t j : heavy)
+      for (size_t t = 0; t < ctx[j]->steps.size(); ++t)
+        if (ctx[j]->steps[t].knn_wait >= 0) ahead.push_back({t, j, (size_t)ctx[j]->steps[t].knn_wait});
+    std::stable_sort(ahead.begin(), ahead.end(), [](const AheadChunk &x, const AheadChunk &y) { return x.step < y.step; });
+    for (size_t j = 0; j < n; ++j) ctx[j]->knn_ev.resize(ctx[j]->knn_chunks.size());
     int rc_waited = -1, items_waited = -1;
     for (size_t t = 0; t < max_steps; ++t) {
       // a session starting stage q at this step needs rc launch q done
@@ -3032,7 +3137,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
             if (t >= c.steps.size()) continue;
             if (ph == kPhaseResolve && sessions[j]->guided != (pass == 1)) continue;
             const Step &stp = c.steps[t];
-            if (ph == kPhaseExhaustive && stp.batch && c.k > 0 && !stp.exhaustive) {
+            if (ph == kPhaseExhaustive && stp.batch && c.k > 0 && !c.knn_ahead && !stp.exhaustive) {
               h_fb.push_back(Segment{0, 0, (uint32_t)j, (uint32_t)t});
               pl.n_fb += 1;
               pl.key_cap = std::max(pl.key_cap, exh_key_cap(c.sd, stp.bd));
@@ -3063,6 +3168,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
           for (uint32_t q = pl.fb0; q < pl.fb0 + pl.n_fb; ++q) last_launch[h_fb[q].session] = launches.size() - 1;
         }
       }
+      if (launches.size() > launches_before) launches[launches_before].first_of = (int)t;
       if (rc_need > rc_waited && launches.size() > launches_before) {
         launches[launches_before].wait_rc = rc_need;
         rc_waited = rc_need;
@@ -3071,7 +3177,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       // gets past stage 0
       int items_need = t == 0 ? 0 : -1;
       for (size_t j = 0; j < n; ++j)
-        if (t < ctx[j]->steps.size() && ctx[j]->steps[t].stage >= 1) items_need = 1;
+        if (!ctx[j]->knn_ahead && t < ctx[j]->steps.size() && ctx[j]->steps[t].stage >= 1) items_need = 1;
       if (items_need > items_waited && launches.size() > launches_before) {
         launches[launches_before].wait_items = items_need;
         items_waited = items_need;
@@ -3082,18 +3188,20 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     DevBuf<StepDev> d_steps;
     DevBuf<Segment> d_segs, d_fb;
     DevBuf<const StepDev *> d_tabs;
-    CUDA_TRY(d_tabs.alloc(n));
-    CUDA_TRY(d_sess.alloc(n));
-    CUDA_TRY(d_steps.alloc(n_steps));
-    CUDA_TRY(d_segs.alloc(h_segs.size()));
-    CUDA_TRY(d_fb.alloc(h_fb.size()));
+    CUDA_TRY(d_tabs.alloc_on(n, st));
+    CUDA_TRY(d_sess.alloc_on(n, st));
+    CUDA_TRY(d_steps.alloc_on(n_steps, st));
+    CUDA_TRY(d_segs.alloc_on(h_segs.size(), st));
+    CUDA_TRY(d_fb.alloc_on(h_fb.size(), st));
     EventPair ev, ev_io;
     ev.create();
     ev_io.create();
     CUDA_TRY(cudaEventRecord(ev.a, st));
     for (current = 0; current < n; ++current) {
       if (sessions[current]->ready.e) CUDA_TRY(cudaStreamWaitEvent(st, sessions[current]->ready.e, 0));
-      run_upload(*ctx[current], st);
+      RunCtx &c = *ctx[current];
+      run_upload(c, st);
+      if (c.knn_ahead) launch_rank_init(c.sd, (uint32_t)c.locked, st);
     }
     CUDA_TRY(cudaMemcpyAsync(d_sess.p, h_sess.data(), n * sizeof(SessionDev), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(d_steps.p, h_steps.data(), n_steps * sizeof(StepDev), cudaMemcpyHostToDevice, st));
@@ -3135,20 +3243,32 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     else
       CUDA_TRY(side_stream(b->device, prio_low, &rg.s));
     for (auto &e : rc_ev) CUDA_TRY(cudaEventCreateWithFlags(&e.e, cudaEventDisableTiming));
+    if (!ahead.empty())
+      for (auto &g : ks) CUDA_TRY(cudaStreamCreateWithPriority(&g.s, cudaStreamNonBlocking, prio_low - 1));
     EventHandle fork, side_done, items_ev[2];
     CUDA_TRY(cudaEventCreateWithFlags(&fork.e, cudaEventDisableTiming));
     CUDA_TRY(cudaEventCreateWithFlags(&side_done.e, cudaEventDisableTiming));
     for (auto &e : items_ev) CUDA_TRY(cudaEventCreateWithFlags(&e.e, cudaEventDisableTiming));
     // the picks of stage 0 (part 0) and of the later stages (part 1), every
-    // session's
+    // session's without k-NN ahead
     auto pick_items = [&](int part) {
       for (size_t j = 0; j < n; ++j) {
         RunCtx &c = *ctx[j];
+        if (c.knn_ahead) continue;
         if (part == 0) run_enqueue_picks_init(c, rg.s);
         for (size_t q = part == 0 ? 0 : 1; q < (part == 0 ? std::min<size_t>(1, c.plan.size()) : c.plan.size()); ++q)
           run_enqueue_picks(c, rg.s);
       }
       CUDA_TRY(cudaEventRecord(items_ev[part].e, rg.s));
+    };
+    // chunk `a` on its session's k-NN stream, after the picks of its stage
+    LaunchTimer lt;
+    auto launch_chunk = [&](const AheadChunk &a) {
+      RunCtx &c = *ctx[a.session];
+      const cudaStream_t kst = ks[a.session % kBatchKnnStreams].s;
+      if (c.picked_stages == 0) run_enqueue_picks_init(c, kst);
+      while ((int)c.picked_stages <= c.knn_chunks[a.chunk].stage) run_enqueue_picks(c, kst);
+      run_enqueue_chunk(c, a.chunk, kst, kst, lt);
     };
     auto launch_rc = [&](size_t i) {
       const PlannedLaunch &pl = rc_launches[i];
@@ -3169,14 +3289,25 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       // first steps run
       CUDA_TRY(cudaEventRecord(fork.e, s));
       CUDA_TRY(cudaStreamWaitEvent(rg.s, fork.e, 0));
+      for (auto &g : ks)
+        if (g.s) CUDA_TRY(cudaStreamWaitEvent(g.s, fork.e, 0));
       pick_items(0);
       size_t rci = 0;
       if (!rc_launches.empty() && rc_pos[0] == 0) launch_rc(rci++);
       pick_items(1);
       for (; rci < rc_launches.size(); ++rci) launch_rc(rci);
       CUDA_TRY(cudaEventRecord(side_done.e, rg.s));
+      size_t made = 0, waited = 0;  // chunks
       for (size_t li = 0; li < launches.size(); ++li) {
         const PlannedLaunch &pl = launches[li];
+        if (pl.first_of >= 0) {
+          // the chunks of the next steps go out before this one's launches, so
+          // that their lists are made while it runs
+          for (; made < ahead.size() && ahead[made].step <= (size_t)pl.first_of + kBatchAheadSteps; ++made)
+            launch_chunk(ahead[made]);
+          for (; waited < made && ahead[waited].step <= (size_t)pl.first_of; ++waited)
+            CUDA_TRY(cudaStreamWaitEvent(s, ctx[ahead[waited].session]->knn_ev[ahead[waited].chunk].e, 0));
+        }
         if (pl.wait_items >= 0) CUDA_TRY(cudaStreamWaitEvent(s, items_ev[pl.wait_items].e, 0));
         if (pl.wait_rc >= 0) CUDA_TRY(cudaStreamWaitEvent(s, rc_ev[pl.wait_rc].e, 0));
         MultiLaunch ml;
@@ -3237,6 +3368,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     bs.sessions = n;
     bs.steps = max_steps;
     bs.launches = launches.size() + rc_launches.size();
+    for (size_t j = 0; j < n; ++j) bs.launches += ctx[j]->launches;
     for (const PlannedLaunch &pl : launches)
       if (pl.phase == kPhaseResolve && pl.n_lean && pl.n_lean < pl.n_segs) bs.launches += 1;  // two kernels
     bs.phase_launches[kPhaseRandom] += rc_launches.size();
@@ -3262,6 +3394,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       run_finish(c);
       c.g->stats.gpu_ms = gpu_ms;
       c.g->stats.kernel_launches = launches.size();
+      c.g->stats.knn_chunks = c.knn_chunks.size();
       bs.output_pixels += c.N;
       bs.resolves += c.resolves;
       bs.cost_evals += c.evals;
@@ -3273,6 +3406,8 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     // nothing may be in flight when the sessions' buffers go
     for (cudaStream_t q : {sg.s, rg.s, cg.s})
       if (q) cudaStreamSynchronize(q);
+    for (auto &g : ks)
+      if (g.s) cudaStreamSynchronize(g.s);
     b->err = "session " + std::to_string(current < n ? current : 0) + ": " + f.msg;
     return f.status;
   }
@@ -3600,7 +3735,7 @@ void server_driver(ts_server *S) {
               const RunCtx &c = *r->c;
               if (ph == kPhaseResolve && r->s->guided != (pass == 1)) continue;
               const Step &stp = c.steps[r->cursor];
-              if (ph == kPhaseExhaustive && stp.batch && c.k > 0 && !stp.exhaustive) {
+              if (ph == kPhaseExhaustive && stp.batch && c.k > 0 && !c.knn_ahead && !stp.exhaustive) {
                 fb.push_back(Segment{0, 0, r->slot, (uint32_t)r->cursor});
                 pl.n_fb += 1;
                 pl.key_cap = std::max(pl.key_cap, exh_key_cap(c.sd, stp.bd));
