@@ -40,3 +40,16 @@ def test_batched(ts, oracle, wl, graph):
         batch.add(ts.builder_from_spec(s).build())
     for g, s in zip(batch.run(), specs):
         assert_same(ts.generated_outputs(g), oracle.run(s, nthreads=8), s["name"])
+
+
+@pytest.mark.parametrize("kind", ["plain", "inpaint", "served"])
+def test_many_random_init(ts, oracle, wl, kind):
+    """More random-init pixels than a 64th: the unresolved list is kept whole."""
+    spec = wl.inpaint_session(19, side=96) if kind == "inpaint" else wl.config0(out=90, ex=24)
+    spec = small(spec, random_init=700)
+    if kind == "served":
+        server = ts.Server()
+        got = ts.generated_outputs(server.wait(server.submit(ts.builder_from_spec(spec).build()))[0])
+    else:
+        got = ts.run_spec(spec)
+    assert_same(got, oracle.run(spec, nthreads=8), kind)

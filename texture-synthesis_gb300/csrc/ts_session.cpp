@@ -1345,14 +1345,13 @@ struct RunCtx {
   std::vector<StagePlan> plan;
   std::vector<Step> steps;
   // host data uploaded at the start of the run
-  std::vector<uint32_t> resolved, items, occ, mir, cells;
+  std::vector<uint32_t> occ, mir, cells;
   int32_t cox = 0, coy = 0;
   uint32_t cgw = 0, cgh = 0;
   InpaintDev inpaint{};
   // colour and state start zeroed on the device (inpainting: from the image
   // and the mask, InpaintDev); init_list holds the pixels that the random init sets
   std::vector<uint32_t> init_list;
-  PinnedBuf<uint32_t> pitems;  // the served form's items
   std::vector<float> luts;
   std::vector<int32_t> tab;
   size_t n_xdiv = 0, n_ydiv = 0;  // entries of the coordinate tables (0: exact sums need none)
@@ -1386,16 +1385,14 @@ struct RunCtx {
   BatchDev pend_bd{};
   uint32_t pend_n = 0, defer_parity = 0;
   size_t res_total = 0;                // resolved-list length at the end of the run
-  std::vector<uint32_t> unresolved;    // pixels not yet picked (the pick chain's state)
-  // dev_picks: the pick chain runs on the device (run_enqueue_picks).  The
-  // unresolved list starts as `unresolved` (inpainting) or as 0, 1, .. with
-  // the entries un_over {position, pixel} that the random init's picks left
-  bool want_dev_picks = false, dev_picks = false;
+  // The pick chain runs on the device (run_enqueue_picks).  Its unresolved
+  // list starts as inpainting's pixels to synthesise or as 0, 1, .. with the
+  // entries un_over {position, pixel} that the random init's picks left
   size_t n_unresolved = 0, n_items = 0;
   size_t pick_len = 0;       // entries of the device's unresolved list after the stages enqueued so far
   uint32_t pick_parity = 0;  // which of d_un holds it
   std::vector<uint32_t> un_over;
-  size_t picked_stages = 0;            // stages whose items are known
+  size_t picked_stages = 0;  // stages whose picks are enqueued
   int32_t x_l = 0, y_b = 0;
   uint64_t dev_bytes = 0;  // device memory run_alloc takes
   // device state
@@ -1412,7 +1409,7 @@ struct RunCtx {
   PinnedBuf<uint8_t> ptab;
   DevBuf<uint32_t> d_color, d_occ, d_mir, d_res, d_items, d_ncnt, d_fbl, d_fbc, d_cells, d_init;
   DevBuf<uint32_t> d_rank, d_kncnt, d_kfbl, d_kfbc;  // knn_ahead
-  DevBuf<uint32_t> d_un[2], d_phead, d_pnext, d_pdraw, d_over;  // dev_picks
+  DevBuf<uint32_t> d_un[2], d_phead, d_pnext, d_pdraw, d_over;  // the picks
   DevBuf<uint32_t> d_wctr;  // per batch: the warp resolve's item counters (BatchDev::work_ctr)
   DevBuf<int32_t> d_knbuf;
   DevBuf<double> d_kmean;
@@ -1482,49 +1479,48 @@ void run_plan(ts_session *s, RunCtx &c) {
   c.g.reset(new (std::nothrow) ts_generated());
   if (!c.g) throw Failure{TS_ERR_OUT_OF_MEMORY, "out of host memory"};
   // ---- initial state (Generator::new / new_from_inpaint) ----
-  std::vector<uint32_t> &resolved = c.resolved;
   c.init_list.clear();
   auto put = [&](uint32_t px, uint32_t col, uint4 sv) {
     c.init_list.insert(c.init_list.end(), {px, col, sv.x, sv.y, sv.z, sv.w});
   };
-  std::vector<uint32_t> &unresolved = c.unresolved;
-  unresolved.clear();
-  c.dev_picks = c.want_dev_picks;
-  // the colours, states and lists of inpainting are made on the device
-  // (k_inpaint_init); the host needs the pixels to synthesise where it picks
-  if (s->inpaint && (!c.dev_picks || p.has_random_init)) {
+  // The colours, states and lists of inpainting are made on the device
+  // (k_inpaint_init), and so is the unresolved list, as it is before the
+  // random init; the entries that its swap-removes change go along.  A few
+  // are kept in a map, many in the list itself (65536 picks of 1024^2: 13.4
+  // ms of planning with the map, under 6 with the list).
+  size_t locked = s->inpaint ? N - s->inpaint_n : 0;
+  size_t n_un = N - locked;
+  const bool dense = p.has_random_init && p.random_init > N / 64;
+  std::vector<uint32_t> unresolved;  // the list, where the host needs it whole
+  if (s->inpaint && p.has_random_init) {
     const size_t wpr = (W + 31) / 32;
     unresolved.reserve(s->inpaint_n);
     for (size_t q = 0; q < s->inpaint_open.size(); ++q)
       for (uint32_t open = s->inpaint_open[q]; open; open &= open - 1)
         unresolved.push_back((uint32_t)((q / wpr) * W + (q % wpr) * 32) + (uint32_t)__builtin_ctz(open));
-  }
-  size_t locked = s->inpaint ? N - s->inpaint_n : 0;
-  if (!c.dev_picks) resolved.resize(locked);  // run_pick reads the entries after them
-  size_t n_un = N - locked;
-  // on the device the list starts as it was before the random init, and the
-  // few entries that the swap-removes change are kept in a map
-  const bool sparse = c.dev_picks;
-  std::unordered_map<uint64_t, uint32_t> moved;
-  if (!s->inpaint && !sparse) {
+  } else if (dense) {
     unresolved.resize(N);
     for (size_t i = 0; i < N; ++i) unresolved[i] = (uint32_t)i;
   }
+  std::unordered_map<uint64_t, uint32_t> moved;
+  std::vector<uint64_t> touched;
+  if (p.has_random_init) c.init_list.reserve(6 * std::min<uint64_t>(p.random_init, N));
+  if (dense) touched.reserve(std::min<uint64_t>(p.random_init, N));
   auto pick = [&](uint64_t seed) -> uint32_t {
     Pcg32 r = pcg_from_u64(seed);
     const uint64_t idx = gen_range_u64(r, n_un--);
-    if (sparse) {
-      auto at = [&](uint64_t i) {
-        const auto it = moved.find(i);
-        return it != moved.end() ? it->second : s->inpaint ? unresolved[i] : (uint32_t)i;
-      };
-      const uint32_t v = at(idx);
-      moved[idx] = at(n_un);
+    if (dense) {
+      const uint32_t v = unresolved[idx];
+      unresolved[idx] = unresolved[n_un];
+      touched.push_back(idx);
       return v;
     }
-    const uint32_t v = unresolved[idx];
-    unresolved[idx] = unresolved.back();
-    unresolved.pop_back();
+    auto at = [&](uint64_t i) {
+      const auto it = moved.find(i);
+      return it != moved.end() ? it->second : s->inpaint ? unresolved[i] : (uint32_t)i;
+    };
+    const uint32_t v = at(idx);
+    moved[idx] = at(n_un);
     return v;
   };
   // ---- random init (session.rs:42-52, ms.rs:427-475): all examples ----
@@ -1545,7 +1541,6 @@ void run_plan(ts_session *s, RunCtx &c) {
       const uint8_t *cc = &im.px[((size_t)y * im.w + x) * 4];
       put(px, (uint32_t)cc[0] | ((uint32_t)cc[1] << 8) | ((uint32_t)cc[2] << 16) | ((uint32_t)cc[3] << 24),
           make_uint4(x | (y << 16), px, map, map));
-      if (!c.dev_picks) resolved.push_back(px);
     }
     locked += p.random_init;
   }
@@ -1554,6 +1549,8 @@ void run_plan(ts_session *s, RunCtx &c) {
   c.un_over.clear();
   for (const auto &e : moved)
     if (e.first < n_un) c.un_over.insert(c.un_over.end(), {(uint32_t)e.first, e.second});
+  for (uint64_t i : touched)  // (an entry may come twice, with the same pixel)
+    if (i < n_un) c.un_over.insert(c.un_over.end(), {(uint32_t)i, unresolved[i]});
   // ---- the schedule of Generator::resolve ----
   const int32_t x_l = (int32_t)((float)W * kTilingBoundary), y_b = (int32_t)((float)H * kTilingBoundary);
   const float sig2 = p.cauchy * p.cauchy;
@@ -1565,7 +1562,6 @@ void run_plan(ts_session *s, RunCtx &c) {
     l2[d] = x2;
   }
   std::vector<StagePlan> &plan = c.plan;
-  std::vector<uint32_t> &items = c.items;
   std::vector<float> &luts = c.luts;
   size_t n_res = locked;
   size_t n_unresolved = n_un;
@@ -1643,14 +1639,9 @@ void run_plan(ts_session *s, RunCtx &c) {
     max_stage_items = std::max<uint32_t>(max_stage_items, (uint32_t)P_eff);
     plan.push_back(std::move(sp));
   }
-  // the items themselves come from the pick chain, stage by stage (run_pick,
-  // or on the device)
+  // the items themselves come from the pick chain, stage by stage
   c.n_items = n_items_total;
   c.res_total = n_res;
-  if (!c.dev_picks) {
-    items.assign(n_items_total, 0);
-    resolved.reserve(n_res);  // the picks append without moving the locked entries
-  }
   c.picked_stages = 0;
   // ---- host tables ----
   const uint32_t wpr = (W + 31) / 32;
@@ -1705,37 +1696,11 @@ void run_plan(ts_session *s, RunCtx &c) {
   uint64_t steps_est = 0;
   for (auto &sp : plan) steps_est += sp.batches.size() + 1;
   c.dev_bytes = N * 4 + N * sizeof(uint4) + 2 * (uint64_t)wpr * H * 4 + c.res_total * 8 + c.n_items * 4 +
-                (c.dev_picks ? c.n_unresolved * 20 : 0) +
+                c.n_unresolved * 20 +
                 c.luts.size() * 4 + c.tab.size() * 4 + mb * kk * 12 + mb * (4 + 8 + 4 + sizeof(Result)) +
                 c.n_batches * 4 + (c.rc_ahead ? (uint64_t)c.n_items : std::max<uint64_t>(c.rc_items, mb)) * m * 8 +
                 dist_table_doubles * 8 + steps_est * sizeof(StepDev) +
                 c.cells.size() * 4 + c.init_list.size() * 4 + (s->inpaint ? 2 * (uint64_t)wpr * H * 4 : 0);
-}
-
-// pick_random_unresolved (ms.rs:380-389) for a stage's items: redo item i
-// is resolved[i + locked]; new item i swap-removes
-// Pcg32::seed_from_u64(seed + i).gen_range(0..len) from the unresolved list.
-// The served form's chain; the other forms pick on the device
-// (run_enqueue_picks).
-void run_pick(RunCtx &c) {
-  const StagePlan &sp = c.plan[c.picked_stages++];
-  std::vector<uint32_t> &unresolved = c.unresolved;
-  uint32_t *it = c.items.data() + sp.items_off;
-  const uint32_t redo = std::min(sp.redo, sp.n_items);
-  for (uint32_t i = 0; i < redo; ++i) it[i] = c.resolved[i + c.locked];
-  const size_t n_new = sp.n_items - redo, len0 = unresolved.size();
-  if (n_new > len0) throw Failure{TS_ERR_INVALID_RANGE, "more new items than unresolved pixels"};
-  uint32_t *un = unresolved.data();
-  size_t len = len0;
-  for (size_t q = 0; q < n_new; ++q) {
-    Pcg32 r = pcg_from_u64(sp.seed + (uint64_t)(redo + q));
-    const uint64_t idx = gen_range_u64(r, len);
-    it[redo + q] = un[idx];
-    un[idx] = un[--len];
-  }
-  unresolved.resize(len);
-  for (const BatchPlan &bp : sp.batches)
-    for (uint32_t t = bp.append_from; t < bp.i1; ++t) c.resolved.push_back(it[t]);
 }
 
 // Let the device's default stream-ordered pool keep freed memory (by
@@ -1930,7 +1895,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
                w_kfbl = wl.add(n_kitems * 4), w_xdiv = wl.add(c.n_xdiv * 8), w_ydiv = wl.add(c.n_ydiv * 8),
                w_dxt = wl.add(c.n_xdiv ? (size_t)W * (2 * R + 1) * 8 : 0),
                w_dy2t = wl.add(c.n_xdiv ? (size_t)H * (2 * R + 1) * 8 : 0);
-  const size_t n_un = c.dev_picks ? c.n_unresolved : 0;
+  const size_t n_un = c.n_unresolved;
   const size_t w_un0 = wl.add(n_un * 4), w_un1 = wl.add(n_un * 4), w_phead = wl.add(n_un * 4),
                w_pnext = wl.add(n_un * 4), w_pdraw = wl.add(n_un * 4);
   CUDA_TRY(A(c.d_zero, zl.off));
@@ -1970,7 +1935,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   if (s->inpaint) {
     c.inpaint.open = (const uint32_t *)(tb + t_open);
     c.inpaint.before = (const uint32_t *)(tb + t_before);
-    c.inpaint.un = c.dev_picks ? c.d_un[0].p : nullptr;
+    c.inpaint.un = c.d_un[0].p;
     c.inpaint.n_un = (uint32_t)n_un;
     c.inpaint.map = s->inpaint_index;
   }
@@ -2227,8 +2192,11 @@ void run_upload(RunCtx &c, cudaStream_t st) {
   }
 }
 
-// The pick chain on the device (dev_picks): the unresolved list's start, then
-// a stage at a time, in stage order, on one stream.
+// The pick chain (pick_random_unresolved, ms.rs:380-389), on the device: the
+// unresolved list's start, then a stage at a time, in stage order, on one
+// stream.  Redo item i is entry i of the resolved list after the locked ones;
+// new item i swap-removes Pcg32::seed_from_u64(seed + i).gen_range(0..len) of
+// the unresolved list.
 void run_enqueue_picks_init(RunCtx &c, cudaStream_t st) {
   c.pick_len = c.n_unresolved;
   // (run_upload made inpainting's list)
@@ -2271,7 +2239,7 @@ void run_enqueue_picks(RunCtx &c, cudaStream_t st) {
 // counts), and next starts with a walk or an exhaustive k-NN launch, not
 // the fused small-step kernel, which reads colours.
 bool can_defer_commit(const RunCtx &c, const Step &stp, const Step *next) {
-  if (!stp.batch || stp.bd.fused_commit || c.k == 0 || stp.bd.append_from < stp.bd.i1) return false;
+  if (!stp.batch || stp.bd.fused_commit || c.k == 0 || c.knn_ahead || stp.bd.append_from < stp.bd.i1) return false;
   if (!next || !next->batch || next->ls || next->stage != stp.stage) return false;
   return !(next->exhaustive && next->resolve == kPhaseTeamFull && team_full_fits(c.sd.k, c.sd.m));
 }
@@ -2422,7 +2390,8 @@ void enqueue_step(RunCtx &c, const Step &stp, cudaStream_t st, LaunchTimer &lt, 
   }
   if (stp.batch) {
     lt.items = stp.n;
-    if (c.k > 0 && stp.exhaustive && stp.resolve == kPhaseTeamFull && team_full_fits(sd.k, sd.m)) {
+    const bool knn = c.k > 0 && !c.knn_ahead;
+    if (knn && stp.exhaustive && stp.resolve == kPhaseTeamFull && team_full_fits(sd.k, sd.m)) {
       // small batch, exhaustive k-NN: neighbours, mean and resolve in one launch
       lt.run(TS_KERNEL_RESOLVE, [&] { launch_step_team_full(sd, stp.st, stp.bd, st); });
       c.launches += 1;
@@ -2432,7 +2401,7 @@ void enqueue_step(RunCtx &c, const Step &stp, cudaStream_t st, LaunchTimer &lt, 
       }
       return;
     }
-    if (c.k > 0) {
+    if (knn) {
       if (stp.exhaustive) {
         lt.run(TS_KERNEL_KNN_EXHAUSTIVE, [&] { launch_knn_exhaustive(sd, stp.st, stp.bd, true, st, pc); });
         ++c.launches;
@@ -2444,7 +2413,7 @@ void enqueue_step(RunCtx &c, const Step &stp, cudaStream_t st, LaunchTimer &lt, 
     }
     // the exhaustive k-NN over a whole batch computes the mean itself, and so
     // do the walk and the fallback k-NN for sessions whose sums are exact
-    if (c.k > 0 && !stp.exhaustive && !sd.exact_sum) {
+    if (knn && !stp.exhaustive && !sd.exact_sum) {
       lt.run(TS_KERNEL_MEAN, [&] { launch_mean(sd, stp.st, stp.bd, st); });
       ++c.launches;
     }
@@ -2601,7 +2570,6 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
     };
     c.want_rc_ahead = true;
     c.want_knn_ahead = true;
-    c.want_dev_picks = true;
     run_plan(s, c);
     const double plan_ms = lap();
     run_alloc(c, st);
@@ -2985,7 +2953,6 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
             std::unique_ptr<RunCtx> c(new RunCtx());
             c->multi = true;
             c->want_rc_ahead = true;
-            c->want_dev_picks = true;
             run_plan(sessions[j], *c);
             ctx[j] = std::move(c);
           });
@@ -3449,13 +3416,13 @@ struct ServerReq {
   std::string err;
   ts_generated *result = nullptr;
   bool done = false;
-  // The pick chain runs ahead of the device: stage 0 on the submitting
-  // thread, the rest on a picker thread, into c->pitems; `picked` counts the
-  // stages whose items are there, `uploaded` those the driver has copied
-  // to the device (driver only), `picks_done` guards c against the picker.
-  std::atomic<uint32_t> picked{0};
-  uint32_t uploaded = 0;
-  bool picks_done = false;  // under the server mutex
+  // Made on streams beside the ticks: the picks (pick_ev per stage, where no
+  // lists are made ahead), and with k-NN ahead the chunks of lists, the step
+  // that needs each, and how many are enqueued.
+  cudaStream_t kst = nullptr;  // the server's
+  std::vector<EventHandle> pick_ev;
+  std::vector<size_t> chunk_step;
+  size_t n_chunks = 0;
   cudaEvent_t up_ev = nullptr, ev = nullptr;  // uploads done; last kernels done
   ~ServerReq() {
     if (up_ev) cudaEventDestroy(up_ev);
@@ -3477,8 +3444,7 @@ struct ts_server {
   uint32_t team_max_items = 2048, team_full_max_items = 256;
   double t0 = 0;
   std::mutex mu;
-  std::condition_variable cv_work, cv_done, cv_complete, cv_pick, cv_picked;
-  std::deque<ServerReq *> to_pick;  // requests whose later stages are still to be picked
+  std::condition_variable cv_work, cv_done, cv_complete;
   std::deque<ServerReq *> pending;
   std::atomic<uint32_t> n_pending{0};  // pending.size(), read by the driver without the mutex
   std::unordered_map<uint64_t, ServerReq *> reqs;  // submitted, not yet collected
@@ -3486,13 +3452,13 @@ struct ts_server {
   std::vector<uint32_t> free_slots;
   uint64_t used = 0;
   uint64_t next_ticket = 1;
-  bool stop = false, stop_completer = false, stop_pickers = false;
+  bool stop = false, stop_completer = false;
   int fatal = TS_OK;
   std::string err;
   std::vector<ServerReq *> active;  // driver thread only
   std::thread driver, completer;
-  std::vector<std::thread> pickers;
   cudaStream_t st = nullptr, ust = nullptr, cst = nullptr;  // compute, upload, completion
+  cudaStream_t ks[kBatchKnnStreams] = {}, rs = nullptr;       // picks and neighbour lists; random candidates
   DevBuf<SessionDev> d_sess;
   DevBuf<const StepDev *> d_tabs;
   struct Ring {
@@ -3512,44 +3478,16 @@ void server_fail(ts_server *S, ServerReq *r, const Failure &f) {
   r->err = f.msg;
 }
 
-// The next stage of a request's pick chain, into its pinned items.
-void server_pick_stage(ServerReq &r) {
-  RunCtx &c = *r.c;
-  const size_t q = c.picked_stages;
-  run_pick(c);
-  const StagePlan &sp = c.plan[q];
-  if (sp.n_items) memcpy(c.pitems.p + sp.items_off, c.items.data() + sp.items_off, (size_t)sp.n_items * 4);
-  r.picked.store((uint32_t)q + 1, std::memory_order_release);
-}
-
-void server_picker(ts_server *S) {
-  for (;;) {
-    ServerReq *r = nullptr;
-    {
-      std::unique_lock<std::mutex> lk(S->mu);
-      S->cv_pick.wait(lk, [&] { return S->stop_pickers || !S->to_pick.empty(); });
-      if (S->to_pick.empty()) return;
-      r = S->to_pick.front();
-      S->to_pick.pop_front();
-    }
-    while (r->picked.load(std::memory_order_relaxed) < r->c->plan.size()) {
-      server_pick_stage(*r);
-      std::lock_guard<std::mutex> lk(S->mu);  // the driver may be waiting for this stage
-      S->cv_picked.notify_all();
-    }
-    std::lock_guard<std::mutex> lk(S->mu);
-    r->picks_done = true;
-    S->cv_picked.notify_all();
-  }
-}
-
 // Device buffers, uploads and slot entries of an admitted request, on the
 // upload stream; the compute stream waits for them before its next tick.
+// Random candidates made ahead go out whole, and so do the picks of a request
+// without lists made ahead.
 void server_admit(ts_server *S, ServerReq *r) {
   RunCtx &c = *r->c;
   if (r->s->ready.e) CUDA_TRY(cudaStreamWaitEvent(S->ust, r->s->ready.e, 0));
   run_alloc(c, S->ust);
   run_upload(c, S->ust);
+  if (c.knn_ahead) launch_rank_init(c.sd, (uint32_t)c.locked, S->ust);
   std::vector<StepDev> h(c.steps.size());
   for (size_t t = 0; t < c.steps.size(); ++t) {
     const Step &stp = c.steps[t];
@@ -3572,6 +3510,51 @@ void server_admit(ts_server *S, ServerReq *r) {
   CUDA_TRY(cudaEventCreateWithFlags(&r->ev, cudaEventDisableTiming | cudaEventBlockingSync));
   CUDA_TRY(cudaEventRecord(r->up_ev, S->ust));
   CUDA_TRY(cudaStreamWaitEvent(S->st, r->up_ev, 0));
+  r->kst = S->ks[r->slot % kBatchKnnStreams];
+  CUDA_TRY(cudaStreamWaitEvent(r->kst, r->up_ev, 0));
+  c.knn_ev.resize(c.knn_chunks.size());
+  for (size_t t = 0; t < c.steps.size(); ++t)
+    if (c.steps[t].knn_wait >= 0) r->chunk_step.push_back(t);
+  if (c.rc_ahead) {
+    CUDA_TRY(cudaStreamWaitEvent(S->rs, r->up_ev, 0));
+    c.rc_ev.resize(c.plan.size());
+    for (size_t q = 0; q < c.plan.size(); ++q) {
+      if (c.rc_step[q] < 0) continue;
+      launch_random_candidates(c.sd, c.steps[c.rc_step[q]].rc_st, S->rs);
+      CUDA_TRY(cudaEventCreateWithFlags(&c.rc_ev[q].e, cudaEventDisableTiming));
+      CUDA_TRY(cudaEventRecord(c.rc_ev[q].e, S->rs));
+    }
+  }
+  if (!c.knn_ahead) {
+    run_enqueue_picks_init(c, r->kst);
+    r->pick_ev.resize(c.plan.size());
+    for (EventHandle &e : r->pick_ev) {
+      run_enqueue_picks(c, r->kst);
+      CUDA_TRY(cudaEventCreateWithFlags(&e.e, cudaEventDisableTiming));
+      CUDA_TRY(cudaEventRecord(e.e, r->kst));
+    }
+  }
+}
+
+// What the request's step t needs from the streams beside the ticks; the
+// chunks of the steps after it go out first, so that their lists are made
+// while it runs.
+void server_before_step(ts_server *S, ServerReq *r, size_t t) {
+  RunCtx &c = *r->c;
+  const Step &stp = c.steps[t];
+  if (c.knn_ahead) {
+    LaunchTimer lt;
+    for (; r->n_chunks < r->chunk_step.size() && r->chunk_step[r->n_chunks] <= t + kBatchAheadSteps; ++r->n_chunks) {
+      const size_t q = (size_t)c.steps[r->chunk_step[r->n_chunks]].knn_wait;
+      if (c.picked_stages == 0) run_enqueue_picks_init(c, r->kst);
+      while ((int)c.picked_stages <= c.knn_chunks[q].stage) run_enqueue_picks(c, r->kst);
+      run_enqueue_chunk(c, q, r->kst, r->kst, lt);
+    }
+    if (stp.knn_wait >= 0) CUDA_TRY(cudaStreamWaitEvent(S->st, c.knn_ev[stp.knn_wait].e, 0));
+  } else if (t == 0 || c.steps[t - 1].stage != stp.stage) {
+    CUDA_TRY(cudaStreamWaitEvent(S->st, r->pick_ev[stp.stage].e, 0));
+  }
+  if (stp.rc && c.rc_ahead && c.rc_ev[stp.stage].e) CUDA_TRY(cudaStreamWaitEvent(S->st, c.rc_ev[stp.stage].e, 0));
 }
 
 void server_driver(ts_server *S) {
@@ -3598,6 +3581,14 @@ void server_driver(ts_server *S) {
         r->slot = S->free_slots.back();
         S->free_slots.pop_back();
         r->slotted = true;
+        // lists and random candidates ahead where the budget has room for them
+        RunCtx &c = *r->c;
+        c.want_knn_ahead = true;
+        const uint64_t rc_b = (uint64_t)c.n_items * c.m * 8, knn_b = knn_ahead_bytes(c);
+        c.want_knn_ahead = knn_ahead_fits(c, c.W, c.H, c.k) && S->used + r->bytes + knn_b <= S->budget;
+        if (c.want_knn_ahead) r->bytes += knn_b;
+        c.rc_ahead = c.m > 0 && (uint64_t)c.n_items * c.m <= kRcandWholeSmall && S->used + r->bytes + rc_b <= S->budget;
+        if (c.rc_ahead) r->bytes += rc_b;
         S->used += r->bytes;
         S->stats.peak_bytes = std::max(S->stats.peak_bytes, S->used);
         lk.unlock();
@@ -3621,27 +3612,9 @@ void server_driver(ts_server *S) {
       S->stats.peak_active = std::max<uint64_t>(S->stats.peak_active, S->active.size());
     }
     if (S->active.empty()) continue;
-    // ---- one tick: the next step of every active session whose items are
-    // picked (the others wait for their picker) ----
+    // ---- one tick: the next step of every active session ----
     std::vector<ServerReq *> &ready = ready_buf;
-    ready.clear();
-    for (ServerReq *r : S->active)
-      if (r->c->steps[r->cursor].stage < (int)r->picked.load(std::memory_order_acquire)) ready.push_back(r);
-    if (ready.empty()) {
-      const double w0 = host_ms();
-      // Wait for a picker (or a new request), re-checking under the mutex:
-      // a picker publishes `picked` before it takes the mutex to notify, so
-      // no wake-up is lost between the check above and the wait.
-      std::unique_lock<std::mutex> lk(S->mu);
-      S->cv_picked.wait_for(lk, std::chrono::microseconds(500), [&] {
-        if (S->stop || (!S->pending.empty() && !S->free_slots.empty())) return true;
-        for (ServerReq *r : S->active)
-          if (r->c->steps[r->cursor].stage < (int)r->picked.load(std::memory_order_acquire)) return true;
-        return false;
-      });
-      S->stats.driver_pick_wait_us += (uint64_t)((host_ms() - w0) * 1e3);
-      continue;
-    }
+    ready = S->active;
     const double t_tick0 = host_ms();
     try {
       ts_server::Ring &R = S->ring[ri];
@@ -3650,17 +3623,6 @@ void server_driver(ts_server *S) {
         const double w0 = host_ms();
         CUDA_TRY(cudaEventSynchronize(R.ev));
         ring_wait = host_ms() - w0;
-      }
-      for (ServerReq *r : ready) {
-        // items of the stages picked so far, in stream order before the launches
-        RunCtx &c = *r->c;
-        const uint32_t upto = r->picked.load(std::memory_order_acquire);
-        for (; r->uploaded < upto; ++r->uploaded) {
-          const StagePlan &sp = c.plan[r->uploaded];
-          if (sp.n_items)
-            CUDA_TRY(cudaMemcpyAsync(c.d_items.p + sp.items_off, c.pitems.p + sp.items_off,
-                                     (size_t)sp.n_items * 4, cudaMemcpyHostToDevice, S->st));
-        }
       }
       uint64_t step_items = 0;
       bool all_team_full = true;
@@ -3683,21 +3645,18 @@ void server_driver(ts_server *S) {
       if (ready.size() == 1) {
         // one session in the tick: its steps with the single-session kernels
         // (no segment lookups at the start of every block).  While nothing
-        // waits for admission it takes up to kLoneSteps consecutive steps
-        // whose items are picked, as the plain path would (a redo-only
-        // batch's commit then rides in the next step's first k-NN launch),
-        // so that the host's per-tick work does not pace a lone request; a
-        // request that arrives meanwhile joins at the next tick.
+        // waits for admission it takes up to kLoneSteps consecutive steps, as
+        // the plain path would (without lists made ahead a redo-only batch's
+        // commit then rides in the next step's first k-NN launch), so that
+        // the host's per-tick work does not pace a lone request; a request
+        // that arrives meanwhile joins at the next tick.
         ServerReq *r0 = ready[0];
         RunCtx &c = *r0->c;
         const uint64_t before = c.launches;
         LaunchTimer lt;
         const double l0 = host_ms();
-        // only stages whose items went up above: a picker may have
-        // published more since
-        const uint32_t uploaded = r0->uploaded;
         const size_t limit = S->n_pending.load(std::memory_order_relaxed) ? 1 : kLoneSteps;
-        auto usable = [&](size_t t) { return t < c.steps.size() && c.steps[t].stage < (int)uploaded; };
+        auto usable = [&](size_t t) { return t < c.steps.size(); };
         const Step *pending = nullptr;
         size_t n = 0;
         while (n < limit && usable(r0->cursor + n)) {
@@ -3714,6 +3673,7 @@ void server_driver(ts_server *S) {
                                                                                          : kPhaseTeamPart;
           }
           const bool defer = more && can_defer_commit(c, stp, &c.steps[r0->cursor + n + 1]);
+          server_before_step(S, r0, r0->cursor + n);
           enqueue_step(c, stp, S->st, lt, pending, defer);
           pending = defer ? &stp : nullptr;
           ++n;
@@ -3722,6 +3682,7 @@ void server_driver(ts_server *S) {
         launch_ms += host_ms() - l0;
         tick_launches = c.launches - before;
       } else {
+        for (ServerReq *r : ready) server_before_step(S, r, r->cursor);
         for (int ph = 0; ph < kPhases; ++ph) {
           PlannedLaunch pl;
           pl.phase = ph;
@@ -3800,10 +3761,6 @@ void server_driver(ts_server *S) {
       std::vector<ServerReq *> still;
       std::vector<ServerReq *> finished;
       for (ServerReq *r : S->active) {
-        if (std::find(ready.begin(), ready.end(), r) == ready.end()) {
-          still.push_back(r);
-          continue;
-        }
         RunCtx &c = *r->c;
         for (size_t q = 0; q < lone_steps; ++q) {
           const Step &stp = c.steps[r->cursor];
@@ -3879,10 +3836,9 @@ void server_completer(ts_server *S) {
     }
     const bool admitted = r->slotted;
     if (r->ev) cudaEventSynchronize(r->ev);  // no kernel of the request is left
-    {
-      std::unique_lock<std::mutex> lk(S->mu);  // nor is its picker (after a failure)
-      S->cv_picked.wait(lk, [&] { return r->picks_done; });
-    }
+    if (r->status != TS_OK)  // nor, after a failure, anything beside the ticks
+      for (cudaStream_t q : {S->ust, r->kst, S->rs, S->st})
+        if (q) cudaStreamSynchronize(q);
     // the run's buffers are pool memory (freed in stream order, no device
     // wait); the session's pyramids are freed with it
     r->c.reset();
@@ -3926,7 +3882,13 @@ ts_server *ts_server_new(int32_t device, uint64_t hbm_budget_bytes, uint32_t max
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
     S->budget = hbm_budget_bytes ? hbm_budget_bytes : (uint64_t)(free_b / 2);
-    CUDA_TRY(cudaStreamCreateWithFlags(&S->st, cudaStreamNonBlocking));
+    // the ticks first, then the lists their next steps need, then the random
+    // candidates
+    int prio_low = 0, prio_high = 0;
+    CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
+    CUDA_TRY(cudaStreamCreateWithPriority(&S->st, cudaStreamNonBlocking, prio_high));
+    for (cudaStream_t &q : S->ks) CUDA_TRY(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, prio_low - 1));
+    CUDA_TRY(cudaStreamCreateWithPriority(&S->rs, cudaStreamNonBlocking, prio_low));
     CUDA_TRY(cudaStreamCreateWithFlags(&S->ust, cudaStreamNonBlocking));
     CUDA_TRY(cudaStreamCreateWithFlags(&S->cst, cudaStreamNonBlocking));
     CUDA_TRY(S->d_sess.alloc(S->max_active));
@@ -3944,10 +3906,6 @@ ts_server *ts_server_new(int32_t device, uint64_t hbm_budget_bytes, uint32_t max
   S->t0 = host_ms();
   S->driver = std::thread(server_driver, S.get());
   S->completer = std::thread(server_completer, S.get());
-  const unsigned hc = std::max(1u, std::thread::hardware_concurrency());
-  // half the host threads (at most eight) run pick chains: with many
-  // requests waiting they, not the device, bound the server's throughput
-  for (unsigned i = 0; i < std::min(8u, std::max(1u, hc / 2)); ++i) S->pickers.emplace_back(server_picker, S.get());
   return S.release();
 }
 
@@ -3965,13 +3923,6 @@ void ts_server_free(ts_server *S) {
     S->cv_complete.notify_all();
   }
   if (S->completer.joinable()) S->completer.join();
-  {
-    std::lock_guard<std::mutex> lk(S->mu);
-    S->stop_pickers = true;
-    S->cv_pick.notify_all();
-  }
-  for (auto &t : S->pickers)
-    if (t.joinable()) t.join();
   for (auto &kv : S->reqs) delete kv.second;
   if (S->st) cudaStreamSynchronize(S->st);
   for (auto &R : S->ring) {
@@ -3983,6 +3934,9 @@ void ts_server_free(ts_server *S) {
   if (S->st) cudaStreamDestroy(S->st);
   if (S->ust) cudaStreamDestroy(S->ust);
   if (S->cst) cudaStreamDestroy(S->cst);
+  for (cudaStream_t q : S->ks)
+    if (q) cudaStreamDestroy(q);
+  if (S->rs) cudaStreamDestroy(S->rs);
   delete S;
 }
 
@@ -4021,16 +3975,13 @@ int ts_server_submit(ts_server *S, ts_session *s, uint64_t *ticket) {
   r->c.reset(new RunCtx());
   try {
     RunCtx &c = *r->c;
+    c.multi = true;
     run_plan(r->s, c);  // host schedule, on the caller's thread
-    if (cudaSuccess != c.pitems.alloc(c.items.size())) throw Failure{TS_ERR_CUDA, "pinned host memory"};
-    if (!c.plan.empty()) server_pick_stage(*r);  // stage 0 here, the rest on a picker thread
   } catch (const Failure &f) {
     S->err = f.msg;
     return f.status;
   }
   r->bytes = r->c->dev_bytes + r->s->dev_bytes;
-  const bool more = r->picked.load() < r->c->plan.size();
-  r->picks_done = !more;
   std::lock_guard<std::mutex> lk(S->mu);
   if (S->fatal) {
     S->err = "server stopped after a device error";
@@ -4039,15 +3990,10 @@ int ts_server_submit(ts_server *S, ts_session *s, uint64_t *ticket) {
   r->ticket = S->next_ticket++;
   *ticket = r->ticket;
   S->reqs[r->ticket] = r.get();
-  if (more) {
-    S->to_pick.push_back(r.get());
-    S->cv_pick.notify_one();
-  }
   S->pending.push_back(r.release());
   S->n_pending.store((uint32_t)S->pending.size(), std::memory_order_relaxed);
   S->stats.submitted += 1;
   S->cv_work.notify_one();
-  S->cv_picked.notify_all();  // a driver waiting on pickers admits it at once
   return TS_OK;
 }
 
