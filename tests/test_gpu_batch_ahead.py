@@ -43,3 +43,19 @@ def test_served(ts, oracle, wl):
     tickets = [server.submit(ts.builder_from_spec(s).build()) for s in specs]
     for q, (t, s) in enumerate(zip(tickets, specs)):
         assert_same(ts.generated_outputs(server.wait(t)[0]), oracle.run(s, nthreads=8), "request %d" % q)
+
+
+@pytest.mark.parametrize("n", [3, 90])
+def test_guided_beside_unguided(ts, wl, n):
+    """Steps whose guided and unguided sessions share a launch, and steps of
+    more blocks than one launch takes (90 sessions of 64^2)."""
+    specs = []
+    for q in range(n):
+        spec = wl.config2(out=64, ex=24) if q % 2 else wl.config0(out=64, ex=24)
+        spec["params"].update({"nearest_neighbors": 4, "random_sample_locations": 2, "seed": q})
+        specs.append(spec)
+    batch = ts.Batch()
+    for s in specs:
+        batch.add(ts.builder_from_spec(s).build())
+    for q, (g, s) in enumerate(zip(batch.run(), specs)):
+        assert_same(ts.generated_outputs(g), ts.run_spec(s), "session %d" % q)

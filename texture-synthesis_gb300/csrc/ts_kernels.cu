@@ -2915,7 +2915,10 @@ __global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
 __global__ void __launch_bounds__(kResolveWarps *kWarp, 8) k_resolve_multi(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
-  resolve_body<false>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+  if (v.s->guided)
+    resolve_body<false>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+  else
+    resolve_body<true>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
 }
 // Segments of sessions without guides.
 __global__ void __launch_bounds__(kResolveWarps *kWarp, 8) k_resolve_multi_lean(MultiLaunch ml) {
@@ -3823,6 +3826,11 @@ size_t multi_smem_bytes(int phase, uint32_t k, uint32_t m) {
   }
 }
 
+static constexpr uint32_t kResolveOneLaunch = 152u * 8u * 8u;
+uint32_t resolve_launches(uint32_t n_lean, uint32_t n_segs, uint32_t blocks) {
+  return n_lean && n_lean < n_segs && blocks > kResolveOneLaunch ? 2 : 1;
+}
+
 void launch_multi(int phase, const MultiLaunch &ml, uint32_t blocks, size_t smem, cudaStream_t stream) {
   if (blocks == 0) return;  // a launch may carry only the exhaustive k-NN's fallback pool (no segments)
   const uint32_t t = multi_threads(phase);
@@ -3833,8 +3841,17 @@ void launch_multi(int phase, const MultiLaunch &ml, uint32_t blocks, size_t smem
     case kPhaseExhaustive: launch_pdl(k_knn_exhaustive_multi, blocks, t, smem, stream, ml); break;
     case kPhaseMean: launch_pdl(k_mean_multi, blocks, t, 0, stream, ml); break;
     case kPhaseResolve: {
-      // segments [0, n_lean) belong to sessions without guides (lean kernel,
-      // blocks [0, lean_blocks)); the rest run the general kernel
+      // Segments [0, n_lean) belong to sessions without guides (blocks
+      // [0, lean_blocks)).  Two launches, one after the other, each wait for
+      // their slowest item, so both kinds share one up to eight rounds of the
+      // GPU's blocks (16 requests: two launches 21.2 ms, one up to 2, 4, 8, 16
+      // rounds 20.0, 19.5, 19.4, 19.3); beyond, where the work counts, the
+      // lean kernel spills less (24 sessions of up to 1024^2: 64.0 ms against
+      // 64.5 always in one)
+      if (ml.n_lean < ml.n_segs && resolve_launches(ml.n_lean, ml.n_segs, blocks) == 1) {
+        launch_pdl(k_resolve_multi, blocks, t, smem, stream, ml);
+        break;
+      }
       MultiLaunch a = ml, g = ml;
       a.n_segs = ml.n_lean;
       g.segs = ml.segs + ml.n_lean;

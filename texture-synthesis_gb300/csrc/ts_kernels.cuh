@@ -238,6 +238,9 @@ enum : int {
 uint32_t multi_threads(int phase);
 uint32_t multi_blocks(int phase, uint32_t n, uint32_t cap);
 size_t multi_smem_bytes(int phase, uint32_t k, uint32_t m);
+// Kernels that a resolve phase of n_segs segments (the first n_lean without
+// guides) and `blocks` blocks goes out as.
+uint32_t resolve_launches(uint32_t n_lean, uint32_t n_segs, uint32_t blocks);
 void launch_multi(int phase, const MultiLaunch &ml, uint32_t blocks, size_t smem, cudaStream_t stream);
 // Lets a phase's multi-session kernel use `bytes` of dynamic shared memory
 // (current device).

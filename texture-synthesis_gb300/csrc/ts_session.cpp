@@ -3337,7 +3337,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     bs.launches = launches.size() + rc_launches.size();
     for (size_t j = 0; j < n; ++j) bs.launches += ctx[j]->launches;
     for (const PlannedLaunch &pl : launches)
-      if (pl.phase == kPhaseResolve && pl.n_lean && pl.n_lean < pl.n_segs) bs.launches += 1;  // two kernels
+      if (pl.phase == kPhaseResolve) bs.launches += resolve_launches(pl.n_lean, pl.n_segs, pl.blocks) - 1;
     bs.phase_launches[kPhaseRandom] += rc_launches.size();
     bs.plan_ms = plan_ms;
     {
@@ -3751,7 +3751,7 @@ void server_driver(ts_server *S) {
         }
         tick_launches = launches.size();
         for (const PlannedLaunch &pl : launches)
-          if (pl.phase == kPhaseResolve && pl.n_lean && pl.n_lean < pl.n_segs) tick_launches += 1;
+          if (pl.phase == kPhaseResolve) tick_launches += resolve_launches(pl.n_lean, pl.n_segs, pl.blocks) - 1;
       }
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(cudaEventRecord(R.ev, S->st));
