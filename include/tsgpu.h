@@ -307,7 +307,8 @@ int ts_builder_batch_schedule(ts_builder *b, uint32_t batch_divisor, uint32_t ma
  * at most `full_max_batch` items score every candidate of an item with one
  * CTA (lowest latency); up to `team_max_batch` items, one CTA per item with
  * early exit; larger batches, one warp per item (highest throughput).
- * Defaults 2048 and 256. */
+ * Defaults 2048 and 256 (1024 and 256 for more than 32 neighbours, where
+ * neither this nor ts_builder_tuning is called). */
 int ts_builder_resolve_team(ts_builder *b, uint32_t team_max_batch, uint32_t full_max_batch);
 /* CUDA device ordinal (default 0). */
 int ts_builder_device(ts_builder *b, int32_t device);
@@ -455,7 +456,8 @@ typedef struct ts_tuning {
   double gpu_ms;                   /* median device time of the workload with this setting */
   double default_gpu_ms;           /* the same with the defaults */
 } ts_tuning;
-/* The defaults: 2048, 256 and 4096 items. */
+/* The defaults: 2048, 256 and 4096 items.  (A session that is given none takes
+ * 1024 instead of 2048 where it has more than 32 neighbours.) */
 void ts_tuning_default(ts_tuning *out);
 /* A fresh, configured builder for one run of the workload on each call; the
  * tuner builds it, runs it and frees it.  NULL ends the tuning with

@@ -18,3 +18,14 @@ def test_warp_form(ts, oracle, wl, n_ex, k, m, w, h):
     spec["params"].update(nearest_neighbors=k, random_sample_locations=m, random_init=3)
     got = ts.run_spec(spec, team_max_batch=0, team_full_max_batch=0)
     assert_same(got, oracle.run(spec, nthreads=4), "warp form %d maps k %d m %d %dx%d" % (n_ex, k, m, w, h))
+
+
+@pytest.mark.parametrize("k", [32, 33])
+def test_default_forms(ts, oracle, wl, k):
+    """Steps of 1024 to 2048 items with the thresholds left alone, on both
+    sides of the neighbour count from which they take the warp form."""
+    spec = wl.config0(out=128, ex=24)
+    spec["params"].update(nearest_neighbors=k, random_sample_locations=3)
+    ref = oracle.run(spec, nthreads=8)
+    assert_same(ts.run_spec(spec), ref, "k = %d" % k)
+    assert_same(ts.run_spec(spec, team_max_batch=2048), ref, "k = %d, thresholds set" % k)

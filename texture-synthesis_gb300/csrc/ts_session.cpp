@@ -54,6 +54,12 @@ constexpr uint64_t kRcandBudget = 64ull << 20;  // random-candidate entries held
 // build a bitmap window instead of more rounds of bitmap loads (the default;
 // ts_builder_tuning sets it per session).
 constexpr uint32_t kWalkWindowItems = 4096;
+// Where the caller leaves the thresholds alone, a single session of more than
+// 32 neighbours (which take a warp two rounds) leaves the CTA per item from
+// this many items of a step on: 2048 -> 1024, k = m = 50: 500^2 5.11 -> 4.94
+// ms, 512^2 5.19 -> 5.14, guided 6.37 -> 6.28, 613x409 4.22 -> 4.17; with 768
+// guided 6.30 and 256^2 2.19 -> 2.26; k = 8, 203x117: 1.10 -> 1.11.
+constexpr uint32_t kTeamItemsWide = 1024;
 // Runs whose random candidates for every stage fit this many entries make
 // them all ahead, on a side stream, while the first stages run.  From
 // kRcandWholeSmall entries (2 GB) on only a run by itself does, and only where
@@ -105,6 +111,7 @@ struct Params {
   bool profile = false;
   uint32_t team_max_batch = 2048;
   uint32_t team_full_max_batch = 256;
+  bool team_set = false;  // by the caller
   uint32_t walk_window_max = kWalkWindowItems;
 };
 
@@ -915,6 +922,7 @@ int ts_builder_resolve_team(ts_builder *b, uint32_t team_max_batch, uint32_t ful
   BUILDER_GUARD(b);
   b->prm.team_max_batch = team_max_batch;
   b->prm.team_full_max_batch = full_max_batch;
+  b->prm.team_set = true;
   return TS_OK;
 }
 int ts_builder_tuning(ts_builder *b, const ts_tuning *t) {
@@ -922,6 +930,7 @@ int ts_builder_tuning(ts_builder *b, const ts_tuning *t) {
   if (!t) return TS_ERR_NULL;
   b->prm.team_max_batch = t->team_max_items;
   b->prm.team_full_max_batch = t->team_full_max_items;
+  b->prm.team_set = true;
   b->prm.walk_window_max = t->walk_window_max_items;
   return TS_OK;
 }
@@ -1827,6 +1836,8 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   } zl, tl, wl;
   const size_t kk = std::max<uint32_t>(k, 1), mb = max_batch_items;
   const size_t rc_n = c.rc_ahead ? c.n_items * m : (size_t)std::max<uint64_t>(rc_items, mb) * m;
+  const uint32_t team_max =
+      !p.team_set && k > 32 ? std::min(p.team_max_batch, kTeamItemsWide) : p.team_max_batch;
   // k-NN ahead: the batch table and the chunks (consecutive batches of a
   // stage with one k-NN form, each at least as large as the stage's items
   // before it, so that a chunk's k-NN overlaps the resolves of the ones
@@ -2096,7 +2107,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
         // a batch of new items only: none of them is in the tree, so no item
         // reads another's pixel, state or bit, and each commits as it resolves
         bd.fused_commit = bp.i0 >= sp.redo ? 1 : 0;
-        if (stp.n <= p.team_max_batch)
+        if (stp.n <= team_max)
           stp.resolve = (stp.n <= p.team_full_max_batch && team_full_fits(k, m)) ? kPhaseTeamFull : kPhaseTeamPart;
         else
           stp.resolve = kPhaseResolve;
