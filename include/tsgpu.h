@@ -131,7 +131,7 @@ enum {
   TS_KERNEL_LEVEL_SWITCH = 5,
   TS_KERNEL_MEAN = 6,
   /* Not a kernel: the main stream waiting for a chunk of neighbour lists
-   * made ahead on the k-NN stream (plain path, power-of-two outputs);
+   * made ahead on the k-NN stream (ts_run_stats.knn_chunks);
    * its time is the main stream's stall. */
   TS_KERNEL_KNN_WAIT = 7,
   TS_KERNEL_KINDS = 8
@@ -338,8 +338,10 @@ const char *ts_session_last_error(const ts_session *s);
  * byte-identical to ts_session_run on it (the same batch schedule, the same
  * kernels' arithmetic); what changes is how the work reaches the GPU: every
  * batch step of every session becomes one segment of a shared launch per
- * phase (k-NN, mean, resolve, commit, ...), so one launch carries the step
- * of up to all sessions at once instead of one tiny launch per session. */
+ * phase (resolve, commit, ...), so one launch carries the step of up to all
+ * sessions at once instead of one tiny launch per session; the neighbour
+ * lists that the steps need are made ahead on other streams, where memory
+ * allows, else in the step. */
 typedef struct ts_batch ts_batch;
 typedef struct ts_batch_stats {
   uint64_t sessions;

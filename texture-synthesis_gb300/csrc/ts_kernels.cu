@@ -1,6 +1,9 @@
 // ts_kernels.cu — sm_103a kernels of the texture-synthesis hot loop.
 //
-// One batch step of a synthesis stage is five launches:
+// One batch step of a synthesis stage is five parts, a launch each where the
+// step makes its own neighbour lists; with the lists made ahead, a chunk of
+// steps at a time on other streams (k_tree_append, then knn_list or knn_walk,
+// knn_exhaustive and mean_ahead), the step is its resolve launch alone:
 //   knn_walk        warp per work item: the k nearest resolved points under
 //                   the (d2, y, x) order, by walking a table of lattice offsets
 //                   sorted in that order and testing a resolved-point bitmap
@@ -10,9 +13,8 @@
 //   mean            thread per item: the mean of the 4x-duplicated distance
 //                   list (ms.rs:417-423), the in-order f64 sum, one item per
 //                   lane (large batches); for whole small batches the
-//                   exhaustive k-NN computes it on one thread in integer
-//                   arithmetic, whose dependent chain is shorter than f64's
-//   resolve         warp per item: neighbour weights (ms.rs:1198-1203) in
+//                   exhaustive k-NN computes it on one thread
+//   resolve         warp per item (a CTA in small steps): neighbour weights (ms.rs:1198-1203) in
 //                   double-f32 arithmetic with an exact f64 fallback,
 //                   coherence + random candidates (ms.rs:478-602), own
 //                   pattern (ms.rs:1151-1181), candidate cost and first-min

@@ -106,7 +106,7 @@ struct SessionDev {
   uint32_t *cells;
   int32_t cox, coy;
   uint32_t cgw, cgh;
-  // Tree positions, for k-NN made ahead of the resolves (plain path,
+  // Tree positions, for k-NN made ahead of the resolves (written by
   // k_tree_append): rank[p] = 1 + p's index in the resolved list, 0 while p
   // has none.  The bitmap, mirror bits, cell counts and resolved list then
   // already hold the points of whole chunks of later batches; a point is in

@@ -5,9 +5,10 @@
 // image validation, input resizes, example / guide pyramids (built on the
 // device), generator initialisation.  run() mirrors Session::run
 // (session.rs:37-66) and Generator::resolve (ms.rs:702-1051): the host lays
-// out the whole data-independent schedule (stage seeds and sizes, the order
-// in which unresolved pixels are picked, the batch steps, the cost tables),
-// uploads it once and enqueues every kernel on one stream; the only
+// out the whole data-independent schedule (stage seeds and sizes, the batch
+// steps, the cost tables), uploads it once and enqueues every kernel: the
+// chain of batch steps on one stream, what does not depend on it (the picks,
+// the neighbour lists, the random candidates) on others; the only
 // synchronisation is at the end (and once per stage when a progress callback
 // is given).
 #include <math.h>
