@@ -29,3 +29,11 @@ def test_default_forms(ts, oracle, wl, k):
     ref = oracle.run(spec, nthreads=8)
     assert_same(ts.run_spec(spec), ref, "k = %d" % k)
     assert_same(ts.run_spec(spec, team_max_batch=2048), ref, "k = %d, thresholds set" % k)
+
+
+@pytest.mark.parametrize("k", [9, 10, 11, 15, 16, 17, 21])
+def test_guided_chunks(ts, oracle, wl, k):
+    """Neighbour counts around the guided loop's chunks (4, then six at a time)."""
+    spec = wl.config2(out=48, ex=40)
+    spec["params"].update(nearest_neighbors=k, random_sample_locations=12)
+    assert_same(ts.run_spec(spec, team_max_batch=0, team_full_max_batch=0), oracle.run(spec, nthreads=8), "k = %d" % k)
