@@ -32,3 +32,24 @@ def test_clustered_points(ts, oracle, wl, w, h, k):
     spec["params"].update(nearest_neighbors=k, random_sample_locations=4)
     got = ts.run_spec(spec)
     assert_same(got, oracle.run(spec, nthreads=8), "clustered %dx%d k %d" % (w, h, k))
+
+
+def test_far_cluster_sums(ts, oracle, wl):
+    """A locked block of 32 x 19 pixels at one end of the widest output: 19 of
+    an item's neighbours fall to one lane, each up to 16383 columns away, so
+    that their squared offsets pass 2^32 (19 * 15035^2).  The sample mask
+    leaves the far items their random candidates, whose scores hold the
+    weights (a neighbour's own candidate would match the block exactly)."""
+    w, h, k = 16384, 32, 256
+    spec = wl.inpaint_session(3, side=32)
+    spec["out_w"], spec["out_h"] = w, h
+    sample = np.zeros((h, w, 4), np.uint8)
+    sample[:, :256] = 255
+    spec["examples"] = [{"image": wl.texture(22, h, w), "sample": "image", "mask": sample}]
+    mask = np.zeros((h, w, 4), np.uint8)
+    mask[:19, :32] = 255
+    spec["inpaint_mask"] = mask
+    spec["params"].update(nearest_neighbors=k, random_sample_locations=2, backtrack_stages=0)
+    got = ts.run_spec(spec, batch_divisor=1)
+    assert got["stats"]["knn_chunks"] > 0
+    assert_same(got, oracle.run(spec, batch_divisor=1, nthreads=16), "far cluster")

@@ -1204,7 +1204,9 @@ __device__ __forceinline__ void knn_list_body(const SessionDev &s, const StageDe
     // each key's place: the number of smaller ones (keys are distinct)
     const uint32_t nout = min(n, s.k);
     int32_t *nbo = b.nbuf + (size_t)local * s.k;
-    uint32_t ux = 0, uy = 0;
+    // 64-bit: a lane holds up to (2 k + 96) / 32 keys, whose squared offsets
+    // reach 2^28 each (a cluster at the other end of a 16384-wide output)
+    unsigned long long units = 0;
     for (uint32_t e0 = 0; e0 < n; e0 += kWarp) {
       const uint32_t e = e0 + lane;
       const unsigned long long key = e < n ? keys[e] : ~0ull;
@@ -1214,12 +1216,11 @@ __device__ __forceinline__ void knn_list_body(const SessionDev &s, const StageDe
       if (e < n && r < nout) {
         const int dx = (int)(key & 0xffffu) - 32768 - px, dy = (int)((key >> 16) & 0xffffu) - 32768 - py;
         nbo[r] = pack_off(dx, dy);
-        ux += (uint32_t)(dx * dx);
-        uy += (uint32_t)(dy * dy);
+        units += exact_units(s, dx, dy);
       }
     }
     if (s.exact_sum) {
-      const unsigned long long units = (warp_sum_units(ux) << s.exact_sx) + (warp_sum_units(uy) << s.exact_sy);
+      units = warp_sum_units(units);
       if (lane == 0 && nout) b.mean[local] = exact_mean(s, units, nout);
     }
     if (lane == 0) b.ncnt[local] = nout;
