@@ -1,0 +1,54 @@
+"""Device memory that runs take and keep, from the driver's counters of the
+default stream-ordered pool."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+class DevMem:
+    def __init__(self):
+        self.cu = C.CDLL("libcuda.so.1")
+        dev, ctx, self.pool = C.c_int(), C.c_void_p(), C.c_void_p()
+        self._check(self.cu.cuInit(0))
+        self._check(self.cu.cuDeviceGet(C.byref(dev), 0))
+        self._check(self.cu.cuDevicePrimaryCtxRetain(C.byref(ctx), dev))
+        self._check(self.cu.cuCtxSetCurrent(ctx))
+        self._check(self.cu.cuDeviceGetDefaultMemPool(C.byref(self.pool), dev))
+
+    @staticmethod
+    def _check(rc):
+        assert rc == 0, "CUDA driver status %d" % rc
+
+    def leaving(self, keep, run):
+        """run() with all but `keep` bytes of the device taken."""
+        self._check(self.cu.cuCtxSynchronize())
+        self._check(self.cu.cuMemPoolTrimTo(self.pool, C.c_size_t(0)))
+        free, total, p = C.c_size_t(), C.c_size_t(), C.c_uint64()
+        self._check(self.cu.cuMemGetInfo_v2(C.byref(free), C.byref(total)))
+        self._check(self.cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(free.value - keep)))
+        try:
+            return run()
+        finally:
+            self._check(self.cu.cuMemFree_v2(p))
+
+
+@pytest.fixture(scope="module")
+def mem():
+    return DevMem()
+
+
+def test_lists_ahead_leave_room(ts, wl, mem):
+    """4.1 GB of neighbour lists with 4 GB of the device free: the run, which
+    needs a quarter of that without them, makes them per step instead."""
+    spec = wl.config0(out=64, ex=64)
+    spec["out_w"], spec["out_h"] = 2000, 1001
+    spec["params"].update(nearest_neighbors=256, random_sample_locations=1)
+    tight = mem.leaving(4 << 30, lambda: ts.run_spec(spec))
+    assert tight["stats"]["knn_chunks"] == 0
+    free = ts.run_spec(spec)
+    assert free["stats"]["knn_chunks"] > 0
+    for key in ("image", "coord", "id", "resolved", "scores"):
+        assert np.array_equal(tight[key], free[key]), key

@@ -1457,9 +1457,11 @@ bool knn_ahead_fits(const RunCtx &c, uint32_t W, uint32_t H, uint32_t k) {
          (uint64_t)c.n_items * ((uint64_t)k * 4 + 16) <= kKnnAheadMaxBytes;
 }
 
-// Bytes the k-NN ahead adds to a run's buffers (run_alloc).
+// Bytes the k-NN ahead adds to a run's buffers (run_alloc); a run by itself
+// also takes the shadow and a second result buffer.
 uint64_t knn_ahead_bytes(const RunCtx &c) {
-  return (uint64_t)c.n_items * ((uint64_t)c.k * 4 + 16) + (uint64_t)c.N * 4;
+  return (uint64_t)c.n_items * ((uint64_t)c.k * 4 + 16) + (uint64_t)c.N * 4 +
+         (c.multi ? 0 : (uint64_t)c.N * 2 * sizeof(uint4) + (uint64_t)c.max_batch_items * sizeof(Result));
 }
 
 // Device memory that the stream-ordered pool can still hand out.
@@ -1473,6 +1475,17 @@ uint64_t device_room(int dev) {
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
     free_b += reserved - used;
   return free_b;
+}
+
+// Whether the device has room for the lists of a run by itself: as with the
+// random candidates, large ones only where there is four times the room beside
+// the rest of the run, so that runs side by side, and what the program holds
+// besides, still fit.  (The query takes the driver some time, which small runs
+// go without; run_alloc_fit covers those.)
+bool knn_ahead_room(const RunCtx &c) {
+  constexpr uint64_t kKnnAheadSmall = 256ull << 20;
+  const uint64_t lists = knn_ahead_bytes(c);
+  return lists <= kKnnAheadSmall || device_room(c.s->prm.device) >= c.dev_bytes + 4 * lists;
 }
 
 // Host schedule of Generator::resolve (ms.rs:702-1051) and the device
@@ -2164,7 +2177,27 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   }
 }
 
-// Uploads of the initial state, enqueued on st.
+// run_alloc; where the device has no memory for it, the lists and then the
+// random candidates are made per step instead of ahead.
+void run_alloc_fit(RunCtx &c, cudaStream_t pool) {
+  for (;;) {
+    try {
+      run_alloc(c, pool);
+      return;
+    } catch (const Failure &f) {
+      if (f.status != TS_ERR_OUT_OF_MEMORY || !(c.knn_ahead || c.rc_ahead)) throw;
+    }
+    cudaGetLastError();  // the refused allocation's status
+    c.d_zero.reset();
+    c.d_tabs.reset();
+    c.d_work.reset();
+    if (c.knn_ahead)
+      c.want_knn_ahead = false;
+    else
+      c.rc_ahead = false;
+  }
+}
+
 // The session's tables in a pinned block laid out as the device's table
 // arena (ready for one copy); the batched form makes it on its planning
 // threads, the other paths in run_upload.
@@ -2577,8 +2610,9 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
     c.want_rc_ahead = true;
     c.want_knn_ahead = true;
     run_plan(s, c);
+    c.want_knn_ahead = knn_ahead_fits(c, c.W, c.H, c.k) && knn_ahead_room(c);
     const double plan_ms = lap();
-    run_alloc(c, st);
+    run_alloc_fit(c, st);
     run_stage_tables(c);  // its pinned block too, before the device clock starts
     const double alloc_ms = lap();
     EventPair ev, ev_up, ev_rb;
@@ -2973,7 +3007,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
           if (ctx[j])
             guarded(j, [&] {
               RunCtx &c = *ctx[j];
-              run_alloc(c, st);
+              run_alloc_fit(c, st);
               run_stage_tables(c);
               // touch the read-back destinations here, in parallel, rather
               // than in the copies at the end of the run
@@ -3489,7 +3523,7 @@ void server_fail(ts_server *S, ServerReq *r, const Failure &f) {
 void server_admit(ts_server *S, ServerReq *r) {
   RunCtx &c = *r->c;
   if (r->s->ready.e) CUDA_TRY(cudaStreamWaitEvent(S->ust, r->s->ready.e, 0));
-  run_alloc(c, S->ust);
+  run_alloc_fit(c, S->ust);
   run_upload(c, S->ust);
   if (c.knn_ahead) launch_rank_init(c.sd, (uint32_t)c.locked, S->ust);
   std::vector<StepDev> h(c.steps.size());
