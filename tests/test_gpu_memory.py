@@ -7,6 +7,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+RESERVED_CURRENT, USED_CURRENT, USED_HIGH = 5, 7, 8  # CUmemPool_attribute
+
 
 class DevMem:
     def __init__(self):
@@ -21,6 +23,20 @@ class DevMem:
     @staticmethod
     def _check(rc):
         assert rc == 0, "CUDA driver status %d" % rc
+
+    def pool_bytes(self, attr):
+        v = C.c_uint64()
+        self._check(self.cu.cuMemPoolGetAttribute(self.pool, attr, C.byref(v)))
+        return v.value
+
+    def peak(self, run):
+        """Most pool bytes that run() adds to those in use."""
+        self._check(self.cu.cuCtxSynchronize())
+        zero = C.c_uint64(0)
+        self._check(self.cu.cuMemPoolSetAttribute(self.pool, USED_HIGH, C.byref(zero)))
+        before = self.pool_bytes(USED_CURRENT)
+        run()
+        return self.pool_bytes(USED_HIGH) - before
 
     def leaving(self, keep, run):
         """run() with all but `keep` bytes of the device taken."""
@@ -38,6 +54,24 @@ class DevMem:
 @pytest.fixture(scope="module")
 def mem():
     return DevMem()
+
+
+def test_sequential_schedule(ts, wl, mem):
+    """One item a step: what the run holds more than one of larger steps is a
+    few words a step (a fallback counter, the table of the steps' trees), not
+    the warp resolve's 512 bytes of counters, which such steps never read."""
+    spec = wl.config0(out=64, ex=16)
+    spec["params"].update(nearest_neighbors=4, random_sample_locations=2)
+    stats = {}
+
+    def run(divisor):
+        stats[divisor] = ts.run_spec(spec, batch_divisor=divisor)["stats"]
+
+    run(8)
+    few, many = mem.peak(lambda: run(8)), mem.peak(lambda: run(0))
+    steps = stats[0]["batches"] - stats[8]["batches"]
+    assert steps > 4096
+    assert many - few <= 64 * steps, (few, many, steps)
 
 
 def test_lists_ahead_leave_room(ts, wl, mem):

@@ -1420,7 +1420,7 @@ struct RunCtx {
   DevBuf<uint32_t> d_color, d_occ, d_mir, d_res, d_items, d_ncnt, d_fbl, d_fbc, d_cells, d_init;
   DevBuf<uint32_t> d_rank, d_kncnt, d_kfbl, d_kfbc;  // knn_ahead
   DevBuf<uint32_t> d_un[2], d_phead, d_pnext, d_pdraw, d_over;  // the picks
-  DevBuf<uint32_t> d_wctr;  // per batch: the warp resolve's item counters (BatchDev::work_ctr)
+  DevBuf<uint32_t> d_wctr;  // per step of the warp form: its item counters (BatchDev::work_ctr)
   DevBuf<int32_t> d_knbuf;
   DevBuf<double> d_kmean;
   DevBuf<uint2> d_btab;
@@ -1892,7 +1892,12 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     }
   }
   const size_t n_chunks = c.knn_chunks.size(), n_kitems = c.knn_ahead ? c.n_items : 0;
-  const size_t n_wctr = c.multi ? 0 : c.n_batches * kWorkCtrs * kWorkCtrStride;
+  // the item counters of the steps that the warp form resolves (a schedule of
+  // many small steps has none: one item a step, 2048^2: 4.3 GB if every step had its own)
+  size_t n_warp_steps = 0;
+  for (const StagePlan &sp : plan)
+    for (const BatchPlan &bp : sp.batches) n_warp_steps += bp.i1 - bp.i0 > team_max ? 1 : 0;
+  const size_t n_wctr = c.multi ? 0 : n_warp_steps * kWorkCtrs * kWorkCtrStride;
   const size_t n_result = (c.knn_ahead && !c.multi ? 2 : 1) * mb;
   // zeroed: colour and state first (inpainting writes them whole instead)
   const size_t z_color = zl.add(N * 4), z_state = zl.add(N * sizeof(uint4)), z_rscore = zl.add(c.res_total * 4),
@@ -2045,7 +2050,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   c.pend = false;
 
   // ---- the steps ----
-  size_t fb_index = 0;
+  size_t fb_index = 0, warp_step = 0;
   uint32_t bidx = 0;
   c.rc_step.assign(plan.size(), -1);
   for (size_t si = 0; si < plan.size(); ++si) {
@@ -2105,7 +2110,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
         bd.res = c.d_result.p;
         stp.n = bp.i1 - bp.i0;
         stp.stage_i0 = bp.i0;
-        if (!c.multi) bd.work_ctr = c.d_wctr.p + (size_t)bidx * kWorkCtrs * kWorkCtrStride;
+        if (!c.multi && stp.n > team_max) bd.work_ctr = c.d_wctr.p + warp_step++ * kWorkCtrs * kWorkCtrStride;
         stp.bidx = bidx++;
         if (c.knn_ahead) {  // the chunk's lists, made ahead on the k-NN stream
           const size_t g0 = (size_t)sp.items_off + bp.i0;
