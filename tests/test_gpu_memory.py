@@ -86,3 +86,20 @@ def test_lists_ahead_leave_room(ts, wl, mem):
     assert free["stats"]["knn_chunks"] > 0
     for key in ("image", "coord", "id", "resolved", "scores"):
         assert np.array_equal(tight[key], free[key]), key
+
+
+def test_served_requests_share_a_tight_budget(ts, wl):
+    """Four equal requests under a budget of four of them run side by side:
+    what could be made ahead does not take the next ones' room."""
+    spec = wl.config0(out=512, ex=64)
+    with ts.Server(hbm_budget=1, max_active=4) as srv:  # alone, nothing made ahead
+        alone = srv.wait(srv.submit(ts.builder_from_spec(spec).build()))[0].into_image()
+        one = srv.stats()["peak_bytes"]
+    sessions = [ts.builder_from_spec(spec).build() for _ in range(4)]
+    with ts.Server(hbm_budget=4 * one, max_active=4) as srv:
+        tickets = [srv.submit(s) for s in sessions]
+        images = [srv.wait(t)[0].into_image() for t in tickets]
+        stats = srv.stats()
+    assert stats["peak_active"] == 4, stats
+    assert stats["peak_bytes"] <= 4 * one
+    assert all(np.array_equal(im, alone) for im in images)

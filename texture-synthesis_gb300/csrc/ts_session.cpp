@@ -3624,13 +3624,25 @@ void server_driver(ts_server *S) {
         r->slot = S->free_slots.back();
         S->free_slots.pop_back();
         r->slotted = true;
-        // lists and random candidates ahead where the budget has room for them
+        // Lists and random candidates ahead where the budget has room for them
+        // beside what may yet share the device: the waiting requests, and one
+        // like this for every slot that is still free.  (Without that the first
+        // requests took the room of the next ones: of four of 512^2 under a
+        // budget of four, three ran at once.)
         RunCtx &c = *r->c;
+        uint64_t others = 0;
+        size_t slots = S->free_slots.size();
+        for (auto q = S->pending.begin(); q != S->pending.end() && slots; ++q, --slots) others += (*q)->bytes;
+        others += slots * r->bytes;
+        const uint64_t held = S->used + others;
+        // (the whole list of candidates takes the place of a chunk's)
+        const uint64_t rc_n = c.n_items, chunk_n = std::max<uint64_t>(c.rc_items, c.max_batch_items);
+        const uint64_t rc_b = (rc_n - std::min(rc_n, chunk_n)) * c.m * 8;
+        const uint64_t knn_b = knn_ahead_bytes(c);
         c.want_knn_ahead = true;
-        const uint64_t rc_b = (uint64_t)c.n_items * c.m * 8, knn_b = knn_ahead_bytes(c);
-        c.want_knn_ahead = knn_ahead_fits(c, c.W, c.H, c.k) && S->used + r->bytes + knn_b <= S->budget;
+        c.want_knn_ahead = knn_ahead_fits(c, c.W, c.H, c.k) && held + r->bytes + knn_b <= S->budget;
         if (c.want_knn_ahead) r->bytes += knn_b;
-        c.rc_ahead = c.m > 0 && (uint64_t)c.n_items * c.m <= kRcandWholeSmall && S->used + r->bytes + rc_b <= S->budget;
+        c.rc_ahead = c.m > 0 && (uint64_t)c.n_items * c.m <= kRcandWholeSmall && held + r->bytes + rc_b <= S->budget;
         if (c.rc_ahead) r->bytes += rc_b;
         S->used += r->bytes;
         S->stats.peak_bytes = std::max(S->stats.peak_bytes, S->used);
