@@ -103,3 +103,11 @@ def test_served_requests_share_a_tight_budget(ts, wl):
     assert stats["peak_active"] == 4, stats
     assert stats["peak_bytes"] <= 4 * one
     assert all(np.array_equal(im, alone) for im in images)
+
+
+def test_pool_is_given_back(ts, wl, mem):
+    """A run of some 18 GB of buffers leaves at most 16 GiB in the pool."""
+    spec = wl.config0(out=2048, ex=64)
+    spec["params"].update(nearest_neighbors=256, random_sample_locations=129)
+    assert mem.peak(lambda: ts.run_spec(spec)) > 16 << 30
+    assert mem.pool_bytes(RESERVED_CURRENT) <= 16 << 30

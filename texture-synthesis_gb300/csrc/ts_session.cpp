@@ -1740,6 +1740,21 @@ void keep_pool(int dev) {
   done.push_back(dev);
 }
 
+// What a run's buffers leave in the device's pool above kPoolKeep goes back to
+// the device when the run is over (declared before the buffers and streams).
+constexpr uint64_t kPoolKeep = 16ull << 30;
+struct PoolTrim {
+  int dev;
+  ~PoolTrim() {
+    cudaMemPool_t pool;
+    uint64_t reserved = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        reserved > kPoolKeep)
+      cudaMemPoolTrimTo(pool, kPoolKeep);
+  }
+};
+
 // Whether a session's neighbour-distance sums (get_distances_to_k_neighs,
 // ms.rs:405-425) are exact.  With W and H powers of two, x / W and y / H are
 // exact, so every distance fma(dx, dx, dy * dy) is an integer multiple of
@@ -2589,7 +2604,8 @@ extern "C" int ts_session_run(ts_session *s, ts_progress_fn progress, void *user
   }
   s->consumed = true;
   const auto t_wall0 = std::chrono::steady_clock::now();
-  StreamGuard sg;  // declared first: the run's pool buffers are freed on it before it goes
+  PoolTrim trim{s->prm.device};
+  StreamGuard sg;  // declared before c: the run's pool buffers are freed on it before it goes
   StreamGuard rg;  // side stream of the random candidates made ahead
   StreamGuard kg;  // k-NN stream (knn_ahead)
   StreamGuard mg;  // the means of inexact lists
@@ -2833,7 +2849,6 @@ struct PlannedLaunch {
 // the same within 1%.  Their buffers take at most kBatchAheadMaxBytes.
 constexpr size_t kBatchKnnStreams = 8, kBatchAheadSteps = 24;
 constexpr uint64_t kBatchAheadMaxBytes = 48ull << 30;
-constexpr uint64_t kBatchPoolKeep = 16ull << 30;
 
 // Blocks of the exhaustive k-NN's fallback pool (three 64 KB CTAs per SM).
 constexpr uint32_t kFallbackPool = 152u * 3u;
@@ -2924,15 +2939,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       for (ts_session *s : v) delete s;
     }
   } owned{sessions};
-  // what the batch's buffers leave in the device's pool above kBatchPoolKeep
-  // goes back to the device
-  struct Trim {
-    int dev;
-    ~Trim() {
-      cudaMemPool_t pool;
-      if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) cudaMemPoolTrimTo(pool, kBatchPoolKeep);
-    }
-  } trim{b->device};
+  PoolTrim trim{b->device};
   // main stream, side stream (picks, random candidates made ahead)
   // and copy stream (read-backs); outside the try so that a failure can
   // drain them before the sessions' buffers go
