@@ -447,7 +447,8 @@ void ts_server_stats_get(ts_server *s, ts_server_stats *out);
  * build a bitmap window in shared memory.  The thresholds between these
  * never change a result, only the speed, which depends on the GPU, the
  * sizes, k and m.  The tuner runs the caller's own workload under candidate
- * thresholds, one threshold at a time starting from the defaults, and keeps
+ * thresholds, one threshold at a time starting from the defaults (of the
+ * builder, for a session), and keeps
  * a candidate only when its median device time over `repeats` runs beats
  * the best so far by more than 1%. */
 typedef struct ts_tuning {
@@ -458,9 +459,12 @@ typedef struct ts_tuning {
   double gpu_ms;                   /* median device time of the workload with this setting */
   double default_gpu_ms;           /* the same with the defaults */
 } ts_tuning;
-/* The defaults: 2048, 256 and 4096 items.  (A session that is given none takes
- * 1024 instead of 2048 where it has more than 32 neighbours.) */
+/* The defaults: 2048, 256 and 4096 items. */
 void ts_tuning_default(ts_tuning *out);
+/* What a session of this builder takes when it is given none: the defaults,
+ * but 1024 instead of 2048 items for more than 32 neighbours (as the builder
+ * has them now).  The session tuner starts from these. */
+int ts_builder_tuning_default(const ts_builder *b, ts_tuning *out);
 /* A fresh, configured builder for one run of the workload on each call; the
  * tuner builds it, runs it and frees it.  NULL ends the tuning with
  * TS_ERR_STATE. */

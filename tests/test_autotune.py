@@ -94,3 +94,13 @@ def test_build_failure_stops_the_tuner(ts, wl):
         ts.autotune_session(make, repeats=1)
     assert e.value.status == 10  # TS_ERR_CUDA
     assert len(calls) == 1
+
+
+def test_default_setting_of_a_builder(ts):
+    """What a session takes that is given no setting, from which the session
+    tuner starts: more than 32 neighbours leave the CTA per item earlier."""
+    for k, team in [(1, 2048), (32, 2048), (33, 1024), (50, 1024)]:
+        t = ts.Session.builder().nearest_neighbors(k).tuning_default()
+        assert (t.team_max_items, t.team_full_max_items, t.walk_window_max_items) == (team, 256, 4096)
+        assert t.trials == 0
+    assert ts.lib().ts_builder_tuning_default(None, C.byref(ts.Tuning())) == TS_ERR_NULL

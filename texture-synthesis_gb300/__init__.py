@@ -226,6 +226,7 @@ SIGNATURES = {
     "ts_autotune_session": (C.c_int, [_BUILDER_FACTORY, C.c_void_p, C.c_uint32, C.POINTER(Tuning)]),
     "ts_autotune_batch": (C.c_int, [C.c_int32, _BATCH_FILLER, C.c_void_p, C.c_uint32, C.POINTER(Tuning)]),
     "ts_builder_tuning": (C.c_int, [C.c_void_p, C.POINTER(Tuning)]),
+    "ts_builder_tuning_default": (C.c_int, [C.c_void_p, C.POINTER(Tuning)]),
     "ts_batch_tuning": (C.c_int, [C.c_void_p, C.POINTER(Tuning)]),
     "ts_server_tuning": (C.c_int, [C.c_void_p, C.POINTER(Tuning)]),
     "ts_measure_gather_peak": (C.c_int, [C.c_int32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_int32,
@@ -478,6 +479,12 @@ class SessionBuilder:
         """Launch-shape thresholds (a Tuning from autotune_session, or
         Tuning.default()); the results do not depend on them."""
         return self._check(lib().ts_builder_tuning(self._h, C.byref(tuning)))
+
+    def tuning_default(self):
+        """The Tuning a session of this builder takes when it is given none."""
+        t = Tuning()
+        self._check(lib().ts_builder_tuning_default(self._h, C.byref(t)))
+        return t
 
     def profile_kernels(self, on=True):
         """Time every kernel launch with CUDA events (measurement runs)."""

@@ -5,7 +5,7 @@
 // run statistics' gpu_ms, CUDA events on the launching stream).  Every
 // threshold setting gives byte-identical results, so the search can only
 // change the speed.  The search is one threshold at a time from the
-// defaults (resolve team range, full-scoring range, walk window range),
+// defaults (a session's: ts_builder_tuning_default; resolve team range, full-scoring range, walk window range),
 // each over a fixed candidate list; a candidate replaces the best setting
 // only when its median time beats it by more than 1%, so that run-to-run
 // noise does not move the setting.
@@ -27,19 +27,18 @@ double median(std::vector<double> v) {
   return n % 2 ? v[n / 2] : 0.5 * (v[n / 2 - 1] + v[n / 2]);
 }
 
-// run_once(setting, &ms) runs the workload once and gives its device time.
+// run_once(setting, &ms) runs the workload once and gives its device time;
+// run_once(nullptr, &ms) runs it untuned and sets `start`.
 template <typename RunOnce>
-int tune(RunOnce &&run_once, uint32_t repeats, bool walk, ts_tuning *out) {
+int tune(RunOnce &&run_once, const ts_tuning &start, uint32_t repeats, bool walk, ts_tuning *out) {
   if (!out) return TS_ERR_NULL;
   if (repeats == 0) repeats = 1;
-  ts_tuning best;
-  ts_tuning_default(&best);
   uint32_t trials = 0;
   auto measure = [&](const ts_tuning &t, double &ms) -> int {
     std::vector<double> v;
     for (uint32_t r = 0; r < repeats; ++r) {
       double one = 0.0;
-      const int rc = run_once(t, one);
+      const int rc = run_once(&t, one);
       ++trials;
       if (rc != TS_OK) return rc;
       v.push_back(one);
@@ -50,16 +49,17 @@ int tune(RunOnce &&run_once, uint32_t repeats, bool walk, ts_tuning *out) {
   // one untimed run first: a process's first runs pay one-time set-up
   // (module loading, memory pools, pinned staging)
   double ms = 0.0;
-  int rc = run_once(best, ms);
+  int rc = run_once(nullptr, ms);
   ++trials;
   if (rc != TS_OK) return rc;
+  ts_tuning best = start;
   double best_ms = 0.0;
   if ((rc = measure(best, best_ms)) != TS_OK) return rc;
   const double default_ms = best_ms;
   auto sweep = [&](uint32_t ts_tuning::*field, const uint32_t *cand, size_t nc) -> int {
-    const ts_tuning start = best;
+    const ts_tuning base = best;
     for (size_t i = 0; i < nc; ++i) {
-      ts_tuning t = start;
+      ts_tuning t = base;
       t.*field = cand[i];
       // full scoring applies only inside the team range
       if (field == &ts_tuning::team_max_items) t.team_full_max_items = std::min(t.team_full_max_items, cand[i]);
@@ -108,11 +108,15 @@ void ts_tuning_default(ts_tuning *out) {
 
 int ts_autotune_session(ts_builder_factory make, void *user, uint32_t repeats, ts_tuning *out) {
   if (!make) return TS_ERR_NULL;
-  auto run_once = [&](const ts_tuning &t, double &ms) -> int {
+  ts_tuning start;
+  ts_tuning_default(&start);
+  auto run_once = [&](const ts_tuning *t, double &ms) -> int {
     ts_builder *b = make(user);
     if (!b) return TS_ERR_STATE;
     ts_session *s = nullptr;
-    int rc = ts_builder_tuning(b, &t);
+    int rc = TS_OK;
+    if (!t) rc = ts_builder_tuning_default(b, &start);
+    if (rc == TS_OK) rc = ts_builder_tuning(b, t ? t : &start);
     if (rc == TS_OK) rc = ts_builder_build(b, &s);
     ts_builder_free(b);
     if (rc != TS_OK) return rc;
@@ -126,15 +130,17 @@ int ts_autotune_session(ts_builder_factory make, void *user, uint32_t repeats, t
     ms = st.gpu_ms;
     return TS_OK;
   };
-  return tune(run_once, repeats, true, out);
+  return tune(run_once, start, repeats, true, out);
 }
 
 int ts_autotune_batch(int32_t device, ts_batch_filler fill, void *user, uint32_t repeats, ts_tuning *out) {
   if (!fill) return TS_ERR_NULL;
-  auto run_once = [&](const ts_tuning &t, double &ms) -> int {
+  ts_tuning start;
+  ts_tuning_default(&start);
+  auto run_once = [&](const ts_tuning *t, double &ms) -> int {
     ts_batch *b = ts_batch_new(device);
     if (!b) return TS_ERR_OUT_OF_MEMORY;
-    int rc = ts_batch_tuning(b, &t);
+    int rc = ts_batch_tuning(b, t ? t : &start);
     if (rc == TS_OK) rc = fill(b, user);
     std::vector<ts_generated *> res(ts_batch_size(b), nullptr);
     if (rc == TS_OK && res.empty()) rc = TS_ERR_STATE;
@@ -148,7 +154,7 @@ int ts_autotune_batch(int32_t device, ts_batch_filler fill, void *user, uint32_t
     ts_batch_free(b);
     return rc;
   };
-  return tune(run_once, repeats, false, out);
+  return tune(run_once, start, repeats, false, out);
 }
 
 }  // extern "C"

@@ -60,7 +60,8 @@ constexpr uint32_t kWalkWindowItems = 4096;
 // this many items of a step on: 2048 -> 1024, k = m = 50: 500^2 5.11 -> 4.94
 // ms, 512^2 5.19 -> 5.14, guided 6.37 -> 6.28, 613x409 4.22 -> 4.17; with 768
 // guided 6.30 and 256^2 2.19 -> 2.26; k = 8, 203x117: 1.10 -> 1.11.
-constexpr uint32_t kTeamItemsWide = 1024;
+constexpr uint32_t kTeamItems = 2048, kTeamItemsWide = 1024, kTeamFullItems = 256;
+uint32_t default_team_items(uint32_t k) { return k > 32 ? kTeamItemsWide : kTeamItems; }
 // Runs whose random candidates for every stage fit this many entries make
 // them all ahead, on a side stream, while the first stages run.  From
 // kRcandWholeSmall entries (2 GB) on only a run by itself does, and only where
@@ -110,9 +111,9 @@ struct Params {
   uint32_t max_batch = 0;
   int device = 0;
   bool profile = false;
-  uint32_t team_max_batch = 2048;
-  uint32_t team_full_max_batch = 256;
-  bool team_set = false;  // by the caller
+  uint32_t team_max_batch = kTeamItems;  // where the caller set it (team_set), else default_team_items
+  uint32_t team_full_max_batch = kTeamFullItems;
+  bool team_set = false;
   uint32_t walk_window_max = kWalkWindowItems;
 };
 
@@ -924,6 +925,12 @@ int ts_builder_resolve_team(ts_builder *b, uint32_t team_max_batch, uint32_t ful
   b->prm.team_max_batch = team_max_batch;
   b->prm.team_full_max_batch = full_max_batch;
   b->prm.team_set = true;
+  return TS_OK;
+}
+int ts_builder_tuning_default(const ts_builder *b, ts_tuning *out) {
+  if (!b || !out) return TS_ERR_NULL;
+  ts_tuning_default(out);
+  out->team_max_items = default_team_items(b->prm.k);
   return TS_OK;
 }
 int ts_builder_tuning(ts_builder *b, const ts_tuning *t) {
@@ -1865,8 +1872,8 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
   } zl, tl, wl;
   const size_t kk = std::max<uint32_t>(k, 1), mb = max_batch_items;
   const size_t rc_n = c.rc_ahead ? c.n_items * m : (size_t)std::max<uint64_t>(rc_items, mb) * m;
-  const uint32_t team_max =
-      !p.team_set && k > 32 ? std::min(p.team_max_batch, kTeamItemsWide) : p.team_max_batch;
+  // (a batch or a server sets its steps' forms itself, from their summed items)
+  const uint32_t team_max = p.team_set ? p.team_max_batch : default_team_items(k);
   // k-NN ahead: the batch table and the chunks (consecutive batches of a
   // stage with one k-NN form, each at least as large as the stage's items
   // before it, so that a chunk's k-NN overlaps the resolves of the ones
