@@ -1626,8 +1626,8 @@ __device__ __forceinline__ float candidate0_score(const SessionDev &s, const Sta
 }
 
 // The reference's sequential find_best_match (ms.rs:1184-1221), for stages or
-// items with non-finite or negative costs, where early exit and argmin need
-// its exact comparison sequence.  One thread.  Candidates from n_coh on lie
+// items with non-finite costs, where early exit and argmin need its exact
+// comparison sequence.  One thread.  Candidates from n_coh on lie
 // `gap` records further.
 template <bool kG = true>
 __device__ void sequential_best(const SessionDev &s, const StageDev &st, const WarpSmem &w, const float *lc,
@@ -1671,6 +1671,83 @@ __device__ void sequential_best(const SessionDev &s, const StageDev &st, const W
       best_s = score;
       best_i = c;
     }
+  }
+}
+
+// Which cost tables a copy of a resolve body takes.  The single-session kernels
+// come in two copies: in order (kLutSigned) and the rest, whose registers and
+// code the former would cost guided runs 1%.
+enum CostMode { kCostPlain, kCostSigned, kCostAny };
+template <int kMode>
+__device__ __forceinline__ bool costs_in_order(const StageDev &st) {
+  return kMode == kCostSigned || (kMode == kCostAny && st.slow_lut == kLutSigned);
+}
+template <int kMode>
+__device__ __forceinline__ bool costs_exact(const StageDev &st) {
+  return kMode == kCostPlain ? st.slow_lut != 0 : kMode == kCostAny && st.slow_lut == kLutExact;
+}
+
+// A warp's candidates in index order (lane l: candidate first + l), each taken
+// where its largest partial sum lies below the best score so far (why:
+// best_in_order).
+__device__ __forceinline__ void take_signed(float sum, float peak, uint32_t first, float &best_s, uint32_t &best_i) {
+  uint32_t later = 0xffffffffu;
+  for (;;) {
+    const uint32_t below = __ballot_sync(0xffffffffu, peak < best_s) & later;
+    if (below == 0) return;
+    const int l = __ffs(below) - 1;
+    best_s = __shfl_sync(0xffffffffu, sum, l);
+    best_i = first + (uint32_t)l;
+    later = 0xfffffffeu << l;
+  }
+}
+
+// find_best_match for finite tables with negative entries (kLutSigned), where a
+// partial sum can fall again: a whole warp, a candidate per lane.  The
+// reference rejects a candidate at the first partial sum that reaches the best
+// score so far, so it takes one exactly when its largest partial sum lies below
+// that score, which its own then replaces.  The score only falls, so a
+// candidate may be left once it reaches the one at the start of its round, and
+// a repeat of an earlier candidate is never taken (that one was rejected by a
+// best that was no lower, or its sum, no more than its largest partial sum,
+// became the best).  Guided inpainting, k = m = 50, one lane going through all
+// candidates against this, device time: 256^2 2.61 against 0.53 ms, 512^2 3.39
+// against 0.91, 1024^2 6.75 against 2.22.
+template <bool kG = true>
+__device__ void best_in_order(const SessionDev &s, const StageDev &st, const WarpSmem &w, const float *lc,
+                              const float *lg, uint32_t nk, uint32_t nc, float &best_s, uint32_t &best_i) {
+  const uint32_t lane = threadIdx.x & 31u;
+  // candidate 0 is always taken (its sums are finite): its terms on all lanes
+  best_s = candidate0_score<kWarp, kG>(s, st, w, lc, lg, nk, (int)lane, 0xffffffffu);
+  best_i = 0;
+  for (uint32_t base = 1; base < nc; base += kWarp) {
+    const uint32_t c = base + lane;
+    float score = 0.0f, peak = __builtin_huge_valf();
+    if (c < nc) {
+      peak = -FLT_MAX;
+      const uint2 cd = w.cand[c];
+      const uint32_t map = cd.y & 0x7fffu;
+      const int sg = (cd.y & kAuxNeg) ? -1 : 1;
+      const MapDesc md = s.maps[map];
+      const uint32_t *lv = s.levels + md.off + (size_t)st.level * md.w * md.h;
+      const int cx = (int)(cd.x & 0xffffu), cy = (int)(cd.x >> 16);
+      for (uint32_t j = 0; j < nk && peak < best_s; ++j) {
+        const uint4 nr = w.nbr[j];
+        const int qx = cx + sg * off_dx(w.off[j]), qy = cy + sg * off_dy(w.off[j]);
+        float nps = lut4(lc, __vabsdiffu4(nr.y, texel(lv, md, qx, qy)), 0.0f);
+        if (kG && s.guided) {
+          const GuideDesc gd = s.gdesc[map];
+          const uint32_t *gv = s.guides + gd.off + (size_t)st.level * gd.w * gd.h;
+          uint32_t gt = kOutside;
+          if ((unsigned)qx < gd.w && (unsigned)qy < gd.h) gt = gv[(size_t)qy * gd.w + qx];
+          nps = lut4(lg, __vabsdiffu4(nr.z, gt), nps);
+        }
+        score = __fadd_rn(score, __fmul_rn(nps, __uint_as_float(nr.w)));
+        peak = fmaxf(peak, score);
+      }
+    }
+    __syncwarp();
+    take_signed(score, peak, base, best_s, best_i);
   }
 }
 
@@ -1835,7 +1912,7 @@ __device__ void write_bad_result(const SessionDev &s, const StageDev &st, const 
 // a 32-bit __match_any_sync: 2 cycles of the SM per distinct value, 4 with 64
 // bits (an atomicMin per lane into a shared hash table: 1 per lane of a slot,
 // and most lanes share one).  Resolves of 2048^2 tiling: 25.8 -> 21.5 ms.
-template <bool kLean>
+template <bool kLean, int kMode>
 __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev &st, const BatchDev &b, uint32_t vb,
                                              uint32_t vg) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1925,9 +2002,9 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
         __syncwarp();
       }
     };
-    coherence(!st.slow_lut);
+    coherence(!costs_exact<kMode>(st));
     const bool nan_any = __any_sync(0xffffffffu, nan_w);
-    if (!st.slow_lut && nan_any) coherence(false);
+    if (!costs_exact<kMode>(st) && nan_any) coherence(false);
     if (__any_sync(0xffffffffu, bad_map)) {
       // the reference panics on this index; record the error and leave the
       // pixel untouched (commit skips results with an invalid map)
@@ -1937,14 +2014,16 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
     // random candidates after the coherence ones
     const uint2 *rc = st.rcand + (size_t)item * s.m;
     for (uint32_t t = lane; t < s.m; t += kWarp) w.cand[ncoh + t] = random_candidate(s, rc, t);
-    const bool slow = st.slow_lut || nan_any;
+    const bool slow = costs_exact<kMode>(st) || nan_any;
     maxoff = __reduce_max_sync(0xffffffffu, maxoff);
     const bool padded = maxoff <= kPad && !s.guide_dims_differ;
     __syncwarp();
     const uint32_t nc = ncoh + s.m;
     float best_s = FLT_MAX;
     uint32_t best_i = 0;
-    if (!slow) {
+    if (!slow && costs_in_order<kMode>(st)) {
+      best_in_order<!kLean>(s, st, w, lc, lg, nk, nc, best_s, best_i);
+    } else if (!slow) {
       // candidate 0 first: its terms on all lanes, their in-order sum on
       // every lane; it wins ties with every later candidate, so the rest run
       // against min(S_0, f32::MAX) from the start, and a cost of 0 ends the
@@ -2000,7 +2079,7 @@ __device__ __forceinline__ void resolve_body(const SessionDev &s, const StageDev
 // result is the reference's.  Latency per item is about one candidate's
 // evaluation, which suits batches too small to fill the GPU with warps.
 // ---------------------------------------------------------------------------
-template <int T, bool kFull>
+template <int T, bool kFull, int kMode>
 __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const StageDev &st, const BatchDev &b,
                                                   uint32_t vb, uint32_t vg) {
   constexpr int NW = T / 32;
@@ -2276,6 +2355,8 @@ __device__ __forceinline__ void resolve_team_body(const SessionDev &s, const Sta
           best_i = red_i[i];
         }
       }
+    } else if (costs_in_order<kMode>(st) && !(sh_flags & 1)) {
+      if (warp == 0) best_in_order(s, st, w, lc, lg, nk, nc, best_s, best_i);
     } else if (tid == 0) {
       sequential_best(s, st, w, lc, lg, nk, nc, best_s, best_i);
     }
@@ -2939,7 +3020,14 @@ __global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
               const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
   pdl_enter();
   if (pc.n) pending_commit(s, pc);
-  resolve_body<false>(s, st, b, blockIdx.x, gridDim.x);
+  resolve_body<false, kCostPlain>(s, st, b, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
+    k_resolve_signed(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
+                     const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
+  pdl_enter();
+  if (pc.n) pending_commit(s, pc);
+  resolve_body<false, kCostSigned>(s, st, b, blockIdx.x, gridDim.x);
 }
 // Sessions without guides (the guide terms compiled out).
 __global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
@@ -2947,21 +3035,21 @@ __global__ void __launch_bounds__(kResolveWarps *kWarp, 8)
                    const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
   pdl_enter();
   if (pc.n) pending_commit(s, pc);
-  resolve_body<true>(s, st, b, blockIdx.x, gridDim.x);
+  resolve_body<true, kCostPlain>(s, st, b, blockIdx.x, gridDim.x);
 }
 __global__ void __launch_bounds__(kResolveWarps *kWarp, 8) k_resolve_multi(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
   if (v.s->guided)
-    resolve_body<false>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+    resolve_body<false, kCostAny>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
   else
-    resolve_body<true>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+    resolve_body<true, kCostPlain>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
 }
 // Segments of sessions without guides.
 __global__ void __launch_bounds__(kResolveWarps *kWarp, 8) k_resolve_multi_lean(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
-  resolve_body<true>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+  resolve_body<true, kCostPlain>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
 }
 
 template <int T, bool kFull>
@@ -2970,13 +3058,13 @@ __global__ void __launch_bounds__(T)
                    const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc) {
   pdl_enter();
   if (pc.n) pending_commit(s, pc);
-  resolve_team_body<T, kFull>(s, st, b, blockIdx.x, gridDim.x);
+  resolve_team_body<T, kFull, kCostPlain>(s, st, b, blockIdx.x, gridDim.x);
 }
 template <int T, bool kFull>
 __global__ void __launch_bounds__(T) k_resolve_team_multi(MultiLaunch ml) {
   pdl_enter();
   const SegView v = find_segment(ml);
-  resolve_team_body<T, kFull>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
+  resolve_team_body<T, kFull, kCostAny>(*v.s, v.d->st, v.d->b, v.vb, v.vg);
 }
 
 // ---------------------------------------------------------------------------
@@ -3015,7 +3103,7 @@ __host__ __device__ __forceinline__ size_t small_smem_bytes(uint32_t k, uint32_t
          (size_t)(k + m) * term_pitch(k) * 4;
 }
 
-template <int T, bool kG>
+template <int T, bool kG, int kMode>
 __device__ __forceinline__ void resolve_small_body(const SessionDev &s, const StageDev &st, const BatchDev &b,
                                                    const PendingCommit &pc, uint32_t F) {
   constexpr int NW = T / kWarp;
@@ -3171,9 +3259,10 @@ __device__ __forceinline__ void resolve_small_body(const SessionDev &s, const St
       ccol[s.k + t] = __ldg(s.plevels + c);
     }
     const bool far = __syncthreads_or(maxoff > kPad) || s.guide_dims_differ;
-    const bool slow = __syncthreads_or(nan_w) || st.slow_lut;
+    const bool in_order = costs_in_order<kMode>(st);
+    const bool slow = __syncthreads_or(nan_w) || costs_exact<kMode>(st);
     // the random candidates' first f texels
-    const uint32_t f = min(F, nk), n_rnd = slow ? 0u : s.m * f;
+    const uint32_t f = in_order ? nk : min(F, nk), n_rnd = slow ? 0u : s.m * f;
     const float rf = __fdividef(1.0f, (float)f);
     auto split = [&](uint32_t i, float r, uint32_t n, uint32_t &c, uint32_t &j) {
       c = (uint32_t)(((float)i + 0.5f) * r);  // i / n, exact below 2^20
@@ -3341,7 +3430,28 @@ __device__ __forceinline__ void resolve_small_body(const SessionDev &s, const St
           my_i = i;
         }
       };
-      if (f == nk) {
+      if (in_order) {
+        // each candidate's {cost, largest partial sum} into its row, then in order
+        const uint32_t nc = ncoh + s.m;
+        for (uint32_t q = tid; q < nc; q += T) {
+          float *row = rows + (q < ncoh ? q : s.k + q - ncoh) * pitch;
+          float sum = 0.0f, peak = -FLT_MAX;
+          for (uint32_t j = 0; j < nk; ++j) {
+            sum = __fadd_rn(sum, row[j]);
+            peak = fmaxf(peak, sum);
+          }
+          *(float2 *)row = make_float2(sum, peak);
+        }
+        __syncthreads();
+        if (warp == 0) {
+          for (uint32_t base = 0; base < nc; base += kWarp) {
+            const uint32_t q = base + lane;
+            float2 v = make_float2(0.0f, __builtin_huge_valf());
+            if (q < nc) v = *(const float2 *)(rows + (q < ncoh ? q : s.k + q - ncoh) * pitch);
+            take_signed(v.x, v.y, base, best_s, best_i);
+          }
+        }
+      } else if (f == nk) {
         for (uint32_t q = tid; q < ncoh + s.m; q += T) offer(row_sum(q < ncoh ? q : s.k + q - ncoh, 0, nk, 0.0f), q);
         block_best(my_s, my_i, best_s, best_i);
       } else {
@@ -3416,12 +3526,12 @@ __device__ __forceinline__ void resolve_small_body(const SessionDev &s, const St
   if (b.fused_commit && tid == 0 && evals) atomicAdd(s.evals, (unsigned long long)evals);
 }
 
-template <int T, bool kG>
+template <int T, bool kG, int kMode>
 __global__ void __launch_bounds__(T, 1024 / T)
     k_resolve_small(const __grid_constant__ SessionDev s, const __grid_constant__ StageDev st,
                     const __grid_constant__ BatchDev b, const __grid_constant__ PendingCommit pc, uint32_t F) {
   pdl_launch();
-  resolve_small_body<T, kG>(s, st, b, pc, F);
+  resolve_small_body<T, kG, kMode>(s, st, b, pc, F);
 }
 
 // One step of a batch of new items whose neighbours the exhaustive k-NN
@@ -3685,6 +3795,8 @@ __global__ void __launch_bounds__(T) k_step_team_full(const __grid_constant__ Se
         best_s = FLT_MAX;
         best_i = 0;
       }
+    } else if (costs_in_order<kCostAny>(st) && !(sh_flags & 1)) {
+      if (warp == 0) best_in_order(s, st, w, lc, lg, nk, nc, best_s, best_i);
     } else if (tid == 0) {
       sequential_best(s, st, w, lc, lg, nk, nc, best_s, best_i);
     }
@@ -3773,6 +3885,8 @@ cudaError_t configure_kernels(uint32_t k, uint32_t m, uint32_t n_maps) {
   if (e != cudaSuccess) return e;
   e = raise_smem(k_resolve_lean, resolve_smem_bytes(k, m));
   if (e != cudaSuccess) return e;
+  e = raise_smem(k_resolve_signed, resolve_smem_bytes(k, m));
+  if (e != cudaSuccess) return e;
   e = raise_smem(k_knn_exhaustive, kExhAllKeys * 8);
   if (e != cudaSuccess) return e;
   e = raise_smem(k_mean_staged, (size_t)k * kMeanThreads * 8);
@@ -3783,8 +3897,11 @@ cudaError_t configure_kernels(uint32_t k, uint32_t m, uint32_t n_maps) {
   if (e != cudaSuccess) return e;
   if (k > 0 && k <= kSmallK && small_smem_bytes(k, m, n_maps) <= kSmallMaxSmem) {
     const size_t b = small_smem_bytes(k, m, n_maps);
-    for (auto kernel : {k_resolve_small<512, false>, k_resolve_small<512, true>, k_resolve_small<256, false>,
-                        k_resolve_small<256, true>, k_resolve_small<128, false>, k_resolve_small<128, true>}) {
+    for (auto kernel :
+         {k_resolve_small<512, false, kCostPlain>, k_resolve_small<512, true, kCostPlain>,
+          k_resolve_small<256, false, kCostPlain>, k_resolve_small<256, true, kCostPlain>,
+          k_resolve_small<128, false, kCostPlain>, k_resolve_small<128, true, kCostPlain>,
+          k_resolve_small<512, true, kCostSigned>, k_resolve_small<256, true, kCostSigned>}) {
       e = raise_smem(kernel, b);
       if (e != cudaSuccess) return e;
     }
@@ -3995,18 +4112,15 @@ void launch_resolve(const SessionDev &s, const StageDev &st, const BatchDev &b, 
   const uint32_t n = b.i1 - b.i0;
   if (n == 0 && pc.n == 0) return;
   const size_t smem = resolve_smem_bytes(s.k, s.m);
+  const auto kernel = !s.guided ? k_resolve_lean : st.slow_lut == kLutSigned ? k_resolve_signed : k_resolve;
   uint32_t grid = cdiv(n, kResolveWarps);
   if (b.work_ctr) {
     // a resident grid whose warps take further items from the counter
-    const uint32_t cap = s.guided ? resident_blocks(k_resolve, kResolveWarps * kWarp, smem)
-                                  : resident_blocks(k_resolve_lean, kResolveWarps * kWarp, smem);
+    const uint32_t cap = resident_blocks(kernel, kResolveWarps * kWarp, smem);
     if (cap) grid = std::min(grid, cap);
   }
   grid = std::max(grid, cdiv(pc.n, kResolveWarps * kWarp));
-  if (s.guided)
-    launch_pdl(k_resolve, grid, kResolveWarps * kWarp, smem, stream, s, st, b, pc);
-  else
-    launch_pdl(k_resolve_lean, grid, kResolveWarps * kWarp, smem, stream, s, st, b, pc);
+  launch_pdl(kernel, grid, kResolveWarps * kWarp, smem, stream, s, st, b, pc);
 }
 
 // The small-step form: up to kSmallK neighbours, the term rows within
@@ -4020,10 +4134,12 @@ static void launch_small_t(const SessionDev &s, const StageDev &st, const BatchD
                            const PendingCommit &pc) {
   const uint32_t grid = std::max(1u, b.i1 - b.i0);
   const size_t smem = small_smem_bytes(s.k, s.m, s.n_maps);
-  if (s.guided)
-    launch_pdl(k_resolve_small<T, true>, grid, T, smem, stream, s, st, b, pc, F);
+  if (!s.guided)
+    launch_pdl(k_resolve_small<T, false, kCostPlain>, grid, T, smem, stream, s, st, b, pc, F);
+  else if (T != 128 && st.slow_lut == kLutSigned)
+    launch_pdl(k_resolve_small<(T != 128 ? T : 256), true, kCostSigned>, grid, T, smem, stream, s, st, b, pc, F);
   else
-    launch_pdl(k_resolve_small<T, false>, grid, T, smem, stream, s, st, b, pc, F);
+    launch_pdl(k_resolve_small<T, true, kCostPlain>, grid, T, smem, stream, s, st, b, pc, F);
 }
 
 // Threads per item by the step's items: 512 while every item has an SM, 256
@@ -4045,9 +4161,17 @@ void launch_resolve_team(const SessionDev &s, const StageDev &st, const BatchDev
   if (n == 0 && pc.n == 0) return;
   // larger steps of more than one round of neighbours are bound by work per
   // item, not its latency: the early-exit form below (k = m = 50: 2.49
-  // against 2.60 ms a 256^2 call; k = m = 8: 1.40 against 1.33)
-  if (small_fits(s) && (full || s.k <= kWarp)) {
-    launch_small(s, st, b, full, stream, pc);
+  // against 2.60 ms a 256^2 call; k = m = 8: 1.40 against 1.33).  Costs that
+  // have to be looked at in order leave early less often: full scoring
+  // (guided inpainting, 250^2 0.53 against 0.58 ms, 256^2 0.53 against 0.54,
+  // 512^2 0.90 either way), else the warp form's copy.
+  const bool in_order = st.slow_lut == kLutSigned;
+  if (small_fits(s) && (full || s.k <= kWarp || in_order)) {
+    launch_small(s, st, b, full || in_order, stream, pc);
+    return;
+  }
+  if (in_order) {
+    launch_resolve(s, st, b, stream, pc);
     return;
   }
   uint32_t grid = n < 152u * 16u ? n : 152u * 16u;

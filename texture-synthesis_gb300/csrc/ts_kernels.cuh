@@ -126,9 +126,15 @@ constexpr int kCell = 8;
 // dx^2 + dy^2 <= kKnnTabRadius^2.
 constexpr int kKnnTabRadius = 36;
 
+// A stage's cost tables: no entry below zero (terms never lower a partial sum:
+// early exit and any-order argmin); finite with negative entries (guided
+// sessions only; candidates are taken in order by their largest partial sums);
+// anything else (the exact sequential argmin).
+enum : int { kLutPlain = 0, kLutSigned = 1, kLutExact = 2 };
+
 struct StageDev {
   uint32_t level;
-  int slow_lut;            // LUT holds a non-finite or negative value: exact sequential argmin
+  int slow_lut;            // kLut*: what the LUT allows
   // Every texel the cost loop can compare has alpha 255 and both LUTs hold
   // +-0 at |a - b| = 0: the alpha channel's term adds +-0 to a partial sum,
   // which leaves it unchanged, so the fast cost loops skip it

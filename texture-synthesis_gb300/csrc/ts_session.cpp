@@ -1242,7 +1242,7 @@ struct StagePlan {
   uint32_t n_res_start;
   uint64_t seed;
   uint32_t items_off, n_items, redo;
-  bool slow_lut;
+  int slow_lut;  // kLut*
   std::vector<BatchPlan> batches;
 };
 
@@ -1616,22 +1616,26 @@ void run_plan(ts_session *s, RunCtx &c) {
       adaptive = (a * a) * a;
     }
     // stage LUTs (ms.rs:853-858): content = (1 - a) * cauchy when guided.
-    // Early exit and any-order argmin need terms that never lower a partial
-    // sum, so a non-finite or negative entry sends the stage to the exact
-    // sequential form.  Negative ones come from guided inpainting: a is
-    // negative once the locked pixels outnumber the ones to synthesise.
-    bool slow = false;
+    // Negative entries come from guided inpainting: a is negative once the
+    // locked pixels outnumber the ones to synthesise.  (kLutSigned: sums of
+    // 256 neighbours' terms stay finite.)
+    bool finite = true, below = false, large = false;
+    auto look = [&](float v) {
+      finite &= std::isfinite(v);
+      below |= v < 0.0f;
+      large |= std::fabs(v) >= 0x1p100f;
+    };
     for (int d = 0; d < 256; ++d) {
       const float cv = s->guided ? (1.0f - adaptive) * cauchy[d] : cauchy[d];
       luts.push_back(cv);
-      slow |= !std::isfinite(cv) || cv < 0.0f;
+      look(cv);
     }
     for (int d = 0; d < 256; ++d) {
       const float gv = s->guided ? adaptive * l2[d] : 0.0f;
       luts.push_back(gv);
-      slow |= !std::isfinite(gv) || gv < 0.0f;
+      look(gv);
     }
-    sp.slow_lut = slow;
+    sp.slow_lut = finite && !below ? kLutPlain : finite && !large && s->guided ? kLutSigned : kLutExact;
     const size_t P_eff = std::min(P, redo + n_unresolved);
     sp.items_off = (uint32_t)n_items_total;
     sp.n_items = (uint32_t)P_eff;
@@ -2089,7 +2093,7 @@ void run_alloc(RunCtx &c, cudaStream_t pool) {
     }
     StageDev sdv{};
     sdv.level = sp.level;
-    sdv.slow_lut = sp.slow_lut ? 1 : 0;
+    sdv.slow_lut = sp.slow_lut;
     sdv.lut = c.d_lut.p + si * 512;
     sdv.opaque = (s->opaque && !sp.slow_lut && c.luts[si * 512] == 0.0f && c.luts[si * 512 + 256] == 0.0f) ? 1 : 0;
     sdv.stage_seed = sp.seed;
