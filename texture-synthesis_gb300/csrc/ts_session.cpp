@@ -3480,7 +3480,7 @@ struct ServerReq {
   // Made on streams beside the ticks: the picks (pick_ev per stage, where no
   // lists are made ahead), and with k-NN ahead the chunks of lists, the step
   // that needs each, and how many are enqueued.
-  cudaStream_t kst = nullptr;  // the server's
+  cudaStream_t kst = nullptr, rst = nullptr;  // the server's: picks and lists; random candidates
   std::vector<EventHandle> pick_ev;
   std::vector<size_t> chunk_step;
   size_t n_chunks = 0;
@@ -3495,6 +3495,12 @@ struct ServerReq {
 
 constexpr uint32_t kServerRing = 8;  // ticks in flight
 constexpr size_t kLoneSteps = 16;    // steps of a tick that holds a single request
+// Streams that the requests' random candidates go to by slot: a small
+// request's launches are one item's long chain of draws each, which one stream
+// ran one after another (16 inpaintings of 64^2, k = 50: m = 50 6.2 ms, m = 200
+// 17.9; on 4, 8, 16 streams 3.6, 3.5, 3.5 and 6.2, 4.2, 3.6; larger requests
+// take the same on any).
+constexpr uint32_t kServerRcStreams = 16;
 
 }  // namespace
 
@@ -3519,7 +3525,7 @@ struct ts_server {
   std::vector<ServerReq *> active;  // driver thread only
   std::thread driver, completer;
   cudaStream_t st = nullptr, ust = nullptr, cst = nullptr;  // compute, upload, completion
-  cudaStream_t ks[kBatchKnnStreams] = {}, rs = nullptr;       // picks and neighbour lists; random candidates
+  cudaStream_t ks[kBatchKnnStreams] = {}, rs[kServerRcStreams] = {};  // picks and neighbour lists; random candidates
   DevBuf<SessionDev> d_sess;
   DevBuf<const StepDev *> d_tabs;
   struct Ring {
@@ -3577,13 +3583,14 @@ void server_admit(ts_server *S, ServerReq *r) {
   for (size_t t = 0; t < c.steps.size(); ++t)
     if (c.steps[t].knn_wait >= 0) r->chunk_step.push_back(t);
   if (c.rc_ahead) {
-    CUDA_TRY(cudaStreamWaitEvent(S->rs, r->up_ev, 0));
+    r->rst = S->rs[r->slot % kServerRcStreams];
+    CUDA_TRY(cudaStreamWaitEvent(r->rst, r->up_ev, 0));
     c.rc_ev.resize(c.plan.size());
     for (size_t q = 0; q < c.plan.size(); ++q) {
       if (c.rc_step[q] < 0) continue;
-      launch_random_candidates(c.sd, c.steps[c.rc_step[q]].rc_st, S->rs);
+      launch_random_candidates(c.sd, c.steps[c.rc_step[q]].rc_st, r->rst);
       CUDA_TRY(cudaEventCreateWithFlags(&c.rc_ev[q].e, cudaEventDisableTiming));
-      CUDA_TRY(cudaEventRecord(c.rc_ev[q].e, S->rs));
+      CUDA_TRY(cudaEventRecord(c.rc_ev[q].e, r->rst));
     }
   }
   if (!c.knn_ahead) {
@@ -3910,7 +3917,7 @@ void server_completer(ts_server *S) {
     const bool admitted = r->slotted;
     if (r->ev) cudaEventSynchronize(r->ev);  // no kernel of the request is left
     if (r->status != TS_OK)  // nor, after a failure, anything beside the ticks
-      for (cudaStream_t q : {S->ust, r->kst, S->rs, S->st})
+      for (cudaStream_t q : {S->ust, r->kst, r->rst, S->st})
         if (q) cudaStreamSynchronize(q);
     // the run's buffers are pool memory (freed in stream order, no device
     // wait); the session's pyramids are freed with it
@@ -3961,7 +3968,7 @@ ts_server *ts_server_new(int32_t device, uint64_t hbm_budget_bytes, uint32_t max
     CUDA_TRY(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
     CUDA_TRY(cudaStreamCreateWithPriority(&S->st, cudaStreamNonBlocking, prio_high));
     for (cudaStream_t &q : S->ks) CUDA_TRY(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, prio_low - 1));
-    CUDA_TRY(cudaStreamCreateWithPriority(&S->rs, cudaStreamNonBlocking, prio_low));
+    for (cudaStream_t &q : S->rs) CUDA_TRY(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, prio_low));
     CUDA_TRY(cudaStreamCreateWithFlags(&S->ust, cudaStreamNonBlocking));
     CUDA_TRY(cudaStreamCreateWithFlags(&S->cst, cudaStreamNonBlocking));
     CUDA_TRY(S->d_sess.alloc(S->max_active));
@@ -4009,7 +4016,8 @@ void ts_server_free(ts_server *S) {
   if (S->cst) cudaStreamDestroy(S->cst);
   for (cudaStream_t q : S->ks)
     if (q) cudaStreamDestroy(q);
-  if (S->rs) cudaStreamDestroy(S->rs);
+  for (cudaStream_t q : S->rs)
+    if (q) cudaStreamDestroy(q);
   delete S;
 }
 
