@@ -2443,6 +2443,7 @@ __global__ void k_inpaint_init(const __grid_constant__ SessionDev s, const __gri
 // picks of each entry linked in any order.  The host's chain of swap-removes
 // takes some 10 ns a pick, 27 ms for the last stage of a 2048^2 output.
 // ---------------------------------------------------------------------------
+constexpr uint32_t kPickChainThreads = 1024;
 __global__ void k_pick_init(uint32_t *un, uint32_t n) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) un[i] = i;
 }
@@ -2450,8 +2451,8 @@ __global__ void k_pick_over(uint32_t *un, const uint32_t *over, uint32_t n_over)
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_over; i += gridDim.x * blockDim.x)
     un[over[2 * (size_t)i]] = over[2 * (size_t)i + 1];
 }
-__global__ void k_pick_draw(const __grid_constant__ PickStage ps) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ps.redo + ps.n_new; i += gridDim.x * blockDim.x) {
+__device__ __forceinline__ void pick_draw(const PickStage &ps, uint32_t first, uint32_t step) {
+  for (uint32_t i = first; i < ps.redo + ps.n_new; i += step) {
     if (i < ps.redo) {
       const uint32_t v = ps.redo_from[i];
       ps.items[i] = v;
@@ -2477,9 +2478,9 @@ __device__ __forceinline__ uint32_t pick_follow(const PickStage &ps, uint32_t p,
     p = ps.len0 - 1u - t;
   }
 }
-__global__ void k_pick_follow(const __grid_constant__ PickStage ps) {
+__device__ __forceinline__ void pick_follow_all(const PickStage &ps, uint32_t first, uint32_t step) {
   // threads [n_new, len0): the entries of the list after the stage
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < ps.len0; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = first; i < ps.len0; i += step) {
     if (i < ps.n_new) {
       const uint32_t v = pick_follow(ps, ps.draw[i], i);
       ps.items[ps.redo + i] = v;
@@ -2487,6 +2488,31 @@ __global__ void k_pick_follow(const __grid_constant__ PickStage ps) {
     } else {
       ps.un_next[i - ps.n_new] = pick_follow(ps, i - ps.n_new, ps.n_new);
     }
+  }
+}
+
+__global__ void k_pick_draw(const __grid_constant__ PickStage ps) {
+  pick_draw(ps, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+__global__ void k_pick_follow(const __grid_constant__ PickStage ps) {
+  pick_follow_all(ps, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+// The whole chain of a run of few items, a block per run: one launch instead
+// of three calls a stage.
+__global__ void __launch_bounds__(kPickChainThreads) k_pick_chain(const PickChain *chains) {
+  const PickChain &ch = chains[blockIdx.x];
+  for (uint32_t i = threadIdx.x; i < ch.n_un; i += blockDim.x) ch.un[i] = i;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < ch.n_over; i += blockDim.x) ch.un[ch.over[2 * i]] = ch.over[2 * i + 1];
+  __syncthreads();
+  for (uint32_t q = 0; q < ch.n; ++q) {
+    const PickStage &ps = ch.st[q];
+    for (uint32_t i = threadIdx.x; i < ps.len0; i += blockDim.x) ps.head[i] = 0;
+    __syncthreads();
+    pick_draw(ps, threadIdx.x, blockDim.x);
+    __syncthreads();
+    if (ps.n_new) pick_follow_all(ps, threadIdx.x, blockDim.x);
+    __syncthreads();
   }
 }
 
@@ -4227,6 +4253,10 @@ void launch_picks(const PickStage &ps, cudaStream_t stream) {
   if (ps.redo + ps.n_new == 0) return;
   k_pick_draw<<<pick_grid((uint64_t)ps.redo + ps.n_new), 256, 0, stream>>>(ps);
   if (ps.n_new) k_pick_follow<<<pick_grid(ps.len0), 256, 0, stream>>>(ps);
+}
+
+void launch_pick_chains(const PickChain *chains, uint32_t n, cudaStream_t stream) {
+  if (n) k_pick_chain<<<n, kPickChainThreads, 0, stream>>>(chains);
 }
 
 void launch_tree_append(const SessionDev &s, const StageDev &st, uint32_t a0, uint32_t a1, uint32_t pos0,

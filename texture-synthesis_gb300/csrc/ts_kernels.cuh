@@ -316,6 +316,17 @@ struct PickStage {
 };
 void launch_picks(const PickStage &ps, cudaStream_t stream);
 // un = 0, 1, .., n - 1, then un[over[2i]] = over[2i + 1] for i < n_over.
+// The chain of a run of few items: un starts as 0, 1, .., n_un - 1 with the
+// entries over (pairs as below) on top, then n stages (whose heads need not be
+// zeroed).  chains: n of them, in device memory.
+constexpr uint32_t kPickChainStages = 8;
+struct PickChain {
+  PickStage st[kPickChainStages];
+  uint32_t n, n_un, n_over;
+  uint32_t *un;
+  const uint32_t *over;
+};
+void launch_pick_chains(const PickChain *chains, uint32_t n, cudaStream_t stream);
 void launch_pick_init(uint32_t *un, uint32_t n, const uint32_t *over, uint32_t n_over, cudaStream_t stream);
 
 // Initial state of an inpainting run.  open: a bit per pixel to synthesise, a

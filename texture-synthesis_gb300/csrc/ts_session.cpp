@@ -2279,11 +2279,12 @@ void run_enqueue_picks_init(RunCtx &c, cudaStream_t st) {
   ++c.launches;
 }
 
-void run_enqueue_picks(RunCtx &c, cudaStream_t st) {
+// The next stage (false: an empty one) and the state after it.
+bool next_pick_stage(RunCtx &c, PickStage &ps) {
   const size_t q = c.picked_stages++;
   const StagePlan &sp = c.plan[q];
-  if (sp.n_items == 0) return;
-  PickStage ps{};
+  if (sp.n_items == 0) return false;
+  ps = PickStage{};
   ps.seed = sp.seed;
   ps.redo = std::min(sp.redo, sp.n_items);
   ps.n_new = sp.n_items - ps.redo;
@@ -2299,12 +2300,40 @@ void run_enqueue_picks(RunCtx &c, cudaStream_t st) {
   ps.next = c.d_pnext.p;
   ps.draw = c.d_pdraw.p;
   if (ps.n_new) {
-    CUDA_TRY(cudaMemsetAsync(c.d_phead.p, 0, c.pick_len * 4, st));
     c.pick_parity ^= 1u;
     c.pick_len -= ps.n_new;
   }
+  return true;
+}
+
+void run_enqueue_picks(RunCtx &c, cudaStream_t st) {
+  PickStage ps;
+  if (!next_pick_stage(c, ps)) return;
+  if (ps.n_new) CUDA_TRY(cudaMemsetAsync(c.d_phead.p, 0, (size_t)ps.len0 * 4, st));
   launch_picks(ps, st);
   c.launches += 2;
+}
+
+// A run of few items (a small inpainting): its picks and lists made ahead are
+// some sixty calls for little work, on the server's one driver thread or the
+// batch's calling thread.  Where several runs share the steps, these make the
+// lists instead, and the picks are one launch (64^2, k = m = 8, inpainted:
+// served 16 at once 3.6 -> 2.7 ms, batches of 16 3.9 -> 2.9; 90 x 80, k = 20: 3.8
+// -> 3.4, 4.2 -> 3.5; from 4500 items on, 48^2 synthesised, lists ahead take
+// half the time).
+constexpr uint64_t kFewItems = 4096;
+bool few_items(const RunCtx &c) { return c.n_items < kFewItems && c.plan.size() <= kPickChainStages; }
+
+PickChain run_pick_chain(RunCtx &c) {
+  PickChain ch{};
+  ch.un = c.d_un[0].p;
+  ch.n_un = c.s->inpaint ? 0 : (uint32_t)c.n_unresolved;  // (run_upload made inpainting's list)
+  ch.over = c.d_over.p;
+  ch.n_over = (uint32_t)(c.un_over.size() / 2);
+  c.pick_len = c.n_unresolved;
+  while (c.picked_stages < c.plan.size())
+    if (next_pick_stage(c, ch.st[ch.n])) ++ch.n;
+  return ch;
 }
 
 // Whether the commit of step `stp` can be left to the first k-NN launch of
@@ -2996,7 +3025,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
         const uint64_t room = device_room(b->device);
         uint64_t left = std::min<uint64_t>(kBatchAheadMaxBytes, room > base ? (room - base) / 2 : 0);
         for (size_t j = 0; j < n; ++j) {
-          if (!ctx[j] || b->graph) continue;
+          if (!ctx[j] || b->graph || (n > 1 && few_items(*ctx[j]))) continue;
           const uint64_t need = knn_ahead_bytes(*ctx[j]);
           if (need > left) continue;
           ctx[j]->want_knn_ahead = true;
@@ -3216,6 +3245,11 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     DevBuf<StepDev> d_steps;
     DevBuf<Segment> d_segs, d_fb;
     DevBuf<const StepDev *> d_tabs;
+    DevBuf<PickChain> d_chains;  // sessions of few items without k-NN ahead
+    std::vector<PickChain> h_chains;
+    for (size_t j = 0; j < n; ++j)
+      if (!ctx[j]->knn_ahead && few_items(*ctx[j])) h_chains.push_back(run_pick_chain(*ctx[j]));
+    CUDA_TRY(d_chains.alloc_on(h_chains.size(), st));
     CUDA_TRY(d_tabs.alloc_on(n, st));
     CUDA_TRY(d_sess.alloc_on(n, st));
     CUDA_TRY(d_steps.alloc_on(n_steps, st));
@@ -3232,6 +3266,9 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
       if (c.knn_ahead) launch_rank_init(c.sd, (uint32_t)c.locked, st);
     }
     CUDA_TRY(cudaMemcpyAsync(d_sess.p, h_sess.data(), n * sizeof(SessionDev), cudaMemcpyHostToDevice, st));
+    if (!h_chains.empty())
+      CUDA_TRY(cudaMemcpyAsync(d_chains.p, h_chains.data(), h_chains.size() * sizeof(PickChain),
+                               cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(d_steps.p, h_steps.data(), n_steps * sizeof(StepDev), cudaMemcpyHostToDevice, st));
     std::vector<const StepDev *> h_tabs(n);
     for (size_t j = 0; j < n; ++j) h_tabs[j] = d_steps.p + step_base[j];
@@ -3280,9 +3317,10 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     // the picks of stage 0 (part 0) and of the later stages (part 1), every
     // session's without k-NN ahead
     auto pick_items = [&](int part) {
+      if (part == 0) launch_pick_chains(d_chains.p, (uint32_t)h_chains.size(), rg.s);
       for (size_t j = 0; j < n; ++j) {
         RunCtx &c = *ctx[j];
-        if (c.knn_ahead) continue;
+        if (c.knn_ahead || few_items(c)) continue;
         if (part == 0) run_enqueue_picks_init(c, rg.s);
         for (size_t q = part == 0 ? 0 : 1; q < (part == 0 ? std::min<size_t>(1, c.plan.size()) : c.plan.size()); ++q)
           run_enqueue_picks(c, rg.s);
@@ -3395,7 +3433,7 @@ int ts_batch_run(ts_batch *b, ts_generated **out) {
     ts_batch_stats bs{};
     bs.sessions = n;
     bs.steps = max_steps;
-    bs.launches = launches.size() + rc_launches.size();
+    bs.launches = launches.size() + rc_launches.size() + (h_chains.empty() ? 0 : 1);
     for (size_t j = 0; j < n; ++j) bs.launches += ctx[j]->launches;
     for (const PlannedLaunch &pl : launches)
       if (pl.phase == kPhaseResolve) bs.launches += resolve_launches(pl.n_lean, pl.n_segs, pl.blocks) - 1;
@@ -3468,6 +3506,7 @@ struct ServerReq {
   ts_session *s = nullptr;  // owned
   std::unique_ptr<RunCtx> c;
   DevBuf<StepDev> d_steps;
+  DevBuf<PickChain> d_chain;  // few_items
   uint32_t slot = 0;
   bool slotted = false;  // holds a slot and its budget charge
   size_t cursor = 0;
@@ -3478,7 +3517,7 @@ struct ServerReq {
   ts_generated *result = nullptr;
   bool done = false;
   // Made on streams beside the ticks: the picks (pick_ev per stage, where no
-  // lists are made ahead), and with k-NN ahead the chunks of lists, the step
+  // lists are made ahead; one for the whole chain of few items), and with k-NN ahead the chunks of lists, the step
   // that needs each, and how many are enqueued.
   cudaStream_t kst = nullptr, rst = nullptr;  // the server's: picks and lists; random candidates
   std::vector<EventHandle> pick_ev;
@@ -3495,6 +3534,10 @@ struct ServerReq {
 
 constexpr uint32_t kServerRing = 8;  // ticks in flight
 constexpr size_t kLoneSteps = 16;    // steps of a tick that holds a single request
+// Other requests, active or waiting, from which one of few items makes no lists
+// ahead (alone, 64^2 inpainted, k = m = 50: 0.50 ms with lists, 0.62 without; of
+// four, 0.99 ms from two others on, 1.12 from four on, with k = m = 8).
+constexpr size_t kServerCrowd = 2;
 // Streams that the requests' random candidates go to by slot: a small
 // request's launches are one item's long chain of draws each, which one stream
 // ran one after another (16 inpaintings of 64^2, k = 50: m = 50 6.2 ms, m = 200
@@ -3555,6 +3598,11 @@ void server_admit(ts_server *S, ServerReq *r) {
   run_alloc_fit(c, S->ust);
   run_upload(c, S->ust);
   if (c.knn_ahead) launch_rank_init(c.sd, (uint32_t)c.locked, S->ust);
+  if (!c.knn_ahead && few_items(c)) {
+    const PickChain ch = run_pick_chain(c);
+    CUDA_TRY(r->d_chain.alloc_on(1, S->ust));
+    CUDA_TRY(cudaMemcpyAsync(r->d_chain.p, &ch, sizeof(ch), cudaMemcpyHostToDevice, S->ust));
+  }
   std::vector<StepDev> h(c.steps.size());
   for (size_t t = 0; t < c.steps.size(); ++t) {
     const Step &stp = c.steps[t];
@@ -3593,7 +3641,13 @@ void server_admit(ts_server *S, ServerReq *r) {
       CUDA_TRY(cudaEventRecord(c.rc_ev[q].e, r->rst));
     }
   }
-  if (!c.knn_ahead) {
+  if (!c.knn_ahead && few_items(c)) {
+    r->pick_ev.resize(1);
+    launch_pick_chains(r->d_chain.p, 1, r->kst);
+    ++c.launches;
+    CUDA_TRY(cudaEventCreateWithFlags(&r->pick_ev[0].e, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(r->pick_ev[0].e, r->kst));
+  } else if (!c.knn_ahead) {
     run_enqueue_picks_init(c, r->kst);
     r->pick_ev.resize(c.plan.size());
     for (EventHandle &e : r->pick_ev) {
@@ -3619,7 +3673,7 @@ void server_before_step(ts_server *S, ServerReq *r, size_t t) {
       run_enqueue_chunk(c, q, r->kst, r->kst, lt);
     }
     if (stp.knn_wait >= 0) CUDA_TRY(cudaStreamWaitEvent(S->st, c.knn_ev[stp.knn_wait].e, 0));
-  } else if (t == 0 || c.steps[t - 1].stage != stp.stage) {
+  } else if (t == 0 || (c.steps[t - 1].stage != stp.stage && (size_t)stp.stage < r->pick_ev.size())) {
     CUDA_TRY(cudaStreamWaitEvent(S->st, r->pick_ev[stp.stage].e, 0));
   }
   if (stp.rc && c.rc_ahead && c.rc_ev[stp.stage].e) CUDA_TRY(cudaStreamWaitEvent(S->st, c.rc_ev[stp.stage].e, 0));
@@ -3665,7 +3719,8 @@ void server_driver(ts_server *S) {
         const uint64_t rc_b = (rc_n - std::min(rc_n, chunk_n)) * c.m * 8;
         const uint64_t knn_b = knn_ahead_bytes(c);
         c.want_knn_ahead = true;
-        c.want_knn_ahead = knn_ahead_fits(c, c.W, c.H, c.k) && held + r->bytes + knn_b <= S->budget;
+        c.want_knn_ahead = knn_ahead_fits(c, c.W, c.H, c.k) && held + r->bytes + knn_b <= S->budget &&
+                           !(few_items(c) && S->active.size() + S->pending.size() >= kServerCrowd);
         if (c.want_knn_ahead) r->bytes += knn_b;
         c.rc_ahead = c.m > 0 && (uint64_t)c.n_items * c.m <= kRcandWholeSmall && held + r->bytes + rc_b <= S->budget;
         if (c.rc_ahead) r->bytes += rc_b;
@@ -3923,6 +3978,7 @@ void server_completer(ts_server *S) {
     // wait); the session's pyramids are freed with it
     r->c.reset();
     r->d_steps.reset();
+    r->d_chain.reset();
     delete r->s;
     r->s = nullptr;
     {
