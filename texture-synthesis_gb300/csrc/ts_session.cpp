@@ -1471,28 +1471,34 @@ uint64_t knn_ahead_bytes(const RunCtx &c) {
          (c.multi ? 0 : (uint64_t)c.N * 2 * sizeof(uint4) + (uint64_t)c.max_batch_items * sizeof(Result));
 }
 
-// Device memory that the stream-ordered pool can still hand out.
-uint64_t device_room(int dev) {
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+// Memory that the stream-ordered pool holds and nobody uses, and with what the
+// device has left: what the pool can still hand out.
+uint64_t pool_idle(int dev) {
   cudaMemPool_t pool;
   uint64_t reserved = 0, used = 0;
   if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
-    free_b += reserved - used;
-  return free_b;
+    return reserved - used;
+  return 0;
+}
+uint64_t device_room(int dev) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 0;
+  return free_b + pool_idle(dev);
 }
 
 // Whether the device has room for the lists of a run by itself: as with the
 // random candidates, large ones only where there is four times the room beside
 // the rest of the run, so that runs side by side, and what the program holds
-// besides, still fit.  (The query takes the driver some time, which small runs
-// go without; run_alloc_fit covers those.)
+// besides, still fit.  (The device's free memory takes the driver up to 0.2 ms
+// to tell, 2048^2, k = m = 8: 16.1 against 15.9 ms a call; small runs, which
+// run_alloc_fit covers, and runs that the pool's idle memory holds go without.)
 bool knn_ahead_room(const RunCtx &c) {
   constexpr uint64_t kKnnAheadSmall = 256ull << 20;
   const uint64_t lists = knn_ahead_bytes(c);
-  return lists <= kKnnAheadSmall || device_room(c.s->prm.device) >= c.dev_bytes + 4 * lists;
+  return lists <= kKnnAheadSmall || pool_idle(c.s->prm.device) >= c.dev_bytes + lists ||
+         device_room(c.s->prm.device) >= c.dev_bytes + 4 * lists;
 }
 
 // Host schedule of Generator::resolve (ms.rs:702-1051) and the device
