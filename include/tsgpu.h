@@ -443,8 +443,9 @@ void ts_server_stats_get(ts_server *s, ts_server_stats *out);
  * Each batch step's launch shape follows its item count: one warp per item
  * for large steps (throughput), one CTA of 128 threads per item with early
  * exit, or of 256 threads scoring every candidate, for small ones
- * (latency); on the plain path, the k-NN walk of a small step may also
- * build a bitmap window in shared memory.  The thresholds between these
+ * (latency); on the plain path, the k-NN walk of a small step (or of a chunk
+ * of steps that begins with one) may also build a bitmap window in shared
+ * memory.  The thresholds between these
  * never change a result, only the speed, which depends on the GPU, the
  * sizes, k and m.  The tuner runs the caller's own workload under candidate
  * thresholds, one threshold at a time starting from the defaults (of the
@@ -454,7 +455,9 @@ void ts_server_stats_get(ts_server *s, ts_server_stats *out);
 typedef struct ts_tuning {
   uint32_t team_max_items;         /* a CTA per item in steps of at most this many items */
   uint32_t team_full_max_items;    /* ... scoring every candidate up to this many */
-  uint32_t walk_window_max_items;  /* plain path: walk steps up to this many items may build a window */
+  /* plain path: walk steps up to this many items may build a window (lists
+   * made ahead: chunks of steps whose first has at most this many) */
+  uint32_t walk_window_max_items;
   uint32_t trials;                 /* runs the tuner made (0 for ts_tuning_default) */
   double gpu_ms;                   /* median device time of the workload with this setting */
   double default_gpu_ms;           /* the same with the defaults */

@@ -121,7 +121,8 @@ class Tuning(C.Structure):
     """Launch-shape thresholds (ts_tuning): a CTA per item in steps of at
     most team_max_items items (every candidate scored up to
     team_full_max_items), and, on the plain path, a walk bitmap window in
-    steps of at most walk_window_max_items.  Results never depend on them."""
+    steps of at most walk_window_max_items (lists made ahead: chunks whose
+    first step is).  Results never depend on them."""
 
     _fields_ = [("team_max_items", C.c_uint32), ("team_full_max_items", C.c_uint32),
                 ("walk_window_max_items", C.c_uint32), ("trials", C.c_uint32), ("gpu_ms", C.c_double),

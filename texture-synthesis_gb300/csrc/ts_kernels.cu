@@ -74,11 +74,6 @@ __device__ __forceinline__ int off_dx(int32_t off) { return (int)(int16_t)(off &
 __device__ __forceinline__ int off_dy(int32_t off) { return off >> 16; }
 __device__ __forceinline__ int32_t pack_off(int dx, int dy) { return (int32_t)((uint32_t)(dx & 0xffff) | ((uint32_t)dy << 16)); }
 
-__device__ __forceinline__ int modi(int a, int b) {
-  int r = a % b;
-  return r < 0 ? r + b : r;
-}
-
 // a in [-n, 2n) wrapped into [0, n): every tree point and its tiling mirrors
 // lie there (the mirror bands are 5% of a side).
 __device__ __forceinline__ int wrap1(int a, int n) { return a < 0 ? a + n : (a >= n ? a - n : a); }
@@ -349,9 +344,10 @@ constexpr size_t kWalkWinBytes = (size_t)kWalkWarps * (kWinRows * kWinWords + kW
 // position per entry, else one bitmap word.  The last stage of a 2048^2 output
 // (2^22 items, beside its resolves): 11.6 -> 6.3 ms.
 //
-// kWin: small (latency-bound) launches, whose sparse items switch to a
-// window in dynamic shared memory (kWalkWinBytes) once the hits so far say
-// more than two further rounds are needed.  With the k-NN made ahead the
+// kWin: launches of small (latency-bound) steps, or of a chunk that begins
+// with one, whose sparse items switch to a window in dynamic shared memory
+// (kWalkWinBytes) once the hits so far say more than two further rounds are
+// needed.  With the k-NN made ahead the
 // window holds later points too: its hits wait in a list and are checked 32
 // at a time, so that a round without a full list waits for no load.
 template <bool kWin>
@@ -1408,7 +1404,7 @@ __device__ __forceinline__ float guided_chunk(const WarpSmem &w, const float *lc
 // within kPad: no bounds checks, gathers issued four neighbours ahead; with a
 // guide, whose evaluations are twice as long, six once a candidate has passed
 // its first four, where most random ones end (512^2, k = m = 50: 6.30 -> 5.95
-// ms; with four, five, seven, eight, twelve 6.10, 6.11, 6.08, 6.15, 6.3;
+// ms; with four, five, seven, eight, twelve 6.10, 6.11, 6.08, 6.15, 6.6;
 // without a guide six cost 2048^2 3%).
 // centre: texel index of the candidate's centre on the padded planes.
 template <bool kGuided, bool kOpaque>
@@ -1711,8 +1707,8 @@ __device__ __forceinline__ void take_signed(float sum, float peak, uint32_t firs
 // a repeat of an earlier candidate is never taken (that one was rejected by a
 // best that was no lower, or its sum, no more than its largest partial sum,
 // became the best).  Guided inpainting, k = m = 50, one lane going through all
-// candidates against this, device time: 256^2 2.61 against 0.53 ms, 512^2 3.39
-// against 0.91, 1024^2 6.75 against 2.22.
+// candidates against this, device time: 256^2 2.61 against 0.51 ms, 512^2 3.39
+// against 0.88, 1024^2 6.75 against 2.19.
 template <bool kG = true>
 __device__ void best_in_order(const SessionDev &s, const StageDev &st, const WarpSmem &w, const float *lc,
                               const float *lg, uint32_t nk, uint32_t nc, float &best_s, uint32_t &best_i) {
@@ -2407,9 +2403,10 @@ __global__ void k_scatter_init(const uint32_t *list, uint32_t n, uint32_t *color
 // Initial state of an inpainting run (Generator::new_from_inpaint,
 // ms.rs:236-293), a warp per 32 pixels of a row: a locked pixel's state, its
 // place in the resolved list and the tree, and the others' place in the
-// unresolved list (both in pixel order; un null: the host keeps that list).  in.before counts the pixels to synthesise before
-// each word.  The host's loops and the upload of colours and states took 1.5 ms
-// of a 512^2 run.
+// unresolved list (both in pixel order; a random init's picks have shortened
+// the latter, and k_pick_over puts in what they moved).  in.before counts the pixels to synthesise before each
+// word.  The host's loops took 1.9 ms of a 512^2 run, beside the upload of
+// colours and states.
 __global__ void k_inpaint_init(const __grid_constant__ SessionDev s, const __grid_constant__ InpaintDev in) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
   if (w >= s.wpr * s.H) return;
@@ -2423,7 +2420,7 @@ __global__ void k_inpaint_init(const __grid_constant__ SessionDev s, const __gri
   const uint32_t p = y * s.W + x, rank = in.before[w] + (uint32_t)__popc(open & ((1u << lane) - 1u));
   if ((open >> lane) & 1u) {
     s.state[p] = make_uint4(0, 0, 0, 0);
-    if (in.un && rank < in.n_un) in.un[rank] = p;
+    if (rank < in.n_un) in.un[rank] = p;
   } else {
     s.state[p] = make_uint4(x | (y << 16), 0, 0, in.map);
     s.resolved[p - rank] = p;

@@ -159,7 +159,7 @@ struct BatchDev {
   double *mean;          // [batch] mean of the 4x-duplicated distance list
   Result *res;           // [batch]
   int grid_first;        // sparse step: search the cell grid without walking the offset table first
-  int walk_window;       // small step (latency-bound): the single-session walk lets sparse items walk a shared-memory bitmap window
+  int walk_window;       // small step, or chunk that begins with one: the single-session walk lets sparse items walk a shared-memory bitmap window
   int fused_commit;      // only new items: the resolve kernels commit each item themselves (no k_commit)
   // k-NN made ahead over several batches (SessionDev::rank): btab[j] =
   // {first stage item, resolved-list length at the start} of the j-th batch
@@ -330,8 +330,8 @@ void launch_pick_chains(const PickChain *chains, uint32_t n, cudaStream_t stream
 void launch_pick_init(uint32_t *un, uint32_t n, const uint32_t *over, uint32_t n_over, cudaStream_t stream);
 
 // Initial state of an inpainting run.  open: a bit per pixel to synthesise, a
-// row's words as in SessionDev::occ; before: such pixels before each word; un (null: not wanted): their list, n_un entries of
-// it; map: the inpainting example.
+// row's words as in SessionDev::occ; before: such pixels before each word; un:
+// their list, n_un entries of it; map: the inpainting example.
 struct InpaintDev {
   const uint32_t *open, *before;
   uint32_t *un;

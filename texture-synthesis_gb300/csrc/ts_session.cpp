@@ -53,7 +53,9 @@ static_assert(kDistTabRadius >= kKnnTabRadius, "the walk's distances come from t
 constexpr uint64_t kRcandBudget = 64ull << 20;  // random-candidate entries held at once
 // Walk steps of at most this many items are latency-bound: their sparse items
 // build a bitmap window instead of more rounds of bitmap loads (the default;
-// ts_builder_tuning sets it per session).
+// ts_builder_tuning sets it per session).  With lists made ahead a chunk's
+// first step decides for its launch (by the chunk's own size, always or never:
+// no better or, always at 2048^2, 3.5% slower).
 constexpr uint32_t kWalkWindowItems = 4096;
 // Where the caller leaves the thresholds alone, a single session of more than
 // 32 neighbours (which take a warp two rounds) leaves the CTA per item from
@@ -1382,11 +1384,11 @@ struct RunCtx {
   bool want_rc_ahead = false, rc_ahead = false;
   std::vector<int> rc_step;
   std::vector<EventHandle> rc_ev;
-  // knn_ahead: the neighbour lists and means of every batch are made on a
-  // k-NN stream, chunk by chunk, as soon as a stage's items are up (they
+  // knn_ahead: the neighbour lists and means of every batch are made on
+  // other streams, chunk by chunk, as soon as a stage's picks are (they
   // depend on the pick chain's order only: which pixels are in the tree at
-  // each batch start); the resolves wait for their chunk's event.  Plain
-  // path, k > 0, exact distance sums.
+  // each batch start); the resolves wait for their chunk's event.  Where
+  // knn_ahead_fits allows it and the device, batch or budget has the room.
   bool want_knn_ahead = false, knn_ahead = false;
   // multi: the steps go out as multi-session launches (batch, server), which
   // commit in launches of their own and take one item per warp
@@ -1454,9 +1456,9 @@ bool exact_sum_ok(uint32_t W, uint32_t H, uint32_t k);
 // the lists of every item of the run, held at once, within kKnnAheadMaxBytes
 // (larger runs keep the per-step form's scratch), and exact sums or an output
 // of kKnnAheadMinPixels (203x117, k = 8: 1.78 against 2.62 ms a call; 500^2:
-// 7.28 against 8.14).  Smaller inexact outputs would gain as well (40^2,
-// k = 50: 2.05 against 3.09 ms) but are documented and tested to keep the
-// per-step form (ts_run_stats.knn_chunks).
+// 7.28 against 8.14).  That limit is ts_run_stats.knn_chunks' documented one,
+// which a test holds, not where the gain ends: 40^2, k = 50 took 2.05 ms ahead
+// against 3.09.
 bool knn_ahead_fits(const RunCtx &c, uint32_t W, uint32_t H, uint32_t k) {
   constexpr uint64_t kKnnAheadMaxBytes = 16ull << 30;
   constexpr uint64_t kKnnAheadMinPixels = 2048;
